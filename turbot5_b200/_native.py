@@ -5,6 +5,7 @@ operator raises, there is no fallback.  `torch` is used here only to read
 pointers, strides and the current stream.
 """
 import ctypes as C
+import importlib
 import os
 
 import torch
@@ -156,6 +157,25 @@ def lib():
         fn.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p]
     _lib = L
     return L
+
+
+class _Host:
+    """The native host extension (argument checks, allocation, launches and autograd nodes of the operators),
+    loaded on first use -- the build imports this package before the extension exists.  Raises if it
+    has not been built (no fallback path)."""
+
+    def __getattr__(self, name):
+        try:
+            module = importlib.import_module("turbot5_b200._host")
+        except ImportError as e:
+            raise RuntimeError("turbot5_b200/_host.so is missing or cannot be loaded: build it with "
+                               "`python -m turbot5_b200.build`.  turbot5_b200 has no CPU or PyTorch fallback.") from e
+        fn = getattr(module, name)
+        setattr(self, name, fn)         # found in the instance from now on
+        return fn
+
+
+host = _Host()
 
 
 def dtype_code(dt: torch.dtype) -> int:

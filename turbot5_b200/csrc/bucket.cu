@@ -26,7 +26,7 @@ static int bucket_of_distance_host(int d, int n_side, int max_distance) {
   return (int)v;
 }
 
-int make_bucket_spec(int num_buckets, int max_distance, int bidirectional, BucketSpec* spec) {
+static int compute_bucket_spec(int num_buckets, int max_distance, int bidirectional, BucketSpec* spec) {
   if (num_buckets < 2 || max_distance < 1 || max_distance > 32000) return T5B_ERR_ARG;
   int n_side = bidirectional ? num_buckets / 2 : num_buckets;
   if (n_side < 2 || n_side > kMaxBucketsPerSide) return T5B_ERR_ARG;
@@ -43,6 +43,26 @@ int make_bucket_spec(int num_buckets, int max_distance, int bidirectional, Bucke
   }
   for (int i = n_side - 1; i < kMaxBucketsPerSide; ++i) spec->first[i] = 32767;
   return T5B_OK;
+}
+
+// The thresholds take a hundred and more logarithms, a few microseconds, on every call of an operator;
+// a program uses one or two settings (encoder and decoder), so each thread keeps its last four.
+int make_bucket_spec(int num_buckets, int max_distance, int bidirectional, BucketSpec* spec) {
+  struct Entry { int nb = 0, md = 0, bidir = 0; BucketSpec spec; };
+  thread_local Entry cache[4];
+  thread_local unsigned next = 0;
+  for (const Entry& e : cache)
+    if (e.nb == num_buckets && e.md == max_distance && e.bidir == (bidirectional ? 1 : 0) && e.nb != 0) {
+      *spec = e.spec;
+      return T5B_OK;
+    }
+  const int st = compute_bucket_spec(num_buckets, max_distance, bidirectional, spec);
+  if (st == T5B_OK) {
+    Entry& e = cache[next++ % 4];
+    e.nb = num_buckets; e.md = max_distance; e.bidir = bidirectional ? 1 : 0;
+    e.spec = *spec;
+  }
+  return st;
 }
 
 int host_bucket_of_delta(const BucketSpec& s, long long delta) {

@@ -15,62 +15,13 @@ from .attention import (flash_attention_with_fusing_bias, flash_attention_with_f
 from .padding import get_unpad_plan, pad_rows, unpad_rows
 
 
+_host = nat.host
+
+
 def rms_layer_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, return_rstd: bool = False):
     """T5 RMSNorm on the device (replaces RMSLayerNorm.apply, src/turbot5/ops/rms_norm.py:129-185);
     differentiable in x and weight."""
-    if not return_rstd and torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
-        return _RMSNormFn.apply(x, weight, eps)
-    return _rms_layer_norm_fwd(x, weight, eps, return_rstd)
-
-
-class _RMSNormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, eps):
-        ctx.save_for_backward(x, weight)
-        ctx.eps = eps
-        return _rms_layer_norm_fwd(x, weight, eps)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
-        d = x.shape[-1]
-        x2 = x.reshape(-1, d)
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        out_dtype = weight.dtype if weight.dtype in (torch.float16, torch.bfloat16) else torch.float32
-        dy2 = dy.reshape(-1, d).to(out_dtype)
-        if dy2.stride(-1) != 1:
-            dy2 = dy2.contiguous()
-        dx = torch.empty((x2.shape[0], d), dtype=x.dtype, device=x.device)
-        dw = torch.zeros((d,), dtype=torch.float32, device=x.device)
-        w = weight.contiguous()
-        with torch.cuda.device(x.device):
-            nat.check(nat.lib().t5b_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), dx.data_ptr(),
-                                                dw.data_ptr(), x2.shape[0], d, x2.stride(0), dy2.stride(0),
-                                                dx.stride(0), nat.dtype_code(x.dtype), nat.dtype_code(w.dtype),
-                                                float(ctx.eps), nat.stream_ptr(x.device)), "rms_layer_norm (backward)")
-        return dx.view(x.shape), dw.to(weight.dtype), None
-
-
-def _rms_layer_norm_fwd(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, return_rstd: bool = False):
-    nat.require_cuda(x, weight)
-    d = x.shape[-1]
-    if weight.shape != (d,):
-        raise ValueError("weight must have the size of the last dimension")
-    x2 = x.reshape(-1, d)
-    if x2.stride(-1) != 1:
-        x2 = x2.contiguous()
-    weight = weight.contiguous()
-    out_dtype = weight.dtype if weight.dtype in (torch.float16, torch.bfloat16) else torch.float32
-    y = torch.empty((x2.shape[0], d), dtype=out_dtype, device=x.device)
-    rstd = torch.empty((x2.shape[0],), dtype=torch.float32, device=x.device) if return_rstd else None
-    with torch.cuda.device(x.device):
-        nat.check(nat.lib().t5b_rmsnorm_fwd(x2.data_ptr(), weight.data_ptr(), y.data_ptr(), nat.ptr(rstd),
-                                            x2.shape[0], d, x2.stride(0), y.stride(0), nat.dtype_code(x.dtype),
-                                            nat.dtype_code(weight.dtype), float(eps), nat.stream_ptr(x.device)),
-                  "rms_layer_norm")
-    y = y.view(*x.shape[:-1], d)
-    return (y, rstd) if return_rstd else y
+    return _host.rmsnorm(x, weight, eps, return_rstd)
 
 
 def add_rms_layer_norm(hidden: torch.Tensor, branch: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
@@ -79,45 +30,14 @@ def add_rms_layer_norm(hidden: torch.Tensor, branch: torch.Tensor, weight: torch
     closes a sub-layer fused with the norm that opens the next one
     (src/turbot5/model/modeling.py:124-128,142-164 + src/turbot5/model/modules.py:52-60).  bf16/fp16,
     forward only; with `inplace` the sum overwrites `hidden`."""
-    nat.require_cuda(hidden, branch, weight)
-    d = hidden.shape[-1]
-    if branch.shape != hidden.shape or branch.dtype != hidden.dtype or weight.shape != (d,):
-        raise ValueError("hidden and branch must match; weight must have the size of the last dimension")
-    h2, b2 = hidden.reshape(-1, d), branch.reshape(-1, d)
-    if h2.stride(-1) != 1:
-        h2 = h2.contiguous()
-    if b2.stride(-1) != 1:
-        b2 = b2.contiguous()
-    same = inplace and h2.data_ptr() == hidden.data_ptr()
-    h_out = h2 if same else torch.empty((h2.shape[0], d), dtype=hidden.dtype, device=hidden.device)
-    normed = torch.empty((h2.shape[0], d), dtype=hidden.dtype, device=hidden.device)
-    weight = weight.contiguous()
-    with torch.cuda.device(hidden.device):
-        nat.check(nat.lib().t5b_add_rmsnorm_fwd(h2.data_ptr(), b2.data_ptr(), weight.data_ptr(), h_out.data_ptr(),
-                                                normed.data_ptr(), h2.shape[0], d, h2.stride(0), b2.stride(0),
-                                                h_out.stride(0), normed.stride(0), nat.dtype_code(hidden.dtype),
-                                                nat.dtype_code(weight.dtype), float(eps),
-                                                nat.stream_ptr(hidden.device)), "add_rms_layer_norm")
-    return h_out.view(hidden.shape), normed.view(hidden.shape)
+    return _host.add_rmsnorm(hidden, branch, weight, eps, inplace)
 
 
 def gated_gelu(x: torch.Tensor) -> torch.Tensor:
     """gelu_tanh(x[..., :F]) * x[..., F:] for the output x of one matrix product with the
     concatenated wi_0 | wi_1 weights (T5DenseGatedActDense, src/turbot5/model/modeling.py:83-100).
     bf16/fp16, forward only."""
-    nat.require_cuda(x)
-    f2 = x.shape[-1]
-    if f2 % 2:
-        raise ValueError("the last dimension holds the two projections side by side")
-    x2 = x.reshape(-1, f2)
-    if x2.stride(-1) != 1:
-        x2 = x2.contiguous()
-    out = torch.empty((x2.shape[0], f2 // 2), dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        nat.check(nat.lib().t5b_gated_gelu_fwd(x2.data_ptr(), out.data_ptr(), x2.shape[0], f2 // 2, x2.stride(0),
-                                               out.stride(0), nat.dtype_code(x.dtype), nat.stream_ptr(x.device)),
-                  "gated_gelu")
-    return out.view(*x.shape[:-1], f2 // 2)
+    return _host.gated_gelu(x)
 
 
 class RMSLayerNorm:
