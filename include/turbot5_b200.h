@@ -277,6 +277,13 @@ T5B_API int t5b_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* 
                             int64_t dx_row_stride, int32_t x_dtype, int32_t w_dtype, float eps,
                             void* stream);
 
+/* The same with a gradient that reaches x on another way added to dx (the residual stream around the norm):
+ * dx = dx_add + gradient through the norm, one rounding.  dx_add has x's type and dx's row stride, may be
+ * dx itself, or NULL. */
+T5B_API int t5b_rmsnorm_bwd_add(const void* x, const void* w, const void* dy, const void* dx_add, void* dx, float* dw,
+                                int64_t rows, int32_t d, int64_t x_row_stride, int64_t dy_row_stride,
+                                int64_t dx_row_stride, int32_t x_dtype, int32_t w_dtype, float eps, void* stream);
+
 /* ---- merge of attention results over disjoint key ranges ---------------------------
  * out = sum_i w_i * part_out[i],  w_i = exp(part_lse[i] - max_j part_lse[j]) / sum: each part is
  * a forward call over its own slice of the keys (out_f32 set, lse requested, q_pos_offset shifted
@@ -321,6 +328,11 @@ T5B_API int t5b_add_rmsnorm_fwd(const void* hidden, const void* branch, const vo
  * aligned rows, row strides in elements. */
 T5B_API int t5b_gated_gelu_fwd(const void* x, void* out, int64_t rows, int32_t d_ff, int64_t x_stride,
                                int64_t out_stride, int32_t dtype, void* stream);
+
+/* Backward of t5b_gated_gelu_fwd: x as in the forward pass, dout (rows, d_ff), dx (rows, 2 * d_ff) written.
+ * Rounding points of autograd through the two separate operators. */
+T5B_API int t5b_gated_gelu_bwd(const void* x, const void* dout, void* dx, int64_t rows, int32_t d_ff, int64_t x_stride,
+                               int64_t dout_stride, int64_t dx_stride, int32_t dtype, void* stream);
 
 /* ---- unpad / pad glue -----------------------------------------------------------
  * Stand in for _get_unpad_data, index_first_axis and pad_input

@@ -278,3 +278,46 @@ def test_fused_encoder_decoder_forward_equals_the_module_passes():
     _, want = orc.t5_model_logits(w, {**TINY_T5, **over}, ids, dec)
     rel = lambda t: ((t.float().cpu() - want).abs().mean() / want.abs().mean()).item()
     assert rel(fused) < 1e-1 and rel(fused) <= 1.1 * rel(plain) + 1e-3
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,f", [(1, 8), (37, 264), (1000, 1024)])
+def test_gated_gelu_backward_vs_autograd(rows, f, dt):
+    """Against float32 autograd of gelu_tanh(a) * b; two roundings of the result and one of gelu(a) or of
+    dout * b: 3 half-ulps of the type relative to the largest factor."""
+    from turbot5_b200 import _native as nat
+    x = seeded((rows, 2 * f), 1, dtype=dt)
+    dout = seeded((rows, f), 2, dtype=dt)
+    ref = x.float().requires_grad_(True)
+    (torch.nn.functional.gelu(ref[:, :f], approximate="tanh") * ref[:, f:]).backward(dout.float())
+    dx = torch.empty((rows, 2 * f), dtype=dt, device="cuda")
+    xd, gd = x.cuda(), dout.cuda()
+    nat.check(nat.lib().t5b_gated_gelu_bwd(xd.data_ptr(), gd.data_ptr(), dx.data_ptr(), rows, f, 2 * f, f, 2 * f,
+                                           nat.dtype_code(dt), nat.stream_ptr(dx.device)), "gated_gelu_bwd")
+    torch.cuda.synchronize()
+    ulp = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    err = (dx.float().cpu() - ref.grad).abs()
+    assert (err <= 3 * ulp * ref.grad.abs() + 2 * ulp * 1e-2).all(), err.max().item()
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,d", [(1, 512), (5, 768), (3000, 768), (20000, 1024), (33, 520)])
+def test_rmsnorm_backward_with_a_residual_gradient(rows, d, dt):
+    """dx = add + gradient through the norm, in place; dw: both against float32 autograd (the weight gradient
+    is a sum over rows of products with the rounded normalised value: relative to its norm)."""
+    from turbot5_b200 import _native as nat
+    x, dy, add = seeded((rows, d), 1, dtype=dt), seeded((rows, d), 2, dtype=dt), seeded((rows, d), 3, dtype=dt)
+    w = (1 + seeded((d,), 4, 0.1)).to(dt)
+    xr, wr = x.float().requires_grad_(True), w.float().requires_grad_(True)
+    (wr * xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-6)).backward(dy.float())
+    want = xr.grad + add.float()
+    dx, dw = add.cuda(), torch.zeros(d, device="cuda")
+    xd, wd, gd = x.cuda(), w.cuda(), dy.cuda()
+    nat.check(nat.lib().t5b_rmsnorm_bwd_add(xd.data_ptr(), wd.data_ptr(), gd.data_ptr(), dx.data_ptr(), dx.data_ptr(),
+                                            dw.data_ptr(), rows, d, d, d, d, nat.dtype_code(dt), nat.dtype_code(dt), 1e-6,
+                                            nat.stream_ptr(dx.device)), "rmsnorm_bwd_add")
+    torch.cuda.synchronize()
+    ulp = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    err = (dx.float().cpu() - want).abs()
+    assert (err <= ulp * want.abs() + ulp * 1e-2).all(), err.max().item()
+    assert (dw.cpu() - wr.grad).norm() <= 2 * ulp * wr.grad.norm()

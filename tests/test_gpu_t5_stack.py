@@ -237,3 +237,42 @@ def test_local_encoder_matches_the_full_encoder_when_one_block_covers_everything
         b = local.encoder(ids)
     assert a.shape == b.shape and torch.isfinite(b.float()).all()
     assert (a.float() - b.float()).abs().max().item() > 1e-3
+
+
+@pytest.mark.parametrize("ff,masked,dtype", [("gated-gelu", False, torch.bfloat16), ("gated-gelu", True, torch.bfloat16),
+                                             ("relu", True, torch.float16)])
+def test_native_training_pass_gradients_equal_the_module_path(ff, masked, dtype):
+    """The whole stack as one autograd node (packed when the batch is padded) against the same weights run
+    module by module (a hook on one module selects that path).  Both round every activation and gradient to
+    the 16-bit type at the same points up to the order of sums: a few 2^-8 (bf16) of each tensor's norm.
+    The fixture's unit-variance weights make every softmax one-hot, and there a bf16 run's gradients differ
+    from the float32 run's by more than their norm whichever path computes them; at 0.3 of them both paths
+    are within 1.2 % of float32, and a sum or difference of two such runs within 4 %."""
+    model = _model(dtype, d_model=256, num_heads=4, d_ff=192, feed_forward_proj=ff).train()
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if p.dim() > 1 and "shared" not in n:
+                p.mul_(0.3)
+    g = torch.Generator().manual_seed(21)
+    B, L, Ld = 3, 150, 37
+    ids, dec = torch.randint(0, 128, (B, L), generator=g).cuda(), torch.randint(0, 128, (B, Ld), generator=g).cuda()
+    mask = None
+    if masked:
+        lens = torch.tensor([150, 61, 1])
+        mask = (torch.arange(L)[None] < lens[:, None]).long().cuda()
+    dout = torch.randn((B, Ld, 128), generator=g).to("cuda", dtype)
+
+    def grads():
+        model.zero_grad(set_to_none=True)
+        logits = model(ids, dec, attention_mask=mask)
+        logits.backward(dout)
+        return logits.detach(), {n: p.grad.float() for n, p in model.named_parameters()}
+    got_out, got = grads()
+    handle = model.encoder.block[0].layer[0].SelfAttention.q.register_forward_hook(lambda *a: None)
+    handle2 = model.decoder.block[0].layer[0].SelfAttention.q.register_forward_hook(lambda *a: None)
+    want_out, want = grads()
+    handle.remove(); handle2.remove()
+    rel = lambda a, b: ((a - b).norm() / b.norm().clamp_min(1e-6)).item()
+    assert rel(got_out.float(), want_out.float()) < 2e-2
+    for n in want:
+        assert rel(got[n], want[n]) < 4e-2, (n, rel(got[n], want[n]))

@@ -18,7 +18,7 @@ SOURCES = ["api.cu", "bucket.cu", "attn_fwd_sm100.cu", "attn_fwd2_sm100.cu", "at
            "rmsnorm.cu", "padding.cu", "fused_ops.cu"]
 HOST = os.path.join(CSRC, "host")
 HOST_LIB = os.path.join(HERE, "_host.so")
-HOST_SOURCES = ["ops.cpp"]
+HOST_SOURCES = ["ops.cpp", "stack.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 
@@ -64,7 +64,7 @@ def _host_flags():
            "/usr/local/cuda/include", sysconfig.get_paths()["include"]]
     compile_flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", *("-I" + i for i in inc)]
     link_flags = ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
-                  "-lc10_cuda", "-L/usr/local/cuda/lib64", "-lcudart", "-L" + HERE, "-l:libturbot5_b200.so",
+                  "-lc10_cuda", "-L/usr/local/cuda/lib64", "-lcudart", "-lcublas", "-L" + HERE, "-l:libturbot5_b200.so",
                   "-Wl,-rpath,$ORIGIN"]
     return compile_flags, link_flags
 

@@ -214,6 +214,50 @@ gated_gelu_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows, in
   }
 }
 
+// Gradient of the gated GELU: with a | b the two halves of x and g = round(gelu(a)),
+//   db = dout * g,  da = round(dout * b) * gelu'(a),
+//   gelu'(a) = s + a s (1 - s) (2u)',  s = sigmoid(2u),  (2u)' = 1.5957691 (1 + 0.134145 a^2)
+// (the roundings are those of autograd through the activation and the product as separate operators).
+// Bound by HBM like the forward: three rows read, two written.
+__device__ __forceinline__ void gelu_tanh_grad(float a, float& g, float& dg) {
+  const float u2 = 1.5957691216057308f * a * fmaf(0.044715f * a, a, 1.f);
+  const float s = __frcp_rn(1.f + fast_exp2(-u2 * kLog2e));
+  g = a * s;
+  dg = fmaf(g * (1.f - s), 1.5957691216057308f * fmaf(0.134145f * a, a, 1.f), s);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+gated_gelu_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dout, T* __restrict__ dx, int64_t rows, int f,
+                      int64_t xs, int64_t gs, int64_t ds) {
+  const int lane = threadIdx.x & 31;
+  const int nvec = f / 8;
+  const int64_t warp_id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t row = warp_id; row < rows; row += n_warps) {
+    const T* xr = x + row * xs;
+    for (int v = lane; v < nvec; v += 32) {
+      const uint4 a4 = ld16(xr + v * 8), b4 = ld16(xr + f + v * 8), g4 = ld16(dout + row * gs + v * 8);
+      const T* ea = reinterpret_cast<const T*>(&a4);
+      const T* eb = reinterpret_cast<const T*>(&b4);
+      const T* eg = reinterpret_cast<const T*>(&g4);
+      uint4 da4, db4;
+      T* oa = reinterpret_cast<T*>(&da4);
+      T* ob = reinterpret_cast<T*>(&db4);
+      #pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float g, dg;
+        gelu_tanh_grad(to_float<T>(ea[k]), g, dg);
+        const float go = to_float<T>(eg[k]);
+        ob[k] = from_float<T>(go * to_float<T>(from_float<T>(g)));
+        oa[k] = from_float<T>(to_float<T>(from_float<T>(go * to_float<T>(eb[k]))) * dg);
+      }
+      *reinterpret_cast<uint4*>(dx + row * ds + v * 8) = da4;
+      *reinterpret_cast<uint4*>(dx + row * ds + f + v * 8) = db4;
+    }
+  }
+}
+
 // ---------------------------------------------------------------- merge of attention partials
 constexpr int kMaxParts = T5B_MERGE_MAX_PARTS;
 
@@ -339,6 +383,27 @@ extern "C" int t5b_gated_gelu_fwd(const void* x, void* out, int64_t rows, int32_
     const int64_t blocks = balanced_blocks((rows + 7) / 8, resident_blocks(kern, 256, per_sm));
     kern<<<(unsigned)blocks, 256, 0, st>>>((const __half*)x, (__half*)out, rows, d_ff, x_stride, out_stride);
   }
+  return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
+}
+
+extern "C" int t5b_gated_gelu_bwd(const void* x, const void* dout, void* dx, int64_t rows, int32_t d_ff, int64_t x_stride,
+                                  int64_t dout_stride, int64_t dx_stride, int32_t dtype, void* stream) {
+  if (rows < 0 || d_ff <= 0) return T5B_ERR_SHAPE;
+  if (rows == 0) return T5B_OK;
+  if (!x || !dout || !dx) return T5B_ERR_ARG;
+  if (dtype != T5B_BF16 && dtype != T5B_F16) return T5B_ERR_DTYPE;
+  if (d_ff % 8 != 0) return T5B_ERR_SHAPE;
+  if ((((uintptr_t)x | (uintptr_t)dout | (uintptr_t)dx) & 15) != 0 || ((x_stride | dout_stride | dx_stride) % 8) != 0) return T5B_ERR_ALIGN;
+  cudaStream_t st = (cudaStream_t)stream;
+  using namespace t5b::fused;
+#define T5B_GGB(T) do { \
+    auto kern = gated_gelu_bwd_kernel<T>; \
+    static std::atomic<int> per_sm{0}; \
+    const int64_t blocks = balanced_blocks((rows + 7) / 8, resident_blocks(kern, 256, per_sm)); \
+    kern<<<(unsigned)blocks, 256, 0, st>>>((const T*)x, (const T*)dout, (T*)dx, rows, d_ff, x_stride, dout_stride, dx_stride); } while (0)
+  if (dtype == T5B_BF16) T5B_GGB(__nv_bfloat16);
+  else T5B_GGB(__half);
+#undef T5B_GGB
   return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
 }
 

@@ -5,12 +5,13 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
-#include <torch/csrc/utils/python_numbers.h>
 
 #include <cmath>
 #include <map>
 #include <mutex>
 #include <tuple>
+
+#include "bindings.h"
 
 namespace t5b_host {
 
@@ -580,44 +581,6 @@ Tensor rows_op(const Tensor& x, const Tensor& dest, int64_t batch, int64_t seqle
 }
 
 // ------------------------------------------------------------------ Python bindings
-Tensor tensor_arg(PyObject* o) {
-  if (o == Py_None) return Tensor();
-  TORCH_CHECK_TYPE(THPVariable_Check(o), "expected a tensor, got ", Py_TYPE(o)->tp_name);
-  return THPVariable_Unpack(o);
-}
-int64_t int_arg(PyObject* o) {
-  if (PyLong_Check(o)) return (int64_t)PyLong_AsLongLong(o);
-  PyObject* n = PyNumber_Long(o);
-  if (!n) throw python_error();
-  const int64_t v = (int64_t)PyLong_AsLongLong(n);
-  Py_DECREF(n);
-  return v;
-}
-double float_arg(PyObject* o) {
-  const double v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) throw python_error();
-  return v;
-}
-bool bool_arg(PyObject* o) {
-  if (o == Py_True) return true;
-  if (o == Py_False || o == Py_None) return false;
-  const int v = PyObject_IsTrue(o);
-  if (v < 0) throw python_error();
-  return v != 0;
-}
-std::optional<int64_t> opt_int(PyObject* o) { return o == Py_None ? std::nullopt : std::optional<int64_t>(int_arg(o)); }
-PyObject* wrap(const Tensor& t) {
-  if (!t.defined()) Py_RETURN_NONE;
-  return THPVariable_Wrap(t);
-}
-PyObject* wrap2(const Tensor& a, const Tensor& b) {
-  PyObject* r = PyTuple_New(2);
-  PyTuple_SET_ITEM(r, 0, wrap(a));
-  PyTuple_SET_ITEM(r, 1, wrap(b));
-  return r;
-}
-void expect(Py_ssize_t got, Py_ssize_t want) { TORCH_CHECK_TYPE(got == want, "expected ", want, " arguments, got ", got); }
-
 // attention(q, k, v, bias, causal, sm_scale, nb, md, q_pos_offset, return_lse, kernel, balance, local_block, window, out_f32)
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -780,7 +743,6 @@ PyObject* py_scratch_items(PyObject*, PyObject* const*, Py_ssize_t) {
   END_HANDLE_TH_ERRORS
 }
 
-#define T5B_METHOD(name, fn) {name, (PyCFunction)(void (*)(void))fn, METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     T5B_METHOD("attention", py_attention), T5B_METHOD("attention_packed", py_attention_packed),
     T5B_METHOD("decode", py_decode), T5B_METHOD("merge", py_merge), T5B_METHOD("rmsnorm", py_rmsnorm),
@@ -794,4 +756,8 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Native host side of the 
 }  // namespace
 }  // namespace t5b_host
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&t5b_host::kModule); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&t5b_host::kModule);
+  if (m && PyModule_AddFunctions(m, t5b_host::stack_methods) < 0) { Py_DECREF(m); return nullptr; }
+  return m;
+}

@@ -180,7 +180,7 @@ namespace rms {
 template <typename TX, typename TW, typename TDY>
 __global__ void __launch_bounds__(256)
 rmsnorm_bwd_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const TDY* __restrict__ dy,
-                   TX* __restrict__ dx, float* __restrict__ dw, int64_t rows, int d,
+                   const TX* dx_add, TX* dx, float* __restrict__ dw, int64_t rows, int d,
                    int64_t x_stride, int64_t dy_stride, int64_t dx_stride, float eps) {
   extern __shared__ float s_dw[];
   for (int c = threadIdx.x; c < d; c += blockDim.x) s_dw[c] = 0.f;
@@ -209,7 +209,8 @@ rmsnorm_bwd_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const TDY
     for (int c = lane; c < d; c += 32) {
       const float xv = to_float(xr[c]);
       const float gv = to_float(gr[c]);
-      dxr[c] = from_float<TX>(rstd * to_float(w[c]) * gv - xv * k);
+      const float other = dx_add ? to_float(dx_add[r * dx_stride + c]) : 0.f;
+      dxr[c] = from_float<TX>(rstd * to_float(w[c]) * gv - xv * k + other);
       const float xhat = to_float(from_float<TW>(xv * rstd));     // as the forward rounds it
       atomicAdd(&s_dw[c], gv * xhat);
     }
@@ -224,17 +225,19 @@ rmsnorm_bwd_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const TDY
 // d = 256 * NT, 16-bit x and dy, 16-byte aligned rows: a lane owns 8 consecutive columns of every
 // 256-column group, reads them with one 16-byte load, keeps the row in registers between the two
 // reductions and the outputs, and carries its share of the weight gradient in registers over all
-// the rows of its warp (one shared-memory add per column and warp at the end).
+// the rows of its warp.  Bound by HBM at large row counts (dx = add + ...: three rows read, one
+// written); a few thousand rows are bound by the end of a block, so the eight warps leave their
+// sums in shared memory side by side and one addition per column and block goes to the result
+// (adding into one shared row with atomics retries eight-fold: 8.3 us against 4.4 us on average over the
+// norms of a training step of 512-wide rows, 512 to 4096 of them).
 template <typename TX, typename TW, int NT>
 __global__ void __launch_bounds__(256)
 rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const TX* __restrict__ dy,
-                       TX* __restrict__ dx, float* __restrict__ dw, int64_t rows,
+                       const TX* dx_add, TX* dx, float* __restrict__ dw, int64_t rows,
                        int64_t x_stride, int64_t dy_stride, int64_t dx_stride, float eps) {
   constexpr int D = 256 * NT;
-  __shared__ float s_dw[D];
-  for (int c = threadIdx.x; c < D; c += blockDim.x) s_dw[c] = 0.f;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
+  __shared__ float s_dw[8][D];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   float wv[NT][8], acc[NT][8];
@@ -244,11 +247,14 @@ rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const
     for (int k = 0; k < 8; ++k) { wv[t][k] = to_float(w[t * 256 + lane * 8 + k]); acc[t][k] = 0.f; }
   for (int64_t r = warp0; r < rows; r += n_warps) {
     float xv[NT][8], gv[NT][8];
+    uint4 add[NT];
     float ss = 0.f, sg = 0.f;
     #pragma unroll
     for (int t = 0; t < NT; ++t) {
       const uint4 xa = ld_stream16(x + r * x_stride + t * 256 + lane * 8);
       const uint4 ga = ld_stream16(dy + r * dy_stride + t * 256 + lane * 8);
+      add[t] = make_uint4(0, 0, 0, 0);
+      if (dx_add) add[t] = *reinterpret_cast<const uint4*>(dx_add + r * dx_stride + t * 256 + lane * 8);
       const TX* xe = reinterpret_cast<const TX*>(&xa);
       const TX* ge = reinterpret_cast<const TX*>(&ga);
       #pragma unroll
@@ -270,9 +276,10 @@ rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const
     for (int t = 0; t < NT; ++t) {
       uint4 oa;
       TX* oe = reinterpret_cast<TX*>(&oa);
+      const TX* ae = reinterpret_cast<const TX*>(&add[t]);
       #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        oe[k] = from_float<TX>(rstd * wv[t][k] * gv[t][k] - xv[t][k] * kk);
+        oe[k] = from_float<TX>(rstd * wv[t][k] * gv[t][k] - xv[t][k] * kk + to_float(ae[k]));
         const float xhat = to_float(from_float<TW>(xv[t][k] * rstd));
         acc[t][k] = fmaf(gv[t][k], xhat, acc[t][k]);
       }
@@ -282,26 +289,32 @@ rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const
   #pragma unroll
   for (int t = 0; t < NT; ++t)
     #pragma unroll
-    for (int k = 0; k < 8; ++k) atomicAdd(&s_dw[t * 256 + lane * 8 + k], acc[t][k]);
+    for (int k = 0; k < 8; k += 4)
+      *reinterpret_cast<float4*>(&s_dw[warp][t * 256 + lane * 8 + k]) =
+          make_float4(acc[t][k], acc[t][k + 1], acc[t][k + 2], acc[t][k + 3]);
   __syncthreads();
   for (int c = threadIdx.x; c < D; c += blockDim.x) {
-    const float g = s_dw[c];
+    float g = 0.f;
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) g += s_dw[k][c];
     if (g != 0.f) atomicAdd(&dw[c], g);
   }
 }
 
 template <typename TX, typename TW, typename TDY>
-int launch_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, int64_t rows, int d,
+int launch_bwd(const void* x, const void* w, const void* dy, const void* dx_add, void* dx, float* dw, int64_t rows, int d,
                int64_t xs, int64_t dys, int64_t dxs, float eps, cudaStream_t st) {
   if constexpr (sizeof(TX) == 2 && std::is_same<TX, TDY>::value) {
     const bool aligned = ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0) && ((uintptr_t)dx % 16 == 0) &&
                          xs % 8 == 0 && dys % 8 == 0 && dxs % 8 == 0;
     if (aligned && (d == 512 || d == 768 || d == 1024)) {
-      int64_t nblk = (rows + 7) / 8;
+      // four rows per warp before a second block joins an SM (every block costs one atomic per column)
+      int64_t nblk = (rows + 31) / 32;
+      if (nblk < 148) nblk = (rows + 7) / 8 < 148 ? (rows + 7) / 8 : 148;
       if (nblk > 148 * 4) nblk = 148 * 4;
 #define T5B_RMSB_VEC(NT)                                                                            \
       rmsnorm_bwd_vec_kernel<TX, TW, NT><<<(unsigned)nblk, 256, 0, st>>>(                               \
-          (const TX*)x, (const TW*)w, (const TX*)dy, (TX*)dx, dw, rows, xs, dys, dxs, eps)
+          (const TX*)x, (const TW*)w, (const TX*)dy, (const TX*)dx_add, (TX*)dx, dw, rows, xs, dys, dxs, eps)
       if (d == 512) T5B_RMSB_VEC(2); else if (d == 768) T5B_RMSB_VEC(3); else T5B_RMSB_VEC(4);
 #undef T5B_RMSB_VEC
       return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
@@ -317,7 +330,7 @@ int launch_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw
   }
   int64_t blocks = (rows + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  kern<<<(unsigned)blocks, 256, smem, st>>>((const TX*)x, (const TW*)w, (const TDY*)dy, (TX*)dx, dw, rows, d,
+  kern<<<(unsigned)blocks, 256, smem, st>>>((const TX*)x, (const TW*)w, (const TDY*)dy, (const TX*)dx_add, (TX*)dx, dw, rows, d,
                                             xs, dys, dxs, eps);
   return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
 }
@@ -325,7 +338,7 @@ int launch_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw
 }  // namespace rms
 }  // namespace t5b
 
-extern "C" int t5b_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw,
+extern "C" int t5b_rmsnorm_bwd_add(const void* x, const void* w, const void* dy, const void* dx_add, void* dx, float* dw,
                                int64_t rows, int32_t d, int64_t x_row_stride, int64_t dy_row_stride,
                                int64_t dx_row_stride, int32_t x_dtype, int32_t w_dtype, float eps, void* stream) {
   using namespace t5b;
@@ -336,7 +349,7 @@ extern "C" int t5b_rmsnorm_bwd(const void* x, const void* w, const void* dy, voi
   // dy has the type of the forward's output: w's type when w is 16-bit, float32 otherwise
 #define T5B_RMSB(TXE, TX, TWE, TW, TDY)                                                       \
   if (x_dtype == TXE && w_dtype == TWE)                                                      \
-    return rms::launch_bwd<TX, TW, TDY>(x, w, dy, dx, dw, rows, d, x_row_stride, dy_row_stride, dx_row_stride, eps, st);
+    return rms::launch_bwd<TX, TW, TDY>(x, w, dy, dx_add, dx, dw, rows, d, x_row_stride, dy_row_stride, dx_row_stride, eps, st);
   T5B_RMSB(T5B_BF16, __nv_bfloat16, T5B_BF16, __nv_bfloat16, __nv_bfloat16)
   T5B_RMSB(T5B_BF16, __nv_bfloat16, T5B_F32, float, float)
   T5B_RMSB(T5B_F16, __half, T5B_F16, __half, __half)
@@ -346,6 +359,13 @@ extern "C" int t5b_rmsnorm_bwd(const void* x, const void* w, const void* dy, voi
   T5B_RMSB(T5B_F32, float, T5B_F16, __half, __half)
 #undef T5B_RMSB
   return T5B_ERR_DTYPE;
+}
+
+extern "C" int t5b_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw,
+                               int64_t rows, int32_t d, int64_t x_row_stride, int64_t dy_row_stride,
+                               int64_t dx_row_stride, int32_t x_dtype, int32_t w_dtype, float eps, void* stream) {
+  return t5b_rmsnorm_bwd_add(x, w, dy, nullptr, dx, dw, rows, d, x_row_stride, dy_row_stride, dx_row_stride, x_dtype, w_dtype,
+                             eps, stream);
 }
 
 extern "C" int t5b_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int64_t rows,

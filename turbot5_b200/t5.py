@@ -24,10 +24,14 @@ from typing import List, Optional
 import torch
 from torch import nn
 
-from .attention import (flash_attention_with_fusing_bias, flash_attention_with_fusing_bias_varlen,
-                        flash_decoding_with_fusing_bias)
+from . import _native as nat
+from .attention import flash_attention_with_fusing_bias, flash_decoding_with_fusing_bias
 from .modules import (T5ATTENTION_TYPES, T5FlashAttention, T5LayerNorm, add_rms_layer_norm, gated_gelu,
                       rms_layer_norm)
+from .padding import get_unpad_plan, pad_rows, unpad_rows
+
+_host = nat.host
+_HALF = (torch.bfloat16, torch.float16)
 
 
 @dataclass
@@ -136,6 +140,20 @@ class DecoderCache:
         self.max_len = max_len
 
 
+class _NativeState:
+    """What the native passes keep with a stack (stacked weights of the last inference pass).  Copies and
+    pickles of the module start without it."""
+
+    def __init__(self):
+        self.cache = _host.new_stack_cache()
+
+    def __deepcopy__(self, memo):
+        return _NativeState()
+
+    def __reduce__(self):
+        return _NativeState, ()
+
+
 class T5Stack(nn.Module):
     def __init__(self, cfg: T5StackConfig, embed_tokens: nn.Embedding, is_decoder: bool):
         super().__init__()
@@ -152,8 +170,15 @@ class T5Stack(nn.Module):
 
     def forward(self, input_ids=None, attention_mask=None, inputs_embeds=None, encoder_hidden_states=None,
                 encoder_attention_mask=None):
-        """Full (uncached) pass.  `attention_mask` is the raw 0/1 (B, L) mask or None."""
+        """Full (uncached) pass.  `attention_mask` is the raw 0/1 (B, L) mask or None.
+
+        A stack of 16-bit full-attention blocks runs as one native launch sequence (one autograd node in
+        training); everything else (float32, block-local attention, replaced modules, hooks) runs
+        module by module."""
         hidden = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
+        native = self._forward_native(hidden, attention_mask, encoder_hidden_states, encoder_attention_mask)
+        if native is not None:
+            return native
         table = self._table()
         for blk in self.block:
             sa = blk.layer[0]
@@ -167,6 +192,41 @@ class T5Stack(nn.Module):
                                                      key_value_states=encoder_hidden_states)[0]
             hidden = blk.layer[-1](hidden)
         return self.final_layer_norm(hidden).to(hidden.dtype)
+
+    def _forward_native(self, hidden, attention_mask, encoder_hidden_states, encoder_attention_mask):
+        """`forward` as one launch sequence, or None when this call is not one it covers."""
+        if self.is_decoder:
+            if encoder_hidden_states is None or encoder_hidden_states.dim() != 3:
+                return None
+            if encoder_attention_mask is None:
+                return self._run_native(hidden, enc=encoder_hidden_states)
+            if encoder_attention_mask.dim() != 2 or not hidden.is_cuda:
+                return None
+            plan = get_unpad_plan(encoder_attention_mask)
+            return self._run_native(hidden, enc=encoder_hidden_states, enc_cu=plan.cu_seqlens, enc_dest=plan.dest,
+                                    enc_max=plan.seqlen)
+        if attention_mask is None:
+            return self._run_native(hidden)
+        if attention_mask.dim() != 2 or not hidden.is_cuda:
+            return None
+        plan = get_unpad_plan(attention_mask)
+        return self._run_native(hidden, mode=2, cu=plan.cu_seqlens, dest=plan.dest, max_len=plan.seqlen)
+
+    def _run_native(self, x, mode=0, cu=None, dest=None, max_len=0, zero_tail=False, enc=None, enc_cu=None, enc_dest=None,
+                    enc_max=0, need_plain=True):
+        """One native pass over the rows x (B, S, d_model); modes as in csrc/host/stack.cpp.  None: not covered."""
+        if not x.is_cuda or x.dtype not in _HALF or torch.is_autocast_enabled():
+            return None
+        if need_plain and torch.nn.modules.module._has_any_global_hook():
+            return None
+        cfg = self.cfg
+        state = self.__dict__.get("_native_state")
+        if state is None:
+            state = self.__dict__["_native_state"] = _NativeState()
+        return _host.stack_forward(self, _STACK_CLASSES, state.cache, self.is_decoder, cfg.num_heads, cfg.d_kv,
+                                   cfg.relative_attention_num_buckets, cfg.relative_attention_max_distance,
+                                   cfg.layer_norm_epsilon, need_plain, x, mode, cu, dest, max_len, zero_tail, enc, enc_cu,
+                                   enc_dest, enc_max)
 
     # ---- inference pass of an encoder with the token-wise work fused around the attention path
     def _stacked_weights(self, i):
@@ -225,33 +285,81 @@ class T5Stack(nn.Module):
         gated_gelu, attention and the partial / merge pair of the sequence-parallel path): tests of
         the sharding logic on CPU ranks pass reference implementations.
         """
-        ops = ops or _FusedOps
-        cfg = self.cfg
         if self.is_decoder and (encoder_hidden_states is None or seq_len is not None):
             raise ValueError("a decoder stack needs encoder_hidden_states and is not sequence parallel")
         if (encoder_plan is not None) != (encoder_hidden_states is not None and encoder_hidden_states.dim() == 2):
             raise ValueError("packed encoder states (T, d_model) go together with encoder_plan")
-        x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
-        plan = None
+        if attention_mask is not None and (self.is_decoder or seq_len is not None):
+            raise ValueError("attention_mask is taken by unsharded encoder stacks")
+        for blk in self.block:
+            if type(blk.layer[0].SelfAttention) is not T5FlashAttention:
+                raise ValueError("forward_fused covers full attention (attention_type='flash')")
+        if seq_len is not None or ops is not None:
+            return self._forward_fused_ops(input_ids, inputs_embeds, seq_len, group, overlap, ops or _FusedOps,
+                                           encoder_hidden_states)
         if attention_mask is not None:
-            if self.is_decoder or seq_len is not None:
-                raise ValueError("attention_mask is taken by unsharded encoder stacks")
-            from .padding import get_unpad_plan, pad_rows, unpad_rows
-            plan = get_unpad_plan(attention_mask)
-            pad_shape = x.shape
-            n_valid = int(plan.cu_seqlens[-1]) if packed_rows is None else int(packed_rows)
-            n_valid = min(max(n_valid, 1), pad_shape[0] * pad_shape[1])
-            x = unpad_rows(x, plan)[:n_valid].unsqueeze(0)                  # (1, T, d_model): kept tokens, zero tail
+            return self._forward_fused_packed(input_ids, inputs_embeds, attention_mask, packed_rows, return_packed)
+        x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
+        if encoder_plan is None:
+            out = self._run_native(x, enc=encoder_hidden_states, need_plain=False)
+        else:
+            # packed encoder states: every decoder sequence has S query rows, its keys are the valid
+            # encoder tokens of the same batch row
+            if encoder_plan.batch != x.shape[0]:
+                raise ValueError("encoder_plan was made for another batch size")
+            out = self._run_native(x, enc=encoder_hidden_states, enc_cu=encoder_plan.cu_seqlens, enc_max=encoder_plan.seqlen,
+                                   need_plain=False)
+        if out is None:
+            raise NotImplementedError("forward_fused covers bf16/fp16 CUDA stacks (contiguous weights of one type, d_model "
+                                      "a multiple of 8 and at most 2048, head dim 16, 32, 64 or 128)")
+        return out
+
+    def _forward_fused_packed(self, input_ids, inputs_embeds, attention_mask, packed_rows, return_packed):
+        """The encoder pass over the valid tokens of a padded batch, packed once."""
+        plan = get_unpad_plan(attention_mask)
+        B, L = plan.batch, plan.seqlen
+        tail, cu = False, plan.cu_seqlens
+        if packed_rows is None:
+            # the valid tokens' ids (or rows) selected by the mask: the one read-back of the pass
+            src = input_ids if inputs_embeds is None else inputs_embeds
+            rows = src[attention_mask != 0]
+            if rows.shape[0] == 0:
+                rows, tail = src.flatten(0, 1)[:1], True
+            x = self.embed_tokens(rows) if inputs_embeds is None else rows
+        else:
             # With a caller's bound there may be rows past the last token.  The attention kernel does not
             # write them, and whatever the allocation held there must not reach a later matrix product
-            # as the value row of a masked key (0 x NaN): those rows are zeroed after every attention call.
-            tail_rows = None
-            cu_att = plan.cu_seqlens
-            if packed_rows is not None:
-                tail_rows = (torch.arange(n_valid, device=x.device) >= plan.cu_seqlens[-1])[:, None, None]
-                # no row past the buffers is ever touched, whatever the bound: the attention calls see the
-                # sequences cut at it (the result is then marked below)
-                cu_att = plan.cu_seqlens.clamp(max=n_valid)
+            # as the value row of a masked key (0 x NaN): the pass keeps them zero after attention.  No row past
+            # the buffers is ever touched, whatever the bound: the attention calls see the sequences cut
+            # at it (the result is then marked below).
+            n = min(max(int(packed_rows), 1), B * L)
+            x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
+            x = unpad_rows(x, plan)[:n]                                    # kept tokens, zero tail
+            tail, cu = True, plan.cu_seqlens.clamp(max=n)
+        normed = self._run_native(x.unsqueeze(0), mode=1, cu=cu, max_len=L, zero_tail=tail, need_plain=False)
+        if normed is None:
+            raise NotImplementedError("forward_fused covers bf16/fp16 CUDA stacks (contiguous weights of one type, d_model "
+                                      "a multiple of 8 and at most 2048, head dim 16, 32, 64 or 128)")
+        normed = normed[0]
+        n = normed.shape[0]
+        if packed_rows is not None:
+            # a bound below the true token count would silently drop tokens: make that loud (NaN
+            # everywhere) without reading anything back
+            normed = normed.masked_fill(plan.cu_seqlens[-1] > n, float("nan"))
+        if return_packed:
+            return normed, plan
+        if packed_rows is not None and n < B * L:
+            # the scatter reads the packed row of every valid token: give it all of them
+            full = normed.new_full((B * L, normed.shape[-1]), float("nan"))
+            full[:n] = normed
+            normed = full
+        return pad_rows(normed, plan)             # (B, L, d_model), zeros at padded positions
+
+    def _forward_fused_ops(self, input_ids, inputs_embeds, seq_len, group, overlap, ops, encoder_hidden_states):
+        """The fused pass operator by operator: sequence-parallel encoders (a collective per layer) and passes
+        with other operators than the library's."""
+        cfg = self.cfg
+        x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
         B, S, _ = x.shape
         H, D = cfg.num_heads, cfg.d_kv
         HD = H * D
@@ -259,28 +367,14 @@ class T5Stack(nn.Module):
         eps = cfg.layer_norm_epsilon
         table = self._table()
         heads = lambda t: t.unflatten(-1, (H, D)).transpose(1, 2)        # (B, L, H*D) -> (B, H, L, D) view
-        x = x.contiguous() if (inputs_embeds is None or plan is not None) else x.clone(memory_format=torch.contiguous_format)
+        x = x.contiguous() if inputs_embeds is None else x.clone(memory_format=torch.contiguous_format)
         normed = ops.rms_layer_norm(x, self.block[0].layer[0].layer_norm.weight, eps).to(x.dtype)
         if seq_len is not None:
             from . import sequence_parallel as sp
-        if encoder_plan is not None:
-            if encoder_plan.batch != B:
-                raise ValueError("encoder_plan was made for another batch size")
-            cu_dec = torch.arange(B + 1, dtype=torch.int32, device=x.device) * S
         for i, blk in enumerate(self.block):
             att, ffl = blk.layer[0].SelfAttention, blk.layer[-1]
-            if type(att) is not T5FlashAttention:
-                raise ValueError("forward_fused covers full attention (attention_type='flash')")
             w = self._stacked_weights(i)
-            if plan is not None:
-                qkv = nn.functional.linear(normed, w["qkv"])[0]                           # (T, 3*H*D)
-                q, k, v = (qkv[:, j * HD:(j + 1) * HD].unflatten(-1, (H, D)) for j in range(3))
-                attn = flash_attention_with_fusing_bias_varlen(q, k, v, table, cu_att, cu_att,
-                                                               plan.seqlen, plan.seqlen, causal=False, sm_scale=1.0,
-                                                               NUM_BUCKETS=nb, MAX_DISTANCE=md)
-                if tail_rows is not None:
-                    attn = attn.masked_fill(tail_rows, 0)
-            elif seq_len is None:
+            if seq_len is None:
                 qkv = nn.functional.linear(normed, w["qkv"])
                 q, k, v = (heads(qkv[..., j * HD:(j + 1) * HD]) for j in range(3))
                 attn = ops.attention(q, k, v, table, self.is_decoder, 1.0, nb, md, 0).transpose(1, 2)
@@ -302,17 +396,8 @@ class T5Stack(nn.Module):
                 x, normed = ops.add_rms_layer_norm(x, o, ca.layer_norm.weight, eps, inplace=True)
                 catt = ca.EncDecAttention
                 ckv = nn.functional.linear(encoder_hidden_states, w["ckv"])
-                if encoder_plan is None:
-                    q = heads(nn.functional.linear(normed, catt.q.weight))
-                    attn = ops.attention(q, heads(ckv[..., :HD]), heads(ckv[..., HD:]), None, False, 1.0, nb, md, 0)
-                    attn = attn.transpose(1, 2)
-                else:
-                    # packed encoder states: every decoder sequence has S query rows, its keys are the valid
-                    # encoder tokens of the same batch row
-                    q = nn.functional.linear(normed, catt.q.weight).view(B * S, H, D)
-                    attn = flash_attention_with_fusing_bias_varlen(
-                        q, ckv[:, :HD].unflatten(-1, (H, D)), ckv[:, HD:].unflatten(-1, (H, D)), None, cu_dec,
-                        encoder_plan.cu_seqlens, S, encoder_plan.seqlen, causal=False, sm_scale=1.0)
+                q = heads(nn.functional.linear(normed, catt.q.weight))
+                attn = ops.attention(q, heads(ckv[..., :HD]), heads(ckv[..., HD:]), None, False, 1.0, nb, md, 0).transpose(1, 2)
                 o = nn.functional.linear(attn.reshape(B, S, HD), catt.o.weight)
             x, normed = ops.add_rms_layer_norm(x, o, ffl.layer_norm.weight, eps, inplace=True)
             ff = ffl.DenseReluDense
@@ -322,19 +407,6 @@ class T5Stack(nn.Module):
                 f = ff(normed)
             nxt = self.block[i + 1].layer[0].layer_norm if i + 1 < len(self.block) else self.final_layer_norm
             x, normed = ops.add_rms_layer_norm(x, f, nxt.weight, eps, inplace=True)
-        if plan is not None:
-            if packed_rows is not None:
-                # a bound below the true token count would silently drop tokens: make that loud (NaN
-                # everywhere) without reading anything back
-                normed = normed.masked_fill(plan.cu_seqlens[-1] > S, float("nan"))
-            if return_packed:
-                return normed[0], plan
-            if packed_rows is not None and S < pad_shape[0] * pad_shape[1]:
-                # the scatter reads the packed row of every valid token: give it all of them
-                full = normed.new_full((pad_shape[0] * pad_shape[1], normed.shape[-1]), float("nan"))
-                full[:S] = normed[0]
-                return pad_rows(full, plan)
-            return pad_rows(normed[0], plan)          # (B, L, d_model), zeros at padded positions
         return normed
 
     # ---- generation with a preallocated cache (decoder only)
@@ -465,6 +537,11 @@ class T5Stack(nn.Module):
         return self.final_layer_norm(hidden).to(hidden.dtype)
 
 
+# the classes of a plain stack, in the order of `Kind` in csrc/host/stack.cpp
+_STACK_CLASSES = (T5Block, nn.ModuleList, T5LayerSelfAttention, T5LayerCrossAttention, T5LayerFF, T5FlashAttention,
+                  T5LayerNorm, nn.Linear, T5DenseGatedActDense, T5DenseActDense, nn.Embedding)
+
+
 class GraphedDecoding:
     """Greedy generation whose single-token step is one CUDA graph.
 
@@ -585,9 +662,31 @@ class T5ForConditionalGeneration(nn.Module):
             enc, plan = self.encoder.forward_fused(input_ids, attention_mask=attention_mask, return_packed=True)
             return self.logits(self.decoder.forward_fused(decoder_input_ids, encoder_hidden_states=enc,
                                                           encoder_plan=plan))
+        if attention_mask is not None:
+            dec = self._packed_training_pass(input_ids, decoder_input_ids, attention_mask)
+            if dec is not None:
+                return self.logits(dec)
         enc = self.encoder(input_ids, attention_mask=attention_mask)
         dec = self.decoder(decoder_input_ids, encoder_hidden_states=enc, encoder_attention_mask=attention_mask)
         return self.logits(dec)
+
+    def _packed_training_pass(self, input_ids, decoder_input_ids, attention_mask):
+        """Decoder states of a padded batch in training: the valid tokens are packed once (padded rows get no
+        gradient and give none), both stacks run as native passes and the cross attention reads the packed
+        encoder states.  None when the stacks are not ones the native passes cover."""
+        enc, dec = self.encoder, self.decoder
+        if not input_ids.is_cuda or self.shared.weight.dtype not in _HALF or self.cfg.attention_type != "flash" or \
+                attention_mask.shape != input_ids.shape or \
+                any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (enc, dec)):
+            return None
+        ids = input_ids[attention_mask != 0]             # the one read-back of the pass
+        if ids.shape[0] == 0:
+            return None
+        plan = get_unpad_plan(attention_mask)
+        states = enc._run_native(enc.embed_tokens(ids).unsqueeze(0), mode=1, cu=plan.cu_seqlens, max_len=plan.seqlen)
+        if states is None:
+            return None
+        return dec._run_native(dec.embed_tokens(decoder_input_ids), enc=states[0], enc_cu=plan.cu_seqlens, enc_max=plan.seqlen)
 
     @torch.no_grad()
     def forward_cuda_graph(self, input_ids, decoder_input_ids):
