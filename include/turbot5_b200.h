@@ -255,6 +255,47 @@ T5B_API int t5b_decode_fwd(const t5b_decode_args* args, void* stream);
 T5B_API int64_t t5b_decode_static_scratch_bytes(void);
 T5B_API int t5b_decode_fwd_static_scratch(const t5b_decode_args* args, void* stream);
 
+/* ---- one cached decoding step of a whole decoder ---------------------------------
+ * Stands in for a single-token step of the reference's decoder stack with its cache
+ * (src/turbot5/model/modeling.py:166-219, 352-632; src/turbot5/model/attentions.py:198,229-234), the LM head
+ * (src/turbot5/heads/t5_heads.py:132-260), the greedy choice and the embedding of the chosen token.
+ *
+ *   hidden   (B, d_model): in: the embedding of the current tokens; out: that of the chosen ones.
+ *   seqlens  int32 (B): cached keys of each row, the new token's included (1 at the first step); the step
+ *            appends key and value at seqlens - 1, writes the chosen token to tokens[row, seqlens - 1] and
+ *            adds one.
+ *   logits   (B, vocab), written.
+ *   Weights are row-major (out, in), contiguous, 16-byte aligned, of `dtype` (bf16 or fp16) like every
+ *   activation: wqkv = [q; k; v], wi = [wi_0; wi_1] when gated (GELU, tanh form), else one matrix (ReLU).
+ *   self_kv (2, B, H, max_len, D); cross_k / cross_v: element strides cross_stride_*, 16-byte aligned rows,
+ *   the first enc_seqlens[b] (int32, optional) or enc_len keys of each row.
+ *   table: causal (unidirectional) bias table of the self attention, read by t5b_decoder_step_prepare, which
+ *   has to run once on the workspace before the first step.  No 1/sqrt(D) (T5).
+ * B <= 64; d_model, H * D and d_ff multiples of 32, at most 2048, 4096 and 8192 (T5B_ERR_UNSUPPORTED
+ * otherwise).  Nothing in the launch sequence depends on values on the device: a step can be captured. */
+typedef struct {
+  const void* ln_self; const void* wqkv; const void* wo;
+  const void* ln_cross; const void* wcq; const void* wco;
+  const void* ln_ff; const void* wi; const void* wff;
+  void* self_kv; const void* cross_k; const void* cross_v;
+} t5b_decoder_layer;
+typedef struct {
+  const t5b_decoder_layer* layers;      /* host array */
+  const void* final_ln; const void* lm_head; const void* embedding; const void* table;
+  void* hidden; void* logits; int64_t* tokens; int32_t* seqlens; const int32_t* enc_seqlens;
+  void* workspace; int64_t workspace_bytes;
+  int64_t tokens_stride, table_stride0;
+  int64_t cross_stride_b, cross_stride_h, cross_stride_n;
+  int32_t dtype, table_dtype;
+  int32_t n_layers, B, H, D, d_model, d_ff, gated, vocab, max_len, enc_len;
+  int32_t num_buckets, max_distance;
+  float eps, lm_scale;                  /* lm_scale multiplies the normed states before the head (tied embeddings) */
+} t5b_decoder_step_args;
+
+T5B_API int64_t t5b_decoder_step_workspace_bytes(const t5b_decoder_step_args* args);
+T5B_API int t5b_decoder_step_prepare(const t5b_decoder_step_args* args, void* stream);
+T5B_API int t5b_decoder_step(const t5b_decoder_step_args* args, void* stream);
+
 /* ---- T5 RMSNorm, forward -------------------------------------------------------
  * Stands in for T5LayerNorm._forward (src/turbot5/model/modules.py:52-60) and
  * RMSLayerNorm.forward / rms_layer_norm_fwd_fused (src/turbot5/ops/rms_norm.py:

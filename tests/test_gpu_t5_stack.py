@@ -276,3 +276,54 @@ def test_native_training_pass_gradients_equal_the_module_path(ff, masked, dtype)
     assert rel(got_out.float(), want_out.float()) < 2e-2
     for n in want:
         assert rel(got[n], want[n]) < 4e-2, (n, rel(got[n], want[n]))
+
+
+@pytest.mark.parametrize("B,L,steps,over,dtype", [
+    (1, 7, 3, dict(), torch.bfloat16),                                             # one row, short memory: every split edge
+    (3, 300, 20, dict(feed_forward_proj="relu"), torch.bfloat16),
+    (17, 65, 5, dict(tie_word_embeddings=True), torch.bfloat16),                   # a second sixteen-row tile with one row
+    (64, 129, 4, dict(), torch.float16),                                           # the largest batch
+    (2, 200, 150, dict(d_model=1056, d_ff=2080, vocab_size=97), torch.bfloat16),   # rows over 1024, ragged vocabulary, split cache
+    (5, 400, 6, dict(d_kv=128, num_heads=2), torch.bfloat16),
+    (2, 90, 6, dict(d_kv=32, num_heads=3, d_ff=96), torch.bfloat16)])
+def test_native_decoding_steps_equal_the_uncached_pass(B, L, steps, over, dtype):
+    """Greedy decoding by the step kernels against the whole uncached decoder pass over the chosen tokens (other
+    kernels throughout): same logits at the last step, and every chosen token is the best of its step or
+    within the difference that two 16-bit passes show."""
+    model = _model(dtype, **{**dict(d_model=128, num_heads=4, d_ff=256), **over})
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if p.dim() > 1 and "shared" not in n:
+                p.mul_(p.shape[-1] ** -0.5)
+    g = torch.Generator().manual_seed(31)
+    enc = torch.randn((B, L, model.cfg.d_model), generator=g).to("cuda", dtype)
+    lens = torch.randint(1, L + 1, (B,), generator=g, dtype=torch.int32)
+    lens[0] = L
+    mask = (torch.arange(L)[None] < lens[:, None]).long().cuda()
+    from turbot5_b200.t5 import _native_decoding
+    with torch.no_grad():
+        assert _native_decoding(model, enc, steps, lens.cuda()) is not None
+        tokens, last = model.greedy_decode(enc, steps, encoder_seqlens=lens.cuda(), use_cuda_graph=True)
+        dec_in = torch.cat([torch.zeros((B, 1), dtype=torch.long, device="cuda"), tokens[:, :-1]], dim=1)
+        full = model.logits(model.decoder(dec_in, encoder_hidden_states=enc, encoder_attention_mask=mask)).float()
+    torch.cuda.synchronize()
+    scale = full.abs().mean().item()
+    assert (full[:, -1] - last[:, -1].float()).abs().max().item() < 0.08 * scale + 0.02
+    chosen = full.gather(-1, tokens[..., None])[..., 0]
+    assert (full.max(-1).values - chosen).max().item() < 0.08 * scale + 0.02
+
+
+def test_graphed_decoding_replays_the_native_step():
+    from turbot5_b200.t5 import GraphedDecoding
+    model = _model(torch.bfloat16, d_model=128, num_heads=4, d_ff=256)
+    enc = torch.randn((3, 200, 128), generator=torch.Generator().manual_seed(32)).cuda().bfloat16()
+    want, last = model.greedy_decode(enc, 9)
+    session = GraphedDecoding(model, enc, 9)
+    for _ in range(2):
+        session.rewind()
+        for _ in range(9):
+            session.step()
+        torch.cuda.synchronize()
+        assert torch.equal(session.tokens, want) and torch.equal(session.last_logits, last)
+    with pytest.raises(RuntimeError):
+        session.step()

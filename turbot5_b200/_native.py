@@ -26,6 +26,7 @@ _DTYPES = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
 SYMBOLS = ("t5b_status_string", "t5b_abi_version", "t5b_bucket_table_host", "t5b_bucket_indices",
            "t5b_attention_fwd", "t5b_attention_workspace_bytes", "t5b_attention_bwd", "t5b_attention_bwd_workspace_bytes", "t5b_decode_workspace_bytes", "t5b_decode_num_splits",
            "t5b_decode_fwd", "t5b_decode_static_scratch_bytes", "t5b_decode_fwd_static_scratch",
+           "t5b_decoder_step_workspace_bytes", "t5b_decoder_step_prepare", "t5b_decoder_step",
            "t5b_rmsnorm_fwd", "t5b_rmsnorm_bwd", "t5b_rmsnorm_bwd_add", "t5b_gated_gelu_bwd", "t5b_unpad_plan", "t5b_gather_rows",
            "t5b_scatter_rows", "t5b_attention_merge", "t5b_add_rmsnorm_fwd", "t5b_gated_gelu_fwd",
            "t5b_check_status", "t5b_selftest_bounded_wait")

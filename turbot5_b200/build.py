@@ -14,7 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libturbot5_b200.so")
-SOURCES = ["api.cu", "bucket.cu", "attn_fwd_sm100.cu", "attn_fwd2_sm100.cu", "attn_bwd_sm100.cu", "attn_fwd_simt.cu", "attn_bwd_simt.cu", "decode.cu",
+SOURCES = ["api.cu", "bucket.cu", "attn_fwd_sm100.cu", "attn_fwd2_sm100.cu", "attn_bwd_sm100.cu", "attn_fwd_simt.cu", "attn_bwd_simt.cu", "decode.cu", "decoder_step.cu",
            "rmsnorm.cu", "padding.cu", "fused_ops.cu"]
 HOST = os.path.join(CSRC, "host")
 HOST_LIB = os.path.join(HERE, "_host.so")

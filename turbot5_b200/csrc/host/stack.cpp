@@ -681,9 +681,151 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ------------------------------------------------------------------ greedy decoding
+// One generation: caches, weights and the argument block of t5b_decoder_step.
+struct DecodeSession {
+  Stack s;
+  std::shared_ptr<Stacked> w;
+  Tensor head, embedding, hidden, logits, tokens, seqlens, enc_seqlens, workspace;
+  std::vector<Tensor> self_kv, ckv;
+  std::vector<t5b_decoder_layer> layers;
+  t5b_decoder_step_args a = {};
+  int64_t start_token = 0;
+
+  void rewind() {
+    hidden.copy_(embedding.select(0, start_token).expand_as(hidden));
+    seqlens.fill_(1);
+  }
+  void step() { check_status(t5b_decoder_step(&a, stream_of(hidden.device())), "decoder step"); }
+};
+
+DecodeSession& session_arg(PyObject* o) {
+  auto* p = (DecodeSession*)PyCapsule_GetPointer(o, "t5b_decode_session");
+  if (!p) throw python_error();
+  return *p;
+}
+void free_session(PyObject* o) { delete (DecodeSession*)PyCapsule_GetPointer(o, "t5b_decode_session"); }
+
+// new_decode_session(stack, types, cache, heads, d_kv, buckets, max_distance, eps,
+//                    memory, enc_seqlens, max_len, lm_head weight, embedding weight, lm_scale, start_token)
+// None when the step kernels do not cover this decoder (types, sizes, replaced modules or hooks).
+PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 15);
+  auto ses = std::make_unique<DecodeSession>();
+  DecodeSession& d = *ses;
+  d.s = collect(a[0], a[1], true, int_arg(a[3]), int_arg(a[4]), (int)int_arg(a[5]), (int)int_arg(a[6]), float_arg(a[7]));
+  const Tensor memory = tensor_arg(a[8]);
+  d.enc_seqlens = tensor_arg(a[9]);
+  const int64_t max_len = int_arg(a[10]);
+  d.head = tensor_arg(a[11]); d.embedding = tensor_arg(a[12]);
+  d.start_token = int_arg(a[14]);
+  const Stack& s = d.s;
+  if (!s.plain || !memory.is_cuda() || memory.dim() != 3 || memory.size(2) != s.d || memory.numel() == 0 || max_len <= 0) Py_RETURN_NONE;
+  const at::ScalarType dt = memory.scalar_type();
+  auto plain = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == dt && t.is_contiguous() && t.dim() == 2 && t.size(1) == s.d; };
+  if (!supported(s, dt) || !plain(d.head) || !plain(d.embedding) || s.table.size(0) != s.nb) Py_RETURN_NONE;
+  if (d.start_token < 0 || d.start_token >= d.embedding.size(0) || d.head.size(0) > d.embedding.size(0)) Py_RETURN_NONE;
+  const int64_t B = memory.size(0), L = memory.size(1), HD = s.H * s.D;
+  if (d.enc_seqlens.defined()) {
+    if (!d.enc_seqlens.is_cuda() || d.enc_seqlens.scalar_type() != at::kInt || d.enc_seqlens.numel() != B) Py_RETURN_NONE;
+    d.enc_seqlens = d.enc_seqlens.contiguous();
+  }
+  const at::Device dev = memory.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  at::AutoGradMode no_grad(false);
+  t5b_decoder_step_args& k = d.a;
+  k.dtype = dtype_code(dt); k.table_dtype = dtype_code(s.table.scalar_type());
+  k.n_layers = (int32_t)s.layers.size(); k.B = (int32_t)B; k.H = (int32_t)s.H; k.D = (int32_t)s.D;
+  k.d_model = (int32_t)s.d; k.d_ff = (int32_t)s.F; k.gated = s.gated; k.vocab = (int32_t)d.head.size(0);
+  k.max_len = (int32_t)max_len; k.enc_len = (int32_t)L;
+  k.num_buckets = s.nb; k.max_distance = s.md;
+  k.eps = (float)s.eps; k.lm_scale = (float)float_arg(a[13]);
+  k.cross_stride_b = L * 2 * HD; k.cross_stride_n = 2 * HD; k.cross_stride_h = s.D;
+  d.workspace = empty_like_dense({t5b_decoder_step_workspace_bytes(&k)}, at::kByte, dev);
+  k.workspace = d.workspace.data_ptr(); k.workspace_bytes = d.workspace.numel();
+  k.table = s.table.data_ptr(); k.table_stride0 = s.table.stride(0);
+  d.layers.resize(s.layers.size());
+  k.layers = d.layers.data();
+  // sizes, bucket settings and head dims no step kernel takes show here, before anything is computed
+  const int st = t5b_decoder_step_prepare(&k, stream_of(dev));
+  if (st == T5B_ERR_UNSUPPORTED) Py_RETURN_NONE;
+  check_status(st, "decoder step");
+  auto* cache = (StackCache*)PyCapsule_GetPointer(a[2], "t5b_stack_cache");
+  if (!cache) throw python_error();
+  {
+    pybind11::gil_scoped_release nogil;
+    d.w = cached_weights(*cache, s);
+    d.hidden = empty_like_dense({B, s.d}, dt, dev);
+    d.logits = empty_like_dense({B, 1, d.head.size(0)}, dt, dev);
+    d.tokens = empty_like_dense({B, max_len}, at::kLong, dev);
+    zero_async(d.tokens);
+    d.seqlens = empty_like_dense({B}, at::kInt, dev);
+    k.hidden = d.hidden.data_ptr(); k.logits = d.logits.data_ptr(); k.tokens = d.tokens.data_ptr<int64_t>();
+    k.tokens_stride = max_len; k.seqlens = d.seqlens.data_ptr<int32_t>();
+    k.enc_seqlens = (const int32_t*)ptr(d.enc_seqlens);
+    k.final_ln = s.final_ln.data_ptr(); k.lm_head = d.head.data_ptr(); k.embedding = d.embedding.data_ptr();
+    const Tensor mem = memory.contiguous().view({B * L, s.d});
+    for (size_t i = 0; i < s.layers.size(); ++i) {
+      // cross keys and values of the layer, projected once: rows of k | v per memory token
+      d.ckv.push_back(new_rows(mem, B * L, 2 * HD));
+      linear(mem, d.w->ckv_of(i), d.ckv.back());
+      d.self_kv.push_back(empty_like_dense({2, B, s.H, max_len, s.D}, dt, dev));
+      const Layer& l = s.layers[i];
+      t5b_decoder_layer& o = d.layers[i];
+      o.ln_self = l.ln_self.data_ptr(); o.wqkv = d.w->qkv_of(i).data_ptr(); o.wo = l.o.data_ptr();
+      o.ln_cross = l.ln_cross.data_ptr(); o.wcq = l.cq.data_ptr(); o.wco = l.co.data_ptr();
+      o.ln_ff = l.ln_ff.data_ptr(); o.wi = d.w->wi_of(i, s).data_ptr(); o.wff = l.wo.data_ptr();
+      o.self_kv = d.self_kv.back().data_ptr();
+      o.cross_k = d.ckv.back().data_ptr();
+      o.cross_v = (const char*)d.ckv.back().data_ptr() + HD * 2;
+    }
+    d.rewind();
+  }
+  return PyCapsule_New(ses.release(), "t5b_decode_session", free_session);
+  END_HANDLE_TH_ERRORS
+}
+
+// decode_session_run(session, steps)
+PyObject* py_decode_session_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 2);
+  DecodeSession& d = session_arg(a[0]);
+  const int64_t steps = int_arg(a[1]);
+  const c10::cuda::CUDAGuard guard(d.hidden.device());
+  {
+    pybind11::gil_scoped_release nogil;
+    for (int64_t i = 0; i < steps; ++i) d.step();
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_decode_session_rewind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 1);
+  at::AutoGradMode no_grad(false);
+  session_arg(a[0]).rewind();
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// (tokens, logits) of the last step
+PyObject* py_decode_session_tensors(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 1);
+  DecodeSession& d = session_arg(a[0]);
+  return wrap2(d.tokens, d.logits);
+  END_HANDLE_TH_ERRORS
+}
+
 }  // namespace
 
 PyMethodDef stack_methods[] = {T5B_METHOD("stack_forward", py_stack_forward), T5B_METHOD("new_stack_cache", py_new_stack_cache),
+                               T5B_METHOD("new_decode_session", py_new_decode_session),
+                               T5B_METHOD("decode_session_run", py_decode_session_run),
+                               T5B_METHOD("decode_session_rewind", py_decode_session_rewind),
+                               T5B_METHOD("decode_session_tensors", py_decode_session_tensors),
                                {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace t5b_host

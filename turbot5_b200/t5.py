@@ -220,10 +220,7 @@ class T5Stack(nn.Module):
         if need_plain and torch.nn.modules.module._has_any_global_hook():
             return None
         cfg = self.cfg
-        state = self.__dict__.get("_native_state")
-        if state is None:
-            state = self.__dict__["_native_state"] = _NativeState()
-        return _host.stack_forward(self, _STACK_CLASSES, state.cache, self.is_decoder, cfg.num_heads, cfg.d_kv,
+        return _host.stack_forward(self, _STACK_CLASSES, self._native_cache(), self.is_decoder, cfg.num_heads, cfg.d_kv,
                                    cfg.relative_attention_num_buckets, cfg.relative_attention_max_distance,
                                    cfg.layer_norm_epsilon, need_plain, x, mode, cu, dest, max_len, zero_tail, enc, enc_cu,
                                    enc_dest, enc_max)
@@ -313,6 +310,12 @@ class T5Stack(nn.Module):
             raise NotImplementedError("forward_fused covers bf16/fp16 CUDA stacks (contiguous weights of one type, d_model "
                                       "a multiple of 8 and at most 2048, head dim 16, 32, 64 or 128)")
         return out
+
+    def _native_cache(self):
+        state = self.__dict__.get("_native_state")
+        if state is None:
+            state = self.__dict__["_native_state"] = _NativeState()
+        return state.cache
 
     def _forward_fused_packed(self, input_ids, inputs_embeds, attention_mask, packed_rows, return_packed):
         """The encoder pass over the valid tokens of a padded batch, packed once."""
@@ -542,14 +545,34 @@ _STACK_CLASSES = (T5Block, nn.ModuleList, T5LayerSelfAttention, T5LayerCrossAtte
                   T5LayerNorm, nn.Linear, T5DenseGatedActDense, T5DenseActDense, nn.Embedding)
 
 
+def _native_decoding(model, encoder_hidden_states, max_len, encoder_seqlens=None):
+    """A native decoding session for this model (caches, projected cross keys, one launch chain per token:
+    csrc/decoder_step.cu), or None when the step kernels do not cover it: float32, more than 64 rows, replaced
+    modules or hooks, sizes they do not take."""
+    dec, head, emb, cfg = model.decoder, model.lm_head, model.decoder.embed_tokens, model.cfg
+    plain = lambda m: not (m._forward_hooks or m._forward_pre_hooks)
+    if type(model).logits is not T5ForConditionalGeneration.logits or type(dec) is not T5Stack or \
+            type(head) is not nn.Linear or type(emb) is not nn.Embedding or head.bias is not None or \
+            emb.max_norm is not None or not (plain(head) and plain(emb) and plain(dec)) or \
+            torch.nn.modules.module._has_any_global_hook() or torch.is_autocast_enabled() or \
+            not encoder_hidden_states.is_cuda or encoder_hidden_states.dtype not in _HALF:
+        return None
+    scale = cfg.d_model ** -0.5 if cfg.tie_word_embeddings else 1.0
+    return _host.new_decode_session(dec, _STACK_CLASSES, dec._native_cache(), cfg.num_heads, cfg.d_kv,
+                                    cfg.relative_attention_num_buckets, cfg.relative_attention_max_distance,
+                                    cfg.layer_norm_epsilon, encoder_hidden_states, encoder_seqlens, max_len, head.weight,
+                                    emb.weight, scale, cfg.decoder_start_token_id)
+
+
 class GraphedDecoding:
     """Greedy generation whose single-token step is one CUDA graph.
 
     The step (all decoder layers, LM head, argmax, token write-back, position update) is run
     once eagerly on a side stream (cuBLAS handles and stacked weights then exist), rewound,
-    captured, and rewound again; `step()` then replays it.  The library's split scratch is kept
-    per stream: the capture stream gets its own, allocated and zeroed inside the graph's memory
-    pool during capture.  The token position and the cached
+    captured, and rewound again; `step()` then replays it.  Where the native step kernels cover the
+    model the captured step is their launch chain; otherwise it is `decode_step_static`, whose split
+    scratch is kept per stream: the capture stream gets its own, allocated and zeroed inside the
+    graph's memory pool during capture.  The token position and the cached
     length live in device tensors that the graph itself advances, so no launch argument
     changes between replays.
     """
@@ -559,13 +582,18 @@ class GraphedDecoding:
         dev = encoder_hidden_states.device
         self.model = model
         self.max_len = max_len
-        self.cache = model.decoder.new_cache(encoder_hidden_states, max_len)
-        self.cur = torch.empty((B, 1), dtype=torch.long, device=dev)
-        self.pos = torch.empty(1, dtype=torch.long, device=dev)
-        self.seqlens = torch.empty(B, dtype=torch.int32, device=dev)
-        self.tokens = torch.zeros((B, max_len), dtype=torch.long, device=dev)
-        self.encoder_seqlens = encoder_seqlens
         self.steps_done = 0
+        self.encoder_seqlens = encoder_seqlens
+        with torch.no_grad():
+            self.session = _native_decoding(model, encoder_hidden_states, max_len, encoder_seqlens)
+        if self.session is not None:
+            self.tokens, self.last_logits = _host.decode_session_tensors(self.session)
+        else:
+            self.cache = model.decoder.new_cache(encoder_hidden_states, max_len)
+            self.cur = torch.empty((B, 1), dtype=torch.long, device=dev)
+            self.pos = torch.empty(1, dtype=torch.long, device=dev)
+            self.seqlens = torch.empty(B, dtype=torch.int32, device=dev)
+            self.tokens = torch.zeros((B, max_len), dtype=torch.long, device=dev)
         self.rewind()
         side = torch.cuda.Stream(dev)
         side.wait_stream(torch.cuda.current_stream(dev))
@@ -579,12 +607,18 @@ class GraphedDecoding:
         self.rewind()
 
     def rewind(self):
-        self.cur.fill_(self.model.cfg.decoder_start_token_id)
-        self.pos.zero_()
-        self.seqlens.fill_(1)
+        if self.session is not None:
+            _host.decode_session_rewind(self.session)
+        else:
+            self.cur.fill_(self.model.cfg.decoder_start_token_id)
+            self.pos.zero_()
+            self.seqlens.fill_(1)
         self.steps_done = 0
 
     def _step(self):
+        if self.session is not None:
+            _host.decode_session_run(self.session, 1)
+            return self.last_logits
         m = self.model
         logits = m.logits(m.decoder.decode_step_static(self.cur, self.cache, self.pos, self.seqlens,
                                                        self.encoder_seqlens))
@@ -720,23 +754,26 @@ class T5ForConditionalGeneration(nn.Module):
     def greedy_decode(self, encoder_hidden_states, steps, encoder_seqlens=None, use_cuda_graph=False):
         """Greedy generation from `decoder_start_token_id` with the preallocated cache.
 
-        With `use_cuda_graph` the whole single-token step (all layers, LM head, argmax, position
-        update) is captured once after a warm-up step and replayed: one graph launch per token
-        instead of a few hundred kernel launches issued from Python.
+        Where the native step kernels cover the model (16-bit plain stacks, up to 64 rows) every token is one
+        native launch chain.  Otherwise, with `use_cuda_graph`, the whole single-token step (all layers, LM
+        head, argmax, position update) is captured once after a warm-up step and replayed: one graph
+        launch per token instead of a few hundred kernel launches issued from Python.
         """
-        B = encoder_hidden_states.shape[0]
-        dev = encoder_hidden_states.device
-        cache = self.decoder.new_cache(encoder_hidden_states, steps)
-        cur = torch.full((B, 1), self.cfg.decoder_start_token_id, dtype=torch.long, device=dev)
-        if not use_cuda_graph:
-            tokens, last_logits = [], None
+        session = _native_decoding(self, encoder_hidden_states, steps, encoder_seqlens)
+        if session is not None:
+            _host.decode_session_run(session, steps)
+            return _host.decode_session_tensors(session)
+        if use_cuda_graph:
+            session = GraphedDecoding(self, encoder_hidden_states, steps, encoder_seqlens)
             for _ in range(steps):
-                last_logits = self.logits(self.decoder.decode_step(cur, cache, encoder_seqlens))
-                cur = last_logits[:, -1:].argmax(-1)
-                tokens.append(cur)
-            return torch.cat(tokens, dim=1), last_logits
-
-        session = GraphedDecoding(self, encoder_hidden_states, steps, encoder_seqlens)
+                session.step()
+            return session.tokens, session.last_logits
+        B = encoder_hidden_states.shape[0]
+        cache = self.decoder.new_cache(encoder_hidden_states, steps)
+        cur = torch.full((B, 1), self.cfg.decoder_start_token_id, dtype=torch.long, device=encoder_hidden_states.device)
+        tokens, last_logits = [], None
         for _ in range(steps):
-            session.step()
-        return session.tokens, session.last_logits
+            last_logits = self.logits(self.decoder.decode_step(cur, cache, encoder_seqlens))
+            cur = last_logits[:, -1:].argmax(-1)
+            tokens.append(cur)
+        return torch.cat(tokens, dim=1), last_logits
