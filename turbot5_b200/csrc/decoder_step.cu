@@ -14,9 +14,10 @@
 //   [norm, wi, activation] [wo, residual]          ... per layer
 //   [norm, LM head, argmax] [choice, append token, embedding]
 //
-// Every kernel lets its successor start (launch_dependents) only AFTER its own wait, so whatever ran two kernels
-// earlier has completed, memory included, when a block starts: weights, cross keys and the cached keys of
-// earlier steps may be read before the wait; activations and the newest key may not.
+// Every kernel lets its successor start at once, so two or three kernels of the chain sit on the SMs with their
+// weights loaded while one computes.  What a block reads before its wait is therefore only what no kernel of the
+// chain writes: weights, cross keys and values, their lengths.  Every kernel waits, and a wait ends when the
+// predecessor has completed, its own wait included: after it everything earlier in the chain is visible.
 //
 // Semantics: the cached step of the decoder stack (src/turbot5/model/modeling.py:166-219 per block,
 // src/turbot5/model/attentions.py:198,229-234), rounding points as the separate operators.
@@ -30,11 +31,11 @@ namespace step {
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// untiled bulk copy, global -> shared, completion on an mbarrier (16-byte aligned, a multiple of 16 bytes)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 r;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a));
@@ -63,28 +64,58 @@ template <> __device__ __forceinline__ void mma16816<__half>(float (&c)[4], uint
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+template <typename T> constexpr bool kIsBf16 = false;
+template <> constexpr bool kIsBf16<__nv_bfloat16> = true;
 template <typename T> __device__ __forceinline__ T round_to(float x) { return from_float<T>(x); }
 template <typename T> __device__ __forceinline__ float rounded(float x) { return to_float<T>(from_float<T>(x)); }
 
+// two elements of the 16-bit type, as float32 and back
+template <typename T> __device__ __forceinline__ float2 unpack2(uint32_t v);
+template <> __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t v) {
+  return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t v) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&v));
+}
+template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// products of two pairs, each rounded once (the float32 product of two 16-bit values is exact)
+template <typename T> __device__ __forceinline__ uint32_t mul2h(uint32_t a, uint32_t b);
+template <> __device__ __forceinline__ uint32_t mul2h<__nv_bfloat16>(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <> __device__ __forceinline__ uint32_t mul2h<__half>(uint32_t a, uint32_t b) {
+  const __half2 h = __hmul2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // ---------------------------------------------------------------- skinny matrix products
-// y[B, N] = f(x)[B, K] w[N, K]^T for B <= 64.  A block owns NT * 8 rows of w (all of K), its warps take the
-// 32-wide pieces of K in turn, sixteen rows of x at a time, and meet in shared memory.  mma.m16n8k16: these
-// products are a stream of weights (16 flop per byte at 16 rows); the tensor unit is idle either way, and a
-// tcgen05 tile of 128 rows would be seven eighths padding.
+// y[B, N] = f(x)[B, K] w[N, K]^T for B <= 64.  A block owns NT * 8 rows of w, its eight warps take the 32-wide pieces
+// of K in turn, sixteen rows of x at a time, and meet in shared memory.  mma.m16n8k16: these products are a
+// stream of weights (16 flop per byte at 16 rows); the tensor unit is idle either way, and a tcgen05 tile of 128
+// rows would be seven eighths padding.
 //
 // Operands are read with 16-byte loads: a lane takes eight consecutive k of its row where the instruction's
 // layout asks for four pairs eight apart; the order of k inside a 32-wide piece is the same for both operands,
 // so the products meet.  Row pitch K * 2 + 64 bytes: the rows of a quarter warp's load fall into different banks.
-enum Epilogue { E_STORE = 0, E_QKV, E_RESIDUAL, E_GATED, E_RELU, E_LOGITS };
+// Rows of x past B and rows of w past N hold whatever was there: an output depends on its own row and column only.
+enum Epilogue { E_STORE = 0, E_QKV, E_RESIDUAL, E_GATED, E_RELU };
 
 struct GemmParams {
   const void* x; const void* w; const void* ln; void* out;
-  const void* residual;            // E_RESIDUAL: hidden (out is hidden too)
   void* kv;                        // E_QKV: cache (2, B, H, max_len, D)
   const int32_t* seqlens;          // E_QKV: cached keys of each row, the new one included
-  float2* cand;                    // E_LOGITS: (value, index bits) of each row and block
+  float2* cand;                    // LM head: (value, index bits) of each row and block
   int32_t B, N, K, F;              // F: E_GATED: rows of wi_0 (w holds wi_0 | wi_1)
-  int32_t H, D, max_len, x_stride;
+  int32_t H, D, max_len;
   float eps, x_scale;              // x_scale: multiplies the normed rows (tied embeddings), 1 = off
 };
 
@@ -100,125 +131,195 @@ __device__ __forceinline__ bool argmax_before(float a, int ia, float b, int ib) 
   return ia < ib;
 }
 
-// kNorm: 0 no norm; 1: rows of up to 1024 (four 16-byte vectors per lane, all of a warp's rows at once);
-// 2: up to 2048 (eight vectors, one row at a time).  Registers are held to what lets three blocks share an SM:
-// the successor's blocks have to find room beside the running ones.
-template <typename T, int WARPS, int NT, int kNorm, int kEpi>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 2)
+constexpr int WARPS = 8, THREADS = WARPS * 32;
+
+// RMSNorm of up to sixteen rows of x into shared memory (rows of `pitch` bytes), with the rounding points of
+// t5b_rmsnorm_fwd.  The block's threads are dealt to the rows that exist (a power of two of them each): at one row the
+// whole block shares it.  VECS: 16-byte vectors of a thread, K <= 4 * W * VECS * 4.  Uses part[W]; ends with the rows written, not yet synchronised.
+template <typename T, int VECS, int W>
+__device__ __forceinline__ void norm_rows(const GemmParams& p, int m0, uint32_t sLn, uint32_t sX, uint32_t pitch, float* part,
+                                          uint32_t ln_bar, volatile int* abort_flag, float scale) {
+  const int tid = threadIdx.x, nvec = p.K >> 3;
+  const int rows = min(16, p.B - m0);
+  constexpr int kAll = W == 16 ? 9 : 8;                                                // log2(threads)
+  const int shift = rows > 8 ? kAll - 4 : rows > 4 ? kAll - 3 : rows > 2 ? kAll - 2 : rows > 1 ? kAll - 1 : kAll;
+  const int tpr = 1 << shift, r = tid >> shift, c0 = tid & (tpr - 1);
+  const bool mine = r < rows;
+  uint4 xv[VECS];
+  #pragma unroll
+  for (int i = 0; i < VECS; ++i) {
+    const int c = c0 + i * tpr;
+    xv[i] = make_uint4(0, 0, 0, 0);
+    if (mine && c < nvec) xv[i] = ld_act((const char*)p.x + ((int64_t)(m0 + r) * p.K + c * 8) * 2);
+  }
+  float s0 = 0.f, s1 = 0.f;
+  #pragma unroll
+  for (int i = 0; i < VECS; ++i) {
+    const uint32_t w[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) { const float2 f = unpack2<T>(w[k]); s0 = fmaf(f.x, f.x, s0); s1 = fmaf(f.y, f.y, s1); }
+  }
+  float ss = s0 + s1;
+  #pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+    if (o < tpr) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (tpr > 32) {                                            // (uniform)
+    if ((tid & 31) == 0) part[tid >> 5] = ss;
+    __syncthreads();
+    const int w0 = (tid >> shift) << (shift - 5);
+    ss = 0.f;
+    for (int w = 0; w < (tpr >> 5); ++w) ss += part[w0 + w];
+  }
+  const float rstd = rsqrtf(ss / (float)p.K + p.eps);
+  mbar_wait_bounded(ln_bar, 0, abort_flag);
+  if (mine) {
+    #pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+      const int c = c0 + i * tpr;
+      if (c < nvec) {
+        const uint4 wv = lds128(sLn + c * 16);
+        const uint32_t x[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w}, w[4] = {wv.x, wv.y, wv.z, wv.w};
+        uint32_t y[4];
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = unpack2<T>(x[k]);
+          y[k] = mul2h<T>(w[k], pack2<T>(f.x * rstd, f.y * rstd));
+          if (scale != 1.f) {                                 // the scale is a float32 factor of the rounded value
+            const float2 n = unpack2<T>(y[k]);
+            y[k] = pack2<T>(n.x * scale, n.y * scale);
+          }
+        }
+        sts128(sX + r * pitch + c * 16, make_uint4(y[0], y[1], y[2], y[3]));
+      }
+    }
+  }
+}
+
+// the warps' sums for one output element
+template <int W, int COLS>
+__device__ __forceinline__ float warp_sums(const float* red, int r, int c) {
+  float s = 0.f;
+  #pragma unroll
+  for (int w = 0; w < W; ++w) s += red[(w * 16 + r) * COLS + c];
+  return s;
+}
+
+// kNorm: the product is of the normed rows.  bf16: y = rstd * sum_k (x w_ln)[k] w[n, k] -- the norm weight goes onto the
+// operand as it is loaded (one rounding where the separate norm has two), every warp sums the squares of its share
+// of the row beside its products, and rstd multiplies the finished sum, so the norm adds no phase to the kernel
+// (as a pass of its own, rows into shared memory and two barriers, it took 1.0 of 2.5 us at one row and 1.8 of 3.1
+// at sixteen).  fp16 has not the range for unnormed products: its rows are normed first (norm_rows).
+// W warps per block; registers are held to what lets the successor's blocks find room beside the running ones.
+template <typename T, int W, int NT, bool kNorm, int kEpi>
+__global__ void __launch_bounds__(W * 32, kNorm && !kIsBf16<T> ? 1 : 2)
 step_gemm_kernel(const __grid_constant__ GemmParams p) {
-  constexpr int THREADS = WARPS * 32;
+  constexpr bool kFold = kNorm && sizeof(T) == 2 && kIsBf16<T>;
+  constexpr bool kRows = kNorm && !kFold;
   constexpr int COLS = NT * 8;                               // accumulator columns of the block
   constexpr int OUT_COLS = kEpi == E_GATED ? COLS / 2 : COLS;
   extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) unsigned long long bar_words[2];
+  __shared__ int abort_word;
+  __shared__ float part[W];
+  __shared__ float squares[kFold ? W : 1][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int K = p.K, nvec = K >> 3;
+  const int K = p.K;
   const uint32_t pitch = (uint32_t)K * 2 + 64;
   const uint32_t sW = smem_u32(smem);
   const uint32_t sLn = sW + COLS * pitch;
   const uint32_t sX = sLn + (kNorm ? (uint32_t)K * 2 : 0u);
-  float* red = reinterpret_cast<float*>(smem + COLS * pitch + (kNorm ? (uint32_t)K * 2 + 16 * pitch : 0u));
-  const int n0 = blockIdx.x * OUT_COLS;
+  float* red = reinterpret_cast<float*>(smem + COLS * pitch + (kNorm ? (uint32_t)K * 2 : 0u) + (kRows ? 16 * pitch : 0u));
+  const uint32_t w_bar = smem_u32(&bar_words[0]), ln_bar = smem_u32(&bar_words[1]);
+  const int n0 = (int)blockIdx.x * OUT_COLS;
+  grid_launch_dependents();
 
   // the block's weights, before anything that depends on an earlier kernel
-  for (int r = warp; r < COLS; r += WARPS) {
-    int n;
-    if (kEpi == E_GATED) n = r < COLS / 2 ? n0 + r : p.F + n0 + r - COLS / 2;
-    else n = n0 + r;
-    const bool ok = kEpi == E_GATED ? n0 + (r % (COLS / 2)) < p.F : n < p.N;
-    const char* src = (const char*)p.w + (int64_t)n * K * 2;
-    for (int c = lane; c < nvec; c += 32) {
-      if (ok) cp_async16(sW + r * pitch + c * 16, src + c * 16);
-      else sts128(sW + r * pitch + c * 16, make_uint4(0, 0, 0, 0));
+  if (tid == 0) {
+    abort_word = 0;
+    mbar_init(w_bar, 1);
+    mbar_init(ln_bar, 1);
+    fence_barrier_init();
+    fence_proxy_async();
+    if (kNorm) {
+      mbar_expect_tx(ln_bar, (uint32_t)K * 2);
+      bulk_load(sLn, p.ln, (uint32_t)K * 2, ln_bar);
     }
   }
-  if (kNorm)
-    for (int c = tid; c < nvec; c += THREADS) cp_async16(sLn + c * 16, (const char*)p.ln + c * 16);
-  cp_async_commit();
+  if (warp == 0) {                                            // one row per lane: a copy costs its issuing thread tens of cycles
+    const int r = lane;
+    const int n = kEpi == E_GATED ? (r < COLS / 2 ? n0 + r : p.F + n0 + r - COLS / 2) : n0 + r;
+    const bool ok = r < COLS && (kEpi == E_GATED ? n0 + r % (COLS / 2) < p.F : n < p.N);
+    const int rows = __popc(__ballot_sync(0xffffffffu, ok));
+    if (lane == 0) mbar_expect_tx(w_bar, (uint32_t)(rows * K * 2));
+    __syncwarp();
+    if (ok) bulk_load(sW + r * pitch, (const char*)p.w + (int64_t)n * K * 2, (uint32_t)K * 2, w_bar);
+  }
+  __syncthreads();
+  volatile int* abort_flag = &abort_word;
+  // (a wait that gave up leaves wrong numbers, never a hang)
+  if (kFold) mbar_wait_bounded(ln_bar, 0, abort_flag);
   grid_wait();
-  grid_launch_dependents();
 
   const int g = lane >> 2, t = lane & 3;
   for (int m0 = 0; m0 < p.B; m0 += 16) {
-    if (kNorm) {
-      constexpr int ROWS = 16 / WARPS;                       // rows per warp
-      constexpr int VECS = kNorm == 2 ? 8 : 4, AT_ONCE = kNorm == 2 ? 1 : ROWS;
-      #pragma unroll 1
-      for (int q0 = 0; q0 < ROWS; q0 += AT_ONCE) {
-        uint4 xv[AT_ONCE][VECS];
-        #pragma unroll
-        for (int q = 0; q < AT_ONCE; ++q) {
-          const int row = m0 + warp + (q0 + q) * WARPS;
-          #pragma unroll
-          for (int i = 0; i < VECS; ++i) {
-            const int c = lane + i * 32;
-            xv[q][i] = make_uint4(0, 0, 0, 0);
-            if (row < p.B && c < nvec) xv[q][i] = ld_act((const char*)p.x + (int64_t)row * p.x_stride * 2 + c * 16);
-          }
-        }
-        if (q0 == 0) {
-          cp_async_wait_all();
-          __syncthreads();                                   // ln is in shared memory; the rows of the last round are done with
-        }
-        #pragma unroll
-        for (int q = 0; q < AT_ONCE; ++q) {
-          float ss = 0.f;
-          #pragma unroll
-          for (int i = 0; i < VECS; ++i) {
-            const T* e = reinterpret_cast<const T*>(&xv[q][i]);
-            #pragma unroll
-            for (int k = 0; k < 8; ++k) { const float f = to_float<T>(e[k]); ss = fmaf(f, f, ss); }
-          }
-          #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-          const float rstd = rsqrtf(ss / (float)K + p.eps);
-          #pragma unroll
-          for (int i = 0; i < VECS; ++i) {
-            const int c = lane + i * 32;
-            if (c < nvec) {
-              const uint4 wv = lds128(sLn + c * 16);
-              const T* e = reinterpret_cast<const T*>(&xv[q][i]);
-              const T* we = reinterpret_cast<const T*>(&wv);
-              uint4 o4;
-              T* oe = reinterpret_cast<T*>(&o4);
-              #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                float y = rounded<T>(to_float<T>(we[k]) * rounded<T>(to_float<T>(e[k]) * rstd));
-                if (kEpi == E_LOGITS && p.x_scale != 1.f) y = rounded<T>(y * p.x_scale);
-                oe[k] = round_to<T>(y);
-              }
-              sts128(sX + (warp + (q0 + q) * WARPS) * pitch + c * 16, o4);
-            }
-          }
-        }
-      }
-    } else {
-      cp_async_wait_all();
+    const int rows = min(16, p.B - m0);
+    if constexpr (kRows) {
+      norm_rows<T, 16, W>(p, m0, sLn, sX, pitch, part, ln_bar, abort_flag, 1.f);
+      __syncthreads();
     }
-    __syncthreads();
-
     float acc[NT][4];
     #pragma unroll
     for (int j = 0; j < NT; ++j)
       #pragma unroll
       for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-    const char* xlo = (const char*)p.x + (int64_t)(m0 + g) * p.x_stride * 2 + t * 16;
-    const char* xhi = xlo + (int64_t)8 * p.x_stride * 2;
-    const bool lo_ok = m0 + g < p.B, hi_ok = m0 + g + 8 < p.B;
-    #pragma unroll 4
-    for (int kb = warp; kb < (K >> 5); kb += WARPS) {
-      uint4 a = make_uint4(0, 0, 0, 0), b = make_uint4(0, 0, 0, 0);     // rows g and g + 8
-      if (kNorm) {
-        a = lds128(sX + g * pitch + kb * 64 + t * 16);
-        b = lds128(sX + (g + 8) * pitch + kb * 64 + t * 16);
-      } else {
-        if (lo_ok) a = ld_act(xlo + kb * 64);
-        if (hi_ok) b = ld_act(xhi + kb * 64);
-      }
+    float sq_lo = 0.f, sq_hi = 0.f;
+    const char* xlo = (const char*)p.x + (int64_t)(m0 + g) * K * 2 + t * 16;
+    const char* xhi = xlo + (int64_t)8 * K * 2;
+    const bool lo_ok = g < rows, hi_ok = g + 8 < rows;
+    bool have_w = false;
+    #pragma unroll 1
+    for (int kb0 = warp; kb0 < (K >> 5); kb0 += 4 * W) {
+      uint4 a[4], b[4];                                       // rows g and g + 8: four pieces in flight
       #pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const uint4 w4 = lds128(sW + (j * 8 + g) * pitch + kb * 64 + t * 16);
-        mma16816<T>(acc[j], a.x, b.x, a.y, b.y, w4.x, w4.y);
-        mma16816<T>(acc[j], a.z, b.z, a.w, b.w, w4.z, w4.w);
+      for (int u = 0; u < 4; ++u) {
+        const int kb = kb0 + u * W;
+        a[u] = b[u] = make_uint4(0, 0, 0, 0);
+        if (kb < (K >> 5)) {
+          if (kRows) {
+            a[u] = lds128(sX + g * pitch + kb * 64 + t * 16);
+            b[u] = lds128(sX + (g + 8) * pitch + kb * 64 + t * 16);
+          } else {
+            if (lo_ok) a[u] = ld_act(xlo + kb * 64);
+            if (hi_ok) b[u] = ld_act(xhi + kb * 64);
+          }
+        }
+      }
+      if (!have_w) { mbar_wait_bounded(w_bar, 0, abort_flag); have_w = true; }
+      #pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int kb = kb0 + u * W;
+        if (kb < (K >> 5)) {
+          if (kFold) {
+            const uint4 l = lds128(sLn + kb * 64 + t * 16);
+            uint32_t* av = reinterpret_cast<uint32_t*>(&a[u]);
+            uint32_t* bv = reinterpret_cast<uint32_t*>(&b[u]);
+            const uint32_t lv[4] = {l.x, l.y, l.z, l.w};
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 fa = unpack2<T>(av[i]), fb = unpack2<T>(bv[i]);
+              sq_lo = fmaf(fa.x, fa.x, fmaf(fa.y, fa.y, sq_lo));
+              sq_hi = fmaf(fb.x, fb.x, fmaf(fb.y, fb.y, sq_hi));
+              av[i] = mul2h<T>(av[i], lv[i]);
+              bv[i] = mul2h<T>(bv[i], lv[i]);
+            }
+          }
+          #pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const uint4 w4 = lds128(sW + (j * 8 + g) * pitch + kb * 64 + t * 16);
+            mma16816<T>(acc[j], a[u].x, b[u].x, a[u].y, b[u].y, w4.x, w4.y);
+            mma16816<T>(acc[j], a[u].z, b[u].z, a[u].w, b[u].w, w4.z, w4.w);
+          }
+        }
       }
     }
     // ---- the warps' partial sums meet: red[warp][row][column]
@@ -228,54 +329,172 @@ step_gemm_kernel(const __grid_constant__ GemmParams p) {
       *reinterpret_cast<float2*>(r0) = make_float2(acc[j][0], acc[j][1]);
       *reinterpret_cast<float2*>(r0 + 8 * COLS) = make_float2(acc[j][2], acc[j][3]);
     }
+    if (kFold) {
+      #pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        sq_lo += __shfl_xor_sync(0xffffffffu, sq_lo, o);
+        sq_hi += __shfl_xor_sync(0xffffffffu, sq_hi, o);
+      }
+      if (t == 0) { squares[warp][g] = sq_lo; squares[warp][g + 8] = sq_hi; }
+    }
     __syncthreads();
-    for (int idx = tid; idx < 16 * OUT_COLS; idx += THREADS) {
+    #pragma unroll 1
+    for (int idx = tid; idx < rows * OUT_COLS; idx += W * 32) {
       const int r = idx / OUT_COLS, c = idx % OUT_COLS;
       const int row = m0 + r, n = n0 + c;
-      float s = 0.f, s2 = 0.f;
-      #pragma unroll
-      for (int w = 0; w < WARPS; ++w) {
-        s += red[(w * 16 + r) * COLS + c];
-        if (kEpi == E_GATED) s2 += red[(w * 16 + r) * COLS + COLS / 2 + c];
-      }
-      const bool ok = row < p.B && n < (kEpi == E_GATED ? p.F : p.N);
-      if (kEpi == E_STORE) {
-        if (ok) ((T*)p.out)[(int64_t)row * p.N + n] = round_to<T>(s);
-      } else if (kEpi == E_RELU) {
-        if (ok) ((T*)p.out)[(int64_t)row * p.N + n] = round_to<T>(fmaxf(s, 0.f));
-      } else if (kEpi == E_GATED) {
-        if (ok) ((T*)p.out)[(int64_t)row * p.F + n] = round_to<T>(rounded<T>(gelu_tanh(rounded<T>(s))) * rounded<T>(s2));
-      } else if (kEpi == E_RESIDUAL) {
-        if (ok) {
-          T* o = (T*)p.out + (int64_t)row * p.N + n;
-          *o = round_to<T>(to_float<T>(*o) + rounded<T>(s));
-        }
-      } else if (kEpi == E_QKV) {
-        if (ok) {
-          const int HD = p.H * p.D;
-          if (n < HD) ((T*)p.out)[(int64_t)row * HD + n] = round_to<T>(s);
-          else {
-            const int kv = n >= 2 * HD ? 1 : 0, m = n - HD - kv * HD, h = m / p.D, d = m - h * p.D;
-            const int pos = p.seqlens[row] - 1;
-            if (pos >= 0 && pos < p.max_len)
-              ((T*)p.kv)[((((int64_t)kv * p.B + row) * p.H + h) * p.max_len + pos) * p.D + d] = round_to<T>(s);
-          }
-        }
-      } else {     // E_LOGITS: a warp holds the 32 columns of one row (NT = 4)
-        const float v = rounded<T>(s);
-        if (ok) ((T*)p.out)[(int64_t)row * p.N + n] = round_to<T>(s);
-        float bv = ok ? v : -INFINITY;
-        int bi = ok ? n : 0x7fffffff;
+      float s = warp_sums<W, COLS>(red, r, c), rstd = 1.f;
+      if (kFold) {
+        float ss = 0.f;
         #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (argmax_before(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+        for (int w = 0; w < W; ++w) ss += squares[w][r];
+        rstd = rsqrtf(ss / (float)K + p.eps);
+        s *= rstd;
+      }
+      if (n >= (kEpi == E_GATED ? p.F : p.N)) continue;
+      if (kEpi == E_STORE) {
+        ((T*)p.out)[(int64_t)row * p.N + n] = round_to<T>(s);
+      } else if (kEpi == E_RELU) {
+        ((T*)p.out)[(int64_t)row * p.N + n] = round_to<T>(fmaxf(s, 0.f));
+      } else if (kEpi == E_GATED) {
+        const float s2 = warp_sums<W, COLS>(red, r, COLS / 2 + c) * rstd;
+        ((T*)p.out)[(int64_t)row * p.F + n] = round_to<T>(rounded<T>(gelu_tanh(rounded<T>(s))) * rounded<T>(s2));
+      } else if (kEpi == E_RESIDUAL) {
+        T* o = (T*)p.out + (int64_t)row * p.N + n;
+        *o = round_to<T>(to_float<T>(*o) + rounded<T>(s));
+      } else {
+        const int HD = p.H * p.D;
+        if (n < HD) ((T*)p.out)[(int64_t)row * HD + n] = round_to<T>(s);
+        else {
+          const int kv = n >= 2 * HD ? 1 : 0, m = n - HD - kv * HD, h = m / p.D, d = m - h * p.D;
+          const int pos = p.seqlens[row] - 1;
+          if (pos >= 0 && pos < p.max_len)
+            ((T*)p.kv)[((((int64_t)kv * p.B + row) * p.H + h) * p.max_len + pos) * p.D + d] = round_to<T>(s);
         }
-        if (lane == 0 && row < p.B) p.cand[(int64_t)row * gridDim.x + blockIdx.x] = make_float2(bv, __int_as_float(bi));
       }
     }
     if (m0 + 16 < p.B) __syncthreads();                       // `red` is written again
+  }
+}
+
+// ---------------------------------------------------------------- LM head
+// Final norm, logits and each block's best token.  One block per SM; the norm is done once per SM, then every warp walks
+// its share of the vocabulary by itself, eight rows of w at a time over all of K, through its own ring of bulk loads
+// (pieces of `piece` columns): no barrier between warps in the loop.  Bound by HBM (66 MB at 32128 x 1024).  Measured at
+// 16 rows: a block per 32 rows of w 43 us, one ring per block with a barrier per tile 21 us, this 15.8 us.
+constexpr int LM_MAX_STAGES = 4;
+
+template <typename T, int M_TILES>
+__global__ void __launch_bounds__(THREADS, 1)
+step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) unsigned long long bar_words[WARPS * LM_MAX_STAGES + 1];
+  __shared__ int abort_word;
+  __shared__ float part[WARPS];
+  __shared__ float best_v[WARPS][16 * M_TILES];
+  __shared__ int best_i[WARPS][16 * M_TILES];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = p.K;
+  const uint32_t pitch = (uint32_t)K * 2 + 64, wpitch = (uint32_t)piece * 2 + 64, stage_bytes = 8 * wpitch;
+  const uint32_t sX = smem_u32(smem), sLn = sX + M_TILES * 16 * pitch, sW = sLn + (uint32_t)K * 2 + warp * stages * stage_bytes;
+  const uint32_t bar0 = smem_u32(&bar_words[warp * LM_MAX_STAGES]), ln_bar = smem_u32(&bar_words[WARPS * LM_MAX_STAGES]);
+  const int tiles = (p.N + 7) / 8, pieces = K / piece;
+  const int first = (int)blockIdx.x * WARPS + warp, step = (int)gridDim.x * WARPS;
+  const int n_mine = first < tiles ? (tiles - first + step - 1) / step : 0;
+  auto load = [&](int it) {                                  // the it-th piece of this warp (a row per lane)
+    if (it >= n_mine * pieces) return;
+    const int tile = first + (it / pieces) * step, k0 = (it % pieces) * piece;
+    const uint32_t bar = bar0 + 8 * (it % stages), dst = sW + (it % stages) * stage_bytes;
+    const int rows = min(8, p.N - tile * 8);
+    if (lane == 0) mbar_expect_tx(bar, (uint32_t)(rows * piece * 2));
+    __syncwarp();
+    if (lane < rows)
+      bulk_load(dst + lane * wpitch, (const char*)p.w + ((int64_t)(tile * 8 + lane) * K + k0) * 2, (uint32_t)piece * 2, bar);
+  };
+  grid_launch_dependents();
+  if (lane == 0) {
+    for (int i = 0; i < stages; ++i) mbar_init(bar0 + 8 * i, 1);
+    if (tid == 0) { abort_word = 0; mbar_init(ln_bar, 1); }
+    fence_barrier_init();
+    fence_proxy_async();
+    if (tid == 0) {
+      mbar_expect_tx(ln_bar, (uint32_t)K * 2);
+      bulk_load(sLn, p.ln, (uint32_t)K * 2, ln_bar);
+    }
+  }
+  __syncwarp();
+  for (int i = 0; i < stages; ++i) load(i);
+  __syncthreads();
+  volatile int* abort_flag = &abort_word;
+  grid_wait();
+  #pragma unroll 1
+  for (int m = 0; m < M_TILES; ++m) {
+    norm_rows<T, 16, WARPS>(p, 16 * m, sLn, sX + 16 * m * pitch, pitch, part, ln_bar, abort_flag, p.x_scale);
+    __syncthreads();
+  }
+  const int g = lane >> 2, t = lane & 3;
+  float bv[M_TILES][2];                                      // best of rows g and g + 8 among this lane's columns
+  int bi[M_TILES][2];
+  #pragma unroll
+  for (int m = 0; m < M_TILES; ++m)
+    #pragma unroll
+    for (int r = 0; r < 2; ++r) { bv[m][r] = -INFINITY; bi[m][r] = 0x7fffffff; }
+  int it = 0;
+  for (int i = 0; i < n_mine; ++i) {
+    const int tile = first + i * step;
+    float acc[M_TILES][2][4];                                // two chains per sixteen rows
+    #pragma unroll
+    for (int m = 0; m < M_TILES; ++m)
+      #pragma unroll
+      for (int e = 0; e < 8; ++e) acc[m][e >> 2][e & 3] = 0.f;
+    for (int pc = 0; pc < pieces; ++pc, ++it) {
+      const uint32_t w0 = sW + (it % stages) * stage_bytes + g * wpitch + t * 16;
+      const uint32_t x0 = sX + g * pitch + pc * piece * 2 + t * 16;
+      mbar_wait_bounded(bar0 + 8 * (it % stages), (uint32_t)((it / stages) & 1), abort_flag);
+      #pragma unroll 4
+      for (int kb = 0; kb < piece / 32; ++kb) {
+        const uint4 w4 = lds128(w0 + kb * 64);
+        #pragma unroll
+        for (int m = 0; m < M_TILES; ++m) {
+          const uint4 a = lds128(x0 + 16 * m * pitch + kb * 64), b = lds128(x0 + (16 * m + 8) * pitch + kb * 64);
+          mma16816<T>(acc[m][0], a.x, b.x, a.y, b.y, w4.x, w4.y);
+          mma16816<T>(acc[m][1], a.z, b.z, a.w, b.w, w4.z, w4.w);
+        }
+      }
+      __syncwarp();                                          // every lane has read the piece: its slot may be filled again
+      load(it + stages);
+    }
+    #pragma unroll
+    for (int m = 0; m < M_TILES; ++m)
+      #pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = 16 * m + g + (e >> 1) * 8, n = tile * 8 + 2 * t + (e & 1);
+        if (row < p.B && n < p.N) {
+          const T o = round_to<T>(acc[m][0][e] + acc[m][1][e]);
+          ((T*)p.out)[(int64_t)row * p.N + n] = o;
+          const float v = to_float<T>(o);
+          // (n increases from tile to tile: a tie stays with the first)
+          if (bi[m][e >> 1] == 0x7fffffff || v > bv[m][e >> 1] || (isnan(v) && !isnan(bv[m][e >> 1]))) { bv[m][e >> 1] = v; bi[m][e >> 1] = n; }
+        }
+      }
+  }
+  #pragma unroll
+  for (int m = 0; m < M_TILES; ++m)
+    #pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      #pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv[m][r], o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi[m][r], o);
+        if (argmax_before(ov, oi, bv[m][r], bi[m][r])) { bv[m][r] = ov; bi[m][r] = oi; }
+      }
+      if (t == 0) { best_v[warp][16 * m + g + 8 * r] = bv[m][r]; best_i[warp][16 * m + g + 8 * r] = bi[m][r]; }
+    }
+  __syncthreads();
+  if (tid < p.B) {
+    float v = best_v[0][tid];
+    int n = best_i[0][tid];
+    for (int w = 1; w < WARPS; ++w)
+      if (argmax_before(best_v[w][tid], best_i[w][tid], v, n)) { v = best_v[w][tid]; n = best_i[w][tid]; }
+    p.cand[(int64_t)tid * gridDim.x + blockIdx.x] = make_float2(v, __int_as_float(n));
   }
 }
 
@@ -292,12 +511,12 @@ struct AttnStepParams {
   int32_t B, H, N, md, splits;
 };
 
-template <typename T, int D, int WARPS, bool kSelf>
-__global__ void __launch_bounds__(WARPS * 32)
+template <typename T, int D, int AW, bool kSelf>
+__global__ void __launch_bounds__(AW * 32)
 step_attention_kernel(const __grid_constant__ AttnStepParams p) {
   constexpr int LPK = D / 8, KPW = 32 / LPK, UNROLL = 4, KPI = KPW * UNROLL;
-  __shared__ float sm_m[WARPS], sm_l[WARPS];
-  __shared__ float sm_o[WARPS][D];
+  __shared__ float sm_m[AW], sm_l[AW];
+  __shared__ float sm_o[AW][D];
   __shared__ int is_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int grp = lane / LPK, gl = lane % LPK;
@@ -310,7 +529,7 @@ step_attention_kernel(const __grid_constant__ AttnStepParams p) {
   auto range = [&]() {
     const int len = p.lens ? min(p.lens[b], p.N) : p.N;
     int chunk = (len + p.splits - 1) / p.splits;
-    chunk = (chunk + WARPS * KPI - 1) / (WARPS * KPI) * (WARPS * KPI);
+    chunk = (chunk + AW * KPI - 1) / (AW * KPI) * (AW * KPI);
     n_begin = min(split * chunk, len);
     n_end = min(n_begin + chunk, len);
     return len;
@@ -332,12 +551,12 @@ step_attention_kernel(const __grid_constant__ AttnStepParams p) {
     }
   };
   int len = 0;
+  grid_launch_dependents();
   if (!kSelf) {                      // the lengths of the memory are constant too
     len = range();
     load(n_begin + warp * KPI, kr[0], vr[0]);
   }
   grid_wait();
-  grid_launch_dependents();
   const uint4 q4 = ld_act((const char*)p.q + 2 * (((int64_t)b * p.H + h) * D + gl * 8));
   if (kSelf) {
     len = range();
@@ -388,13 +607,13 @@ step_attention_kernel(const __grid_constant__ AttnStepParams p) {
   };
   int it = n_begin + warp * KPI;
   while (it < n_end) {
-    load(it + WARPS * KPI, kr[1], vr[1]);
+    load(it + AW * KPI, kr[1], vr[1]);
     consume(it, kr[0], vr[0]);
-    it += WARPS * KPI;
+    it += AW * KPI;
     if (it >= n_end) break;
-    load(it + WARPS * KPI, kr[0], vr[0]);
+    load(it + AW * KPI, kr[0], vr[0]);
     consume(it, kr[1], vr[1]);
-    it += WARPS * KPI;
+    it += AW * KPI;
   }
 
   // ---- merge lane groups, then warps
@@ -418,10 +637,10 @@ step_attention_kernel(const __grid_constant__ AttnStepParams p) {
   float mm = -INFINITY, l = 0.f, o = 0.f;
   if (tid < D) {
     #pragma unroll
-    for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, sm_m[w]);
+    for (int w = 0; w < AW; ++w) mm = fmaxf(mm, sm_m[w]);
     const float m_safe = mm == -INFINITY ? 0.f : mm;
     #pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
+    for (int w = 0; w < AW; ++w) {
       const float sc = fast_exp2(sm_m[w] - m_safe);
       l += sm_l[w] * sc;
       o += sm_o[w][tid] * sc;
@@ -468,8 +687,8 @@ step_choose_kernel(const float2* cand, int n_cand, int64_t* tokens, int64_t toke
   __shared__ float sv[8];
   __shared__ int si[8];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-  grid_wait();
   grid_launch_dependents();
+  grid_wait();
   float bv = -INFINITY;
   int bi = 0x7fffffff;
   for (int i = tid; i < n_cand; i += 256) {
@@ -525,52 +744,87 @@ struct Launcher {
   }
 };
 
-template <typename T, int WARPS, int NT, int kNorm, int kEpi>
-static void launch_gemm(Launcher& go, const GemmParams& p) {
-  auto kern = step_gemm_kernel<T, WARPS, NT, kNorm, kEpi>;
-  const size_t pitch = (size_t)p.K * 2 + 64;
-  const size_t smem = NT * 8 * pitch + (kNorm ? (size_t)p.K * 2 + 16 * pitch : 0) + (size_t)WARPS * 16 * NT * 8 * 4;
-  static std::atomic<bool> attr_set[64];
+// Opt in to all of an SM's shared memory, once per device and kernel (`done`: a static of the call site).
+template <typename F>
+static bool allow_smem(F kern, std::atomic<bool>* done) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
-      cudaGetLastError();
-      go.status = T5B_ERR_LAUNCH;
-      return;
-    }
-    if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+  if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return true;
+  cudaFuncAttributes fa;
+  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
-  if (smem > 227 * 1024) { go.status = T5B_ERR_UNSUPPORTED; return; }
+  if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+  return true;
+}
+constexpr size_t kMaxSmem = 223 * 1024, kLmSmem = 220 * 1024;       // dynamic; the kernels' own words take the rest
+
+template <typename T, int W, int NT, bool kNorm, int kEpi>
+static void launch_gemm(Launcher& go, const GemmParams& p) {
+  auto kern = step_gemm_kernel<T, W, NT, kNorm, kEpi>;
+  const size_t K = p.K, pitch = K * 2 + 64;
+  const size_t smem = NT * 8 * pitch + (kNorm ? K * 2 : 0) + (kNorm && !kIsBf16<T> ? 16 * pitch : 0) + (size_t)W * 16 * NT * 8 * 4;
+  static std::atomic<bool> attributes[64];
+  if (smem > kMaxSmem) { go.status = T5B_ERR_UNSUPPORTED; return; }
+  if (!allow_smem(kern, attributes)) { go.status = T5B_ERR_LAUNCH; return; }
   const int cols = kEpi == E_GATED ? NT * 4 : NT * 8, n = kEpi == E_GATED ? p.F : p.N;
-  go(kern, dim3((unsigned)((n + cols - 1) / cols), 1, 1), WARPS * 32, smem, p);
+  go(kern, dim3((unsigned)((n + cols - 1) / cols), 1, 1), W * 32, smem, p);
 }
 
-// Rows of w per block: one tensor-core tile (8 rows) while that gives at most two blocks per SM, so that all SMs
-// pull weights and the successor's blocks still find room; two or four tiles beyond.
-template <typename T, int kNorm, int kEpi>
-static void gemm_sized(Launcher& go, const GemmParams& p) {
-  const int tiles = ((kEpi == E_GATED ? p.F : p.N) + 7) / 8;
+// Rows of w per block of the products that start with a norm: one tensor-core tile (8 rows) while that gives at
+// most two blocks per SM, so that all SMs pull weights and the successor's blocks still find room; two or
+// four tiles beyond.
+template <typename T, int kEpi>
+static void norm_gemm(Launcher& go, const GemmParams& p) {
+  const int tiles = ((kEpi == E_GATED ? 2 * p.F : p.N) + 7) / 8;
   if constexpr (kEpi == E_GATED) {
-    if (tiles <= 592) launch_gemm<T, 8, 2, kNorm, kEpi>(go, p);       // one tile of wi_0 and of wi_1 is four rows of each
-    else launch_gemm<T, 8, 4, kNorm, kEpi>(go, p);
-  } else if constexpr (kEpi == E_RESIDUAL) {
-    // K = d_ff can be long: sixteen warps keep twice as many rows of x in flight
-    if (p.K >= 2048) launch_gemm<T, 16, 1, kNorm, kEpi>(go, p);
-    else launch_gemm<T, 8, 1, kNorm, kEpi>(go, p);
-  } else if constexpr (kEpi == E_LOGITS) {
-    launch_gemm<T, 8, 4, kNorm, kEpi>(go, p);
+    if (tiles <= 592) launch_gemm<T, 16, 2, true, kEpi>(go, p);
+    else launch_gemm<T, 16, 4, true, kEpi>(go, p);
   } else {
-    if (tiles <= 296) launch_gemm<T, 8, 1, kNorm, kEpi>(go, p);
-    else if (tiles <= 592) launch_gemm<T, 8, 2, kNorm, kEpi>(go, p);
-    else launch_gemm<T, 8, 4, kNorm, kEpi>(go, p);
+    if (tiles <= 296) launch_gemm<T, 16, 1, true, kEpi>(go, p);
+    else if (tiles <= 592) launch_gemm<T, 16, 2, true, kEpi>(go, p);
+    else launch_gemm<T, 16, 4, true, kEpi>(go, p);
   }
 }
-template <typename T, bool kNorm, int kEpi>
-static void gemm(Launcher& go, const GemmParams& p) {
-  if constexpr (!kNorm) gemm_sized<T, 0, kEpi>(go, p);
-  else if (p.K <= 1024) gemm_sized<T, 1, kEpi>(go, p);
-  else gemm_sized<T, 2, kEpi>(go, p);
+// Output projections: at K = 4096 a block of one tile reads 128 KB of activations for 64 KB of weights, so from there
+// on a block takes two (4.2 us against 5.2 us at 16 rows).
+template <typename T>
+static void residual_gemm(Launcher& go, const GemmParams& p) {
+  if (p.K >= 4096) launch_gemm<T, 16, 2, false, E_RESIDUAL>(go, p);
+  else launch_gemm<T, 16, 1, false, E_RESIDUAL>(go, p);
+}
+
+static int lm_blocks(int vocab) {
+  static std::atomic<int> sms[64];
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64) n = sms[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 148; }
+    if (dev >= 0 && dev < 64) sms[dev].store(n, std::memory_order_relaxed);
+  }
+  const int blocks = ((vocab + 7) / 8 + WARPS - 1) / WARPS;
+  return blocks < n ? blocks : n;
+}
+// Pieces of half of K where that is whole 32s (a ring of two to four then fits beside the normed rows), else all of K.
+template <typename T, int M_TILES>
+static void launch_logits(Launcher& go, const GemmParams& p) {
+  auto kern = step_logits_kernel<T, M_TILES>;
+  const size_t fixed = (size_t)p.K * 2 + (size_t)M_TILES * 16 * ((size_t)p.K * 2 + 64);
+  int piece = p.K, stages = 0;
+  auto fits = [&]() {
+    const size_t stage = (size_t)WARPS * 8 * ((size_t)piece * 2 + 64);
+    const size_t n = fixed < kLmSmem ? (kLmSmem - fixed) / stage : 0;
+    stages = n > LM_MAX_STAGES ? LM_MAX_STAGES : (int)n;
+  };
+  fits();
+  while (stages < 2 && piece % 64 == 0) { piece /= 2; fits(); }
+  static std::atomic<bool> attributes[64];
+  if (stages < 1) { go.status = T5B_ERR_UNSUPPORTED; return; }
+  if (!allow_smem(kern, attributes)) { go.status = T5B_ERR_LAUNCH; return; }
+  go(kern, dim3((unsigned)lm_blocks(p.N), 1, 1), THREADS, fixed + (size_t)stages * WARPS * 8 * ((size_t)piece * 2 + 64), p, piece, stages);
 }
 
 template <typename T, bool kSelf>
@@ -582,15 +836,16 @@ static void attention(Launcher& go, const AttnStepParams& p, int D) {
     case 16: go(step_attention_kernel<T, 16, W, kSelf>, grid, W * 32, 0, p); break;
     case 32: go(step_attention_kernel<T, 32, W, kSelf>, grid, W * 32, 0, p); break;
     case 64: go(step_attention_kernel<T, 64, W, kSelf>, grid, W * 32, 0, p); break;
-    case 128: go(step_attention_kernel<T, 128, 8, kSelf>, grid, 256, 0, p); break;
+    case 128: go(step_attention_kernel<T, 128, W, kSelf>, grid, W * 32, 0, p); break;
     default: go.status = T5B_ERR_HEAD_DIM;
   }
 }
 
-// Splits of the keys: enough blocks for two per SM, at least 128 keys per split.
+// Splits of the keys: a block per SM, at least 128 keys per split.  (More blocks than that lose: at 16 x 16 heads and
+// 1024 keys one split takes 12.4 us, two 17.3 us, four 20.0 us.)
 static int splits_for(int B, int H, int N) {
   const long long bh = (long long)B * H;
-  long long want = (296 + bh - 1) / bh, cap = (N + 127) / 128;
+  long long want = (148 + bh - 1) / bh, cap = (N + 127) / 128;
   long long s = want < cap ? want : cap;
   return (int)(s < 1 ? 1 : (s > 64 ? 64 : s));
 }
@@ -604,7 +859,7 @@ static Layout layout(const t5b_decoder_step_args& a) {
   l.self_splits = splits_for(a.B, a.H, a.max_len);
   l.cross_splits = splits_for(a.B, a.H, a.enc_len);
   const int s = l.self_splits > l.cross_splits ? l.self_splits : l.cross_splits;
-  l.n_cand = (a.vocab + 31) / 32;
+  l.n_cand = lm_blocks(a.vocab);
   l.q = take(a.B * HD * 2);
   l.attn = take(a.B * HD * 2);
   l.act = take((int64_t)a.B * a.d_ff * 2);
@@ -628,11 +883,11 @@ static int run_step(const t5b_decoder_step_args& a, cudaStream_t stream) {
     GemmParams g = {};
     g.B = a.B; g.eps = a.eps; g.x_scale = 1.f; g.H = a.H; g.D = a.D; g.max_len = a.max_len; g.F = a.d_ff;
     auto project = [&](const void* x, int K, const void* weight, const void* ln, void* out, int N) {
-      g.x = x; g.K = K; g.x_stride = K; g.w = weight; g.ln = ln; g.out = out; g.N = N;
+      g.x = x; g.K = K; g.w = weight; g.ln = ln; g.out = out; g.N = N;
     };
     project(a.hidden, a.d_model, w.wqkv, w.ln_self, ws + l.q, 3 * HD);
     g.kv = w.self_kv; g.seqlens = a.seqlens;
-    gemm<T, true, E_QKV>(go, g);
+    norm_gemm<T, E_QKV>(go, g);
     AttnStepParams s = {};
     s.B = a.B; s.H = a.H; s.q = ws + l.q; s.out = ws + l.attn;
     s.counters = (int32_t*)(ws + l.counters); s.part_ml = (float*)(ws + l.ml); s.part_o = (float*)(ws + l.o);
@@ -641,27 +896,29 @@ static int run_step(const t5b_decoder_step_args& a, cudaStream_t stream) {
     s.lens = a.seqlens; s.bias = (const float*)(ws + l.bias); s.md = a.max_distance; s.N = a.max_len; s.splits = l.self_splits;
     attention<T, true>(go, s, a.D);
     project(ws + l.attn, HD, w.wo, nullptr, a.hidden, a.d_model);
-    gemm<T, false, E_RESIDUAL>(go, g);
+    residual_gemm<T>(go, g);
 
     project(a.hidden, a.d_model, w.wcq, w.ln_cross, ws + l.q, HD);
-    gemm<T, true, E_STORE>(go, g);
+    norm_gemm<T, E_STORE>(go, g);
     s.k = w.cross_k; s.v = w.cross_v;
     s.k_stride_b = a.cross_stride_b; s.k_stride_h = a.cross_stride_h; s.k_stride_n = a.cross_stride_n;
     s.lens = a.enc_seqlens; s.bias = nullptr; s.N = a.enc_len; s.splits = l.cross_splits;
     attention<T, false>(go, s, a.D);
     project(ws + l.attn, HD, w.wco, nullptr, a.hidden, a.d_model);
-    gemm<T, false, E_RESIDUAL>(go, g);
+    residual_gemm<T>(go, g);
 
     project(a.hidden, a.d_model, w.wi, w.ln_ff, ws + l.act, a.gated ? 2 * a.d_ff : a.d_ff);
-    if (a.gated) gemm<T, true, E_GATED>(go, g);
-    else gemm<T, true, E_RELU>(go, g);
+    if (a.gated) norm_gemm<T, E_GATED>(go, g);
+    else norm_gemm<T, E_RELU>(go, g);
     project(ws + l.act, a.d_ff, w.wff, nullptr, a.hidden, a.d_model);
-    gemm<T, false, E_RESIDUAL>(go, g);
+    residual_gemm<T>(go, g);
   }
   GemmParams g = {};
-  g.B = a.B; g.eps = a.eps; g.x_scale = a.lm_scale; g.x = a.hidden; g.K = a.d_model; g.x_stride = a.d_model;
+  g.B = a.B; g.eps = a.eps; g.x_scale = a.lm_scale; g.x = a.hidden; g.K = a.d_model;
   g.w = a.lm_head; g.ln = a.final_ln; g.out = a.logits; g.N = a.vocab; g.cand = (float2*)(ws + l.cand);
-  gemm<T, true, E_LOGITS>(go, g);
+  if (a.B <= 16) launch_logits<T, 1>(go, g);
+  else if (a.B <= 32) launch_logits<T, 2>(go, g);
+  else launch_logits<T, 4>(go, g);
   go(step_choose_kernel<T>, dim3((unsigned)a.B, 1, 1), 256, 0, (const float2*)(ws + l.cand), l.n_cand, a.tokens, a.tokens_stride,
      a.seqlens, (const T*)a.embedding, (T*)a.hidden, a.d_model, a.max_len);
   return go.status;

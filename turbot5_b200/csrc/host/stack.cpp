@@ -697,6 +697,39 @@ struct DecodeSession {
     seqlens.fill_(1);
   }
   void step() { check_status(t5b_decoder_step(&a, stream_of(hidden.device())), "decoder step"); }
+
+  // `n` steps.  A step is a chain of one to two hundred launches of 2-4 us each, about what the host needs to issue
+  // one; from a few steps on the chain is recorded once (a CUDA graph on a stream of its own: nothing in it
+  // depends on the step) and launched n times.
+  void run(int64_t n) {
+    const cudaStream_t stream = stream_of(hidden.device());
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) cudaGetLastError();
+    if (n < kGraphSteps || capturing != cudaStreamCaptureStatusNone) {
+      for (int64_t i = 0; i < n; ++i) step();
+      return;
+    }
+    step();                            // kernel attributes are set by a kernel's first launch, outside a capture
+    cudaStream_t side = nullptr;
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    int st = T5B_ERR_LAUNCH;
+    if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      st = t5b_decoder_step(&a, side);
+      if (cudaStreamEndCapture(side, &graph) != cudaSuccess) st = T5B_ERR_LAUNCH;
+    }
+    if (st == T5B_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) st = T5B_ERR_LAUNCH;
+    for (int64_t i = 1; st == T5B_OK && i < n; ++i)
+      if (cudaGraphLaunch(exec, stream) != cudaSuccess) st = T5B_ERR_LAUNCH;
+    // an executable graph may be destroyed while its launches are still running: it is freed when they are done
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    if (side) cudaStreamDestroy(side);
+    if (st != T5B_OK) cudaGetLastError();
+    check_status(st, "decoder step");
+  }
+  static constexpr int64_t kGraphSteps = 6;
 };
 
 DecodeSession& session_arg(PyObject* o) {
@@ -795,7 +828,7 @@ PyObject* py_decode_session_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const c10::cuda::CUDAGuard guard(d.hidden.device());
   {
     pybind11::gil_scoped_release nogil;
-    for (int64_t i = 0; i < steps; ++i) d.step();
+    d.run(steps);
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
