@@ -589,3 +589,24 @@ def test_sliding_window_refuses_what_it_cannot_do():
         t5b.flash_attention_with_fusing_bias(q.float(), q.float(), q.float(), None, sm_scale=1.0, window=128)
     with pytest.raises(NotImplementedError):       # not together with the causal mask
         t5b.flash_attention_with_fusing_bias(q, q, q, None, causal=True, sm_scale=1.0, window=128)
+
+
+# edges of the CUDA-core kernel's tiles (32 or 64 rows, 32 or 64 keys), both row counts (64 from 64 x 148 rows on)
+@pytest.mark.parametrize("B,H,M,N,D,causal", [
+    (1, 1, 1, 1, 64, False), (1, 2, 31, 63, 64, False), (1, 2, 33, 65, 64, True), (2, 3, 64, 64, 32, True),
+    (1, 2, 65, 129, 16, False), (1, 2, 130, 33, 128, False), (1, 1, 97, 31, 128, True), (1, 2, 5, 0, 64, False),
+    (4, 19, 129, 129, 64, True), (4, 19, 127, 200, 128, False), (4, 19, 128, 64, 16, False), (4, 19, 131, 190, 32, True)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_cuda_core_forward_tile_edges(B, H, M, N, D, causal, aligned):
+    t5b = _ops()
+    pad = 0 if aligned else 1                   # rows that start one element past a vector's boundary
+    q, k, v = (seeded((B, H, n, D + pad), s)[..., pad:] for n, s in ((M, 1), (N, 2), (N, 3)))
+    table = seeded((32, H), 4, 0.5)
+    qd, kd, vd = (t.cuda() if aligned else torch.nn.functional.pad(t, (pad, 0)).cuda()[..., pad:] for t in (q, k, v))
+    out, lse = t5b.flash_attention_with_fusing_bias(qd, kd, vd, table.cuda(), causal=causal, sm_scale=0.5, return_lse=True)
+    assert out.dtype == torch.float32
+    if N == 0:
+        assert (out == 0).all() and torch.isneginf(lse).all()
+        return
+    want = orc.attention_basic(q, k, v, table, causal=causal, sm_scale=0.5, compute_dtype=torch.float64)
+    check_close(out, want, torch.float32, str((B, H, M, N, D, causal, aligned)))
