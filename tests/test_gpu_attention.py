@@ -610,3 +610,50 @@ def test_cuda_core_forward_tile_edges(B, H, M, N, D, causal, aligned):
         return
     want = orc.attention_basic(q, k, v, table, causal=causal, sm_scale=0.5, compute_dtype=torch.float64)
     check_close(out, want, torch.float32, str((B, H, M, N, D, causal, aligned)))
+
+
+# Causal tiles are dealt over a group of (batch, head) pairs; the groups here are 34 and 33 pairs.  A tile does not
+# depend on the order, so every pair has the bits it has alone.
+def test_causal_tile_order_covers_every_pair():
+    t5b = _ops()
+    H, L, D = 67, 4096 - 37, 64
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v, do = (torch.randn((1, H, L, D), generator=g, device="cuda").bfloat16() * s for s in (0.3, 0.3, 1, 1))
+    table = (torch.randn((32, H), generator=g, device="cuda") * 0.1).bfloat16()
+
+    def both(*t):
+        t = [x.detach().contiguous().requires_grad_() for x in t]
+        out = t5b.flash_attention_with_fusing_bias(*t, causal=True, sm_scale=1.0)
+        return out, t
+
+    out, ins = both(q, k, v, table)
+    grads = torch.autograd.grad(out, ins, do)
+    for h in (0, 1, 33, 34, 65, 66):
+        s = slice(h, h + 1)
+        o1, in1 = both(q[:, s], k[:, s], v[:, s], table[:, s])
+        g1 = torch.autograd.grad(o1, in1, do[:, s].contiguous())
+        assert torch.equal(out[:, s], o1)
+        for a, b in zip(grads[:3], g1[:3]):
+            assert torch.equal(a[:, s], b)
+        torch.testing.assert_close(grads[3][:, s], g1[3], rtol=2e-2, atol=1e-3)
+    t5b.check_device_status()
+
+
+# One kernel per form of call: every form against the CUDA-core kernel, on sizes with and without a ragged edge and
+# with the diagonal inside, at the edge of and outside the bias table's range (md 40 and 128).
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (64, torch.float16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("M,N,causal,off,md", [(256, 256, False, None, 128), (200, 333, False, 0, 40), (513, 513, True, None, 128),
+                                               (300, 700, True, None, 40), (256, 1024, False, -500, 128), (256, 1024, True, 900, 40)])
+def test_every_form_of_call_matches_the_cuda_core_kernel(D, dtype, M, N, causal, off, md):
+    t5b = _ops()
+    B, H = 2, 3
+    q, k, v = (seeded((B, H, n, D), s, dtype=dtype).cuda() * c for n, s, c in ((M, 1, 0.5), (N, 2, 0.5), (N, 3, 1)))
+    table = seeded((32, H), 4, 0.3, dtype=dtype).cuda()
+    kw = dict(causal=causal, sm_scale=0.7, MAX_DISTANCE=md)
+    got, want = (t5b.flash_attention_with_fusing_bias(q, k, v, table, kernel=kn, q_pos_offset=off, **kw) for kn in ("tcgen05", "simt"))
+    check_close(got, want, dtype)
+    flat = [t.transpose(1, 2).reshape(-1, H, D) for t in (q, k, v)]
+    cu_q, cu_k = (torch.arange(B + 1, dtype=torch.int32, device="cuda") * n for n in (M, N))
+    got, want = (t5b.flash_attention_with_fusing_bias_varlen(*flat, table, cu_q, cu_k, M, N, kernel=kn, **kw) for kn in ("tcgen05", "simt"))
+    check_close(got, want, dtype)
+    t5b.check_device_status()

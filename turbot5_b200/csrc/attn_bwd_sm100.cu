@@ -201,8 +201,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       part = ee - tail_slot * parts;
       tile_lin = e.q_tail_first + tail_slot;
     }
-    const int tx = tile_lin % p.tiles_x;
-    const int hb = tile_lin / p.tiles_x;
+    int tx, hb;
+    dense_order(p, tile_lin, p.tiles_x, tx, hb);
     h = hb % p.H;
     batch_idx = hb / p.H;
     w = dense_tile<BM>(p, tx, batch_idx);
@@ -682,8 +682,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
       part = ee - tail_slot * parts;
       tile_lin = e.k_tail_first + tail_slot;
     }
-    const int tx = tile_lin % tiles_k;
-    const int hb = tile_lin / tiles_k;
+    int tx, hb;
+    dense_order(p, tile_lin, tiles_k, tx, hb);
     h = hb % p.H;
     batch_idx = b = hb / p.H;
     key0 = tx * BM;
@@ -1262,8 +1262,8 @@ attn_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gri
       part = ee - tail_slot * parts;
       tile_lin = e.k_tail_first + tail_slot;
     }
-    const int tx = tile_lin % tiles_k;
-    const int hb = tile_lin / tiles_k;
+    int tx, hb;
+    dense_order(p, tile_lin, tiles_k, tx, hb);
     h = hb % p.H;
     batch_idx = b = hb / p.H;
     key0 = tx * BM;

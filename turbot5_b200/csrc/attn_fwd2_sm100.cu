@@ -162,8 +162,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q,
       part = e - tail_slot * parts;
       tile_lin = p.tail_first + tail_slot;
     }
-    const int tx = tile_lin % p.tiles_x;
-    const int hb = tile_lin / p.tiles_x;
+    int tx, hb;
+    dense_order(p, tile_lin, p.tiles_x, tx, hb);
     h = hb % p.H;
     batch_idx = hb / p.H;
     w = dense_tile<BLOCK_M>(p, tx, batch_idx);

@@ -113,6 +113,19 @@ __host__ __device__ inline size_t smem_bytes(int lut_entries) {
 }
 
 
+// What is known of the call when a kernel is compiled.  Work-item decoding, masks and the merge of a split last wave
+// that a call cannot need still shift the kernel's register allocation, which sits at its limit: with the causal
+// tile order in one kernel for all calls, calls without a mask lost 1-3 %.
+enum {
+  MODE_ANY = 0,   // nothing (head dims 16 and 32, the sliding window, the polynomial exponential)
+  MODE_CAUSAL,    // dense, causal
+  MODE_SPLIT,     // dense, no mask, the last wave split along the keys
+  MODE_FULL,      // dense, no mask, nothing split
+  MODE_PACKED,    // packed sequences, causal or not
+  MODE_LOCAL,     // block-local
+  N_MODES
+};
+
 // kPoly: of every 8 column pairs of an unmasked tile, this many take their exponentials on the FMA
 // pipe (PolyExp above) instead of the exponential unit; 8 = all of them (used by the parity tests).
 // kWindow: the sliding-window mode is compiled into a kernel of its own (with it in the plain kernel
@@ -120,17 +133,14 @@ __host__ __device__ inline size_t smem_bytes(int lut_entries) {
 // 264 bytes and the 8k forward went from 0.577 to 0.67 ms).
 // kNarrow: head dims 16 and 32 (run as head dim 64, see the epilogue) have kernels of their own for the
 // same reason: the column test in the epilogue, outside every loop, cost the plain kernel 3 %.
-template <bool kBf16, int HD, int kPoly, bool kWindow = false, bool kNarrow = false>
-__global__ void __launch_bounds__(HD == 64 ? 288 : MAX_THREADS, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
-                const __grid_constant__ CUtensorMap tmap_k,
-                const __grid_constant__ CUtensorMap tmap_v,
-                const __grid_constant__ AttnParams p,
-                const __grid_constant__ BucketSpec spec) {
+template <bool kBf16, int HD, int kPoly, bool kWindow, bool kNarrow, int kMode>
+__device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmap_q, const CUtensorMap& tmap_k, const CUtensorMap& tmap_v,
+                                              const AttnParams& p, const BucketSpec& spec) {
   using G = Geo<HD>;
   // head dim 64: warp 8 does the loads and the matrix products (288 threads); head dim 128: the
   // loads keep a warp of their own (its tiles are shorter, the refill has less slack)
   constexpr bool kOneIoThread = HD == 64;
+  constexpr bool kSplits = kMode == MODE_ANY || kMode == MODE_SPLIT;
   constexpr int NUM_THREADS = kOneIoThread ? 288 : MAX_THREADS;
   constexpr int WARP_MMA = kOneIoThread ? 8 : 9;
   constexpr int BN = G::BN, NSUB = G::NSUB, SUB_Q = G::SUB_Q, SUB_KV = G::SUB_KV;
@@ -158,9 +168,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
   TileWork* shared_work = reinterpret_cast<TileWork*>(&ctl->work[0]);
   TileWork w;
   int h, batch_idx = 0, part = 0, parts = 1, tail_slot = 0;
-  if (p.cu_q == nullptr) {
+  if (kMode == MODE_CAUSAL) {
+    int tx, hb;
+    dense_order(p, (int)blockIdx.x, p.tiles_x, tx, hb);
+    h = hb % p.H;
+    batch_idx = hb / p.H;
+    w = dense_tile<BM>(p, tx, batch_idx);
+  } else if (kMode != MODE_PACKED && (kMode != MODE_ANY || p.cu_q == nullptr)) {
     int tile_lin = (int)blockIdx.x;
-    if (tile_lin >= p.tail_first) {
+    if (kSplits && tile_lin >= p.tail_first) {
       const int e = tile_lin - p.tail_first;
       parts = p.tail_parts;
       tail_slot = e / parts;
@@ -191,7 +207,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
   // scores are the bare bias) and the TMA zero fill supplies them.  So the key range becomes
   // [n_base, len_k) with a negative n_base for the first block and len_k past the tensor's end.
   int n_base = 0;
-  if (p.local_block > 0) {
+  if (kMode == MODE_LOCAL || (kMode == MODE_ANY && p.local_block > 0)) {
     const int bl = p.M < p.local_block ? p.M : p.local_block;      // a shorter sequence is one block
     const int blk = q_row0 / bl;
     n_base = (blk - 1) * bl;
@@ -199,9 +215,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
   }
 
   const int window = kWindow ? p.window : 0;
+  const bool causal = kMode == MODE_CAUSAL || ((kMode == MODE_ANY || kMode == MODE_PACKED) && p.causal);
   // keys this tile can see
   int kv_end = len_k;
-  if (p.causal) kv_end = min(len_k, qpos0 + rows_in_tile);
+  if (causal) kv_end = min(len_k, qpos0 + rows_in_tile);
   // Sliding window (T5LocalAttention with its padding mask: |n - query| < window over the valid keys):
   // the tile walks the key tiles that hold a visible key for any of its rows.
   if (window > 0) {
@@ -450,7 +467,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (lane == 0) mbar_arrive(bar(BAR_S_FREE));
 
       // tile classification (uniform over the block)
-      const bool need_mask = (n0 + BN > len_k) || (p.causal && (n0 + BN - 1 > qpos0)) ||
+      const bool need_mask = (n0 + BN > len_k) || (causal && (n0 + BN - 1 > qpos0)) ||
                              (window > 0 && (n0 <= qpos0 + BM - 1 - window || n0 + BN - 1 >= qpos0 + window));
       int bias_mode = 0;            // 0 none, 1 constant over the tile, 2 per element
       float bias_const = 0.f;
@@ -483,10 +500,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
             }
           top_raw = fmaxf(fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)), fmaxf(fmaxf(m4, m5), fmaxf(m6, m7)));
           mx = fmaf(top_raw, scale, bias_const);
+        } else if (!need_mask && bias_mode == 2) {
+          // near the diagonal, every column visible: column c of this tile reads brow[c] of the padded table
+          const float* brow = lut + (n0 + c0 - qpos + md + LUT_PAD);
+          #pragma unroll
+          for (int c = 0; c < NCH; ++c) {
+            #pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              float x0 = brow[c * 32 + i], x1 = brow[c * 32 + i + 1], x2 = brow[c * 32 + i + 2], x3 = brow[c * 32 + i + 3];
+              fma2v(x0, x1, __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]), scale, x0, x1);
+              fma2v(x2, x3, __uint_as_float(sv[c][i + 2]), __uint_as_float(sv[c][i + 3]), scale, x2, x3);
+              sv[c][i] = __float_as_uint(x0);     sv[c][i + 1] = __float_as_uint(x1);
+              sv[c][i + 2] = __float_as_uint(x2); sv[c][i + 3] = __float_as_uint(x3);
+              m0 = fmaxf(m0, x0); m1 = fmaxf(m1, x1); m2 = fmaxf(m2, x2); m3 = fmaxf(m3, x3);
+            }
+            asm volatile("" ::: "memory");   // keep the table reads of one chunk from piling up in registers
+          }
+          mx = max3(fmaxf(m0, m1), m2, m3);
+          top_raw = mx;
         } else {
           // per-row window into the padded table: column c of this tile reads brow[c]
           const float* brow = lut + (n0 + c0 - qpos + md + LUT_PAD);
-          int n_valid = (p.causal ? min(len_k, qpos + 1) : len_k) - n0 - c0;   // columns < n_valid are visible
+          int n_valid = (causal ? min(len_k, qpos + 1) : len_k) - n0 - c0;   // columns < n_valid are visible
           int n_lo = -(1 << 30);                                               // ... from column n_lo on
           if (window > 0) {
             n_valid = min(n_valid, qpos + window - n0 - c0);
@@ -498,7 +533,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
             for (int i = 0; i < 32; ++i) {
               const float bias = bias_mode == 2 ? brow[c * 32 + i] : bias_const;
               float x = fmaf(__uint_as_float(sv[c][i]), scale, bias);
-              if (need_mask && (c * 32 + i >= n_valid || c * 32 + i < n_lo)) x = -INFINITY;
+              if (need_mask && (c * 32 + i >= n_valid || (kWindow && c * 32 + i < n_lo))) x = -INFINITY;
               sv[c][i] = __float_as_uint(x);
               if ((i & 3) == 0) m0 = fmaxf(m0, x); else if ((i & 3) == 1) m1 = fmaxf(m1, x);
               else if ((i & 3) == 2) m2 = fmaxf(m2, x); else m3 = fmaxf(m3, x);
@@ -664,7 +699,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
         for (int i = 0; i < 32; ++i) o[32 * c + i] = __uint_as_float(v[i]);
       }
       bool write_out = row_ok;
-      if (parts > 1 && row_ok) {
+      if (kSplits && parts > 1 && row_ok) {
         // This block saw only part of the keys.  Publish (max, sum, unnormalised O) for this
         // row half; the last of the `parts` blocks to arrive merges them (no waiting).
         const int64_t slot = (int64_t)tail_slot * parts + part;
@@ -726,7 +761,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
         if (p.lse != nullptr && half == 0) {
           const float lse = l_sum > 0.f ? (m_use + log2f(l_sum)) * kLn2 : -INFINITY;
-          if (p.cu_q == nullptr) p.lse[((int64_t)batch_idx * p.H + h) * p.M + row] = lse;
+          if (kMode != MODE_PACKED && (kMode != MODE_ANY || p.cu_q == nullptr)) p.lse[((int64_t)batch_idx * p.H + h) * p.M + row] = lse;
           else p.lse[row * p.H + h] = lse;
         }
       }
@@ -741,6 +776,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q,
     tc_fence_after();
     tmem_dealloc(tmem, TMEM_COLS);
   }
+}
+
+#define T5B_FWD_ARGS \
+  const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, \
+  const __grid_constant__ AttnParams p, const __grid_constant__ BucketSpec spec
+
+// the plain kernel merges the parts of a split last wave; its special forms take any call
+template <bool kBf16, int HD, int kPoly, bool kWindow = false, bool kNarrow = false>
+__global__ void __launch_bounds__(HD == 64 ? 288 : MAX_THREADS, 2) attn_fwd_kernel(T5B_FWD_ARGS) {
+  attn_fwd_body<kBf16, HD, kPoly, kWindow, kNarrow, kPoly != 8 && !kWindow && !kNarrow ? MODE_SPLIT : MODE_ANY>(tmap_q, tmap_k, tmap_v, p, spec);
+}
+template <bool kBf16, int HD, int kMode>
+__global__ void __launch_bounds__(HD == 64 ? 288 : MAX_THREADS, 2) attn_fwd_case_kernel(T5B_FWD_ARGS) {
+  attn_fwd_body<kBf16, HD, HD == 64 ? T5B_FWD_POLY64 : 0, false, false, kMode>(tmap_q, tmap_k, tmap_v, p, spec);
 }
 
 // ------------------------------------------------------------------ host side
@@ -855,24 +904,38 @@ int sm100_attention_fwd(const t5b_attn_args& a, const BucketSpec& spec, cudaStre
     grid = dim3((unsigned)blocks, 1, 1);
   }
   if (grid.y > 65535 || grid.z > 65535) return T5B_ERR_SHAPE;
-  // kernel variant: [head dim 128][bf16][0: default, 1: every exponential on the FMA pipe, 2: sliding window,
-  // 3: default for head dims 16 and 32].  At head dim 64 the variants 1 and 2 also take the narrow heads.
+  // [head dim 128][bf16][mode]; MODE_ANY: head dims 16 and 32
   using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, AttnParams, BucketSpec);
-  static const KernelFn kernels[2][2][4] = {
-      {{attn_fwd_kernel<false, 64, T5B_FWD_POLY64>, attn_fwd_kernel<false, 64, 8, false, true>,
-        attn_fwd_kernel<false, 64, 0, true, true>, attn_fwd_kernel<false, 64, T5B_FWD_POLY64, false, true>},
-       {attn_fwd_kernel<true, 64, T5B_FWD_POLY64>, attn_fwd_kernel<true, 64, 8, false, true>,
-        attn_fwd_kernel<true, 64, 0, true, true>, attn_fwd_kernel<true, 64, T5B_FWD_POLY64, false, true>}},
-      {{attn_fwd_kernel<false, 128, 0>, attn_fwd_kernel<false, 128, 8>, attn_fwd_kernel<false, 128, 0, true>, nullptr},
-       {attn_fwd_kernel<true, 128, 0>, attn_fwd_kernel<true, 128, 8>, attn_fwd_kernel<true, 128, 0, true>, nullptr}}};
-  int all_poly = a.window > 0 ? 2 : (a.kernel == T5B_KERNEL_TCGEN05_POLYEXP ? 1 : 0);
-  if (all_poly == 0 && a.D < 64) all_poly = 3;
-  const KernelFn kern = kernels[HD == 64 ? 0 : 1][bf16 ? 1 : 0][all_poly];
+#define T5B_FWD_MODES(BF16, HD, ANY, SPLIT) \
+  {ANY, attn_fwd_case_kernel<BF16, HD, MODE_CAUSAL>, SPLIT, attn_fwd_case_kernel<BF16, HD, MODE_FULL>, \
+   attn_fwd_case_kernel<BF16, HD, MODE_PACKED>, attn_fwd_case_kernel<BF16, HD, MODE_LOCAL>}
+  static const KernelFn kernels[2][2][N_MODES] = {
+      {T5B_FWD_MODES(false, 64, (attn_fwd_kernel<false, 64, T5B_FWD_POLY64, false, true>), (attn_fwd_kernel<false, 64, T5B_FWD_POLY64>)),
+       T5B_FWD_MODES(true, 64, (attn_fwd_kernel<true, 64, T5B_FWD_POLY64, false, true>), (attn_fwd_kernel<true, 64, T5B_FWD_POLY64>))},
+      {T5B_FWD_MODES(false, 128, nullptr, (attn_fwd_kernel<false, 128, 0>)),
+       T5B_FWD_MODES(true, 128, nullptr, (attn_fwd_kernel<true, 128, 0>))}};
+#undef T5B_FWD_MODES
+  // every exponential on the FMA pipe; sliding window.  At head dim 64 both also take the narrow heads.
+  static const KernelFn special[2][2][2] = {
+      {{attn_fwd_kernel<false, 64, 8, false, true>, attn_fwd_kernel<false, 64, 0, true, true>},
+       {attn_fwd_kernel<true, 64, 8, false, true>, attn_fwd_kernel<true, 64, 0, true, true>}},
+      {{attn_fwd_kernel<false, 128, 8>, attn_fwd_kernel<false, 128, 0, true>},
+       {attn_fwd_kernel<true, 128, 8>, attn_fwd_kernel<true, 128, 0, true>}}};
+  int variant;
+  if (a.window > 0) variant = N_MODES + 1;
+  else if (a.kernel == T5B_KERNEL_TCGEN05_POLYEXP) variant = N_MODES;
+  else if (a.D < 64) variant = MODE_ANY;
+  else if (varlen) variant = MODE_PACKED;
+  else if (a.local_block > 0) variant = MODE_LOCAL;
+  else if (a.causal) variant = MODE_CAUSAL;
+  else variant = p.tail_parts > 1 ? MODE_SPLIT : MODE_FULL;
+  const KernelFn kern = variant < N_MODES ? kernels[HD == 64 ? 0 : 1][bf16 ? 1 : 0][variant]
+                                          : special[HD == 64 ? 0 : 1][bf16 ? 1 : 0][variant - N_MODES];
   // opt in to > 48 KB of dynamic shared memory once per device and kernel (any thread may get here first)
-  static std::atomic<bool> attr_set[64][16];
+  static std::atomic<bool> attr_set[64][4 * (N_MODES + 2)];
   int dev = 0;
   cudaGetDevice(&dev);
-  const int which = (bf16 ? 1 : 0) + (HD == 64 ? 0 : 2) + 4 * all_poly;
+  const int which = (bf16 ? 1 : 0) + (HD == 64 ? 0 : 2) + 4 * variant;
   const size_t smem_max = HD == 64 ? smem_bytes<64>(2 * 2048 + 1 + 2 * LUT_PAD) : smem_bytes<128>(2 * 2048 + 1 + 2 * LUT_PAD);
   if (dev < 0 || dev >= 64 || !attr_set[dev][which].load(std::memory_order_acquire)) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max) != cudaSuccess) {
