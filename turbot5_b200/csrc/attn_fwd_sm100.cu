@@ -843,6 +843,12 @@ TailPlan sm100_tail_plan(const t5b_attn_args& a) {
   const int rem = (int)(n_total % slots);
   const int n_kv = (a.N + BN - 1) / BN;
   if (rem == 0) return t;
+  // Behind whole waves the blocks have drifted apart and a short last wave runs on alone, one block per SM and so nearly
+  // twice as fast; the parts' own set-up, scratch rows and merge cost more than that until a tile is long.  Split
+  // against unsplit, us.  Head dim 64: 8192 keys 578 / 597, 6144 278 / 301, 5120 243 / 258, 4096 329 / 322, 2048
+  // 197 / 183, 1024 125 / 120.  Head dim 128: 8192 866 / 913, 7168 725 / 726, 6144 414 / 397, 5120 264 / 248.
+  // A launch that does not fill one wave is always worth splitting (128 x 4000, 96 tiles: 47.7 / 51.6).
+  if (n_total > slots && a.N < (HD == 64 ? 4608 : 7168)) return t;
   int parts = slots / rem;
   if (parts > n_kv / 4) parts = n_kv / 4;     // at least four key tiles per part
   if (parts > 8) parts = 8;
