@@ -491,3 +491,45 @@ def test_gradients_at_a_long_sequence():
     check_close(got[0], want[0], dt, "out")
     for g, w, nm in zip(got[1:], want[1:], ("dq", "dk", "dv", "dtable")):
         check_grad_close(g, w, "4k " + nm, floor=2.0 if nm == "dtable" else 1e-6)
+
+
+@pytest.mark.parametrize("pin", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("layout", ["transposed", "stacked", "packed"])
+def test_gradients_with_saved_tensors_on_the_host(layout, dtype, pin):
+    """Saved-tensor hooks may give back another layout: `save_on_cpu` packs a transposed view into a dense tensor
+    (pinned) and a slice of a stacked projection into rows without the gaps (not pinned).  Same gradients as without
+    hooks, in every element, for views of a projection's rows and a table that is a slice itself."""
+    from turbot5_b200 import flash_attention_with_fusing_bias, flash_attention_with_fusing_bias_varlen
+    B, L, H, D = 2, 150, 3, 64
+    rows = seeded((B, L, 3 * H * D), 1, 0.5, dtype).cuda().requires_grad_()
+    wide = seeded((32, 2 * H), 2, 0.1, dtype).cuda().requires_grad_()
+    dout = seeded((B, H, L, D), 3, dtype=dtype).cuda()
+    cu = torch.tensor([0, 37, 37, B * L], dtype=torch.int32, device="cuda")
+
+    def grads():
+        table = wide[:, :H]
+        if layout == "packed":
+            q, k, v = (t.unflatten(-1, (H, D)) for t in rows.flatten(0, 1).split(H * D, -1))
+            out = flash_attention_with_fusing_bias_varlen(q, k, v, table, cu, cu, L, L, sm_scale=1.0)
+            return torch.autograd.grad(out, (rows, wide), dout.transpose(1, 2).flatten(0, 1))
+        parts = rows.split(H * D, -1) if layout == "stacked" else [t.contiguous() for t in rows.split(H * D, -1)]
+        q, k, v = (t.unflatten(-1, (H, D)).transpose(1, 2) for t in parts)
+        out = flash_attention_with_fusing_bias(q, k, v, table, causal=True, sm_scale=1.0)
+        return torch.autograd.grad(out, (rows, wide), dout)
+    want = grads()
+    with torch.autograd.graph.save_on_cpu(pin_memory=pin):
+        got = grads()
+    # the same kernels on the same values: only the order of the table gradient's additions may differ
+    assert torch.equal(got[0], want[0])
+    assert (got[1].float() - want[1].float()).norm() <= 1e-2 * want[1].float().norm()
+
+
+def test_a_hook_that_gives_back_another_tensor_is_refused():
+    from turbot5_b200 import flash_attention_with_fusing_bias
+    q = seeded((1, 2, 64, 64), 1, dtype=torch.bfloat16).cuda().requires_grad_()
+    for unpack in (lambda t: t.float(), lambda t: t[..., :32] if t.dim() == 4 else t):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            out = flash_attention_with_fusing_bias(q, q, q, None)
+            with pytest.raises(RuntimeError, match="saved tensor"):
+                out.sum().backward()

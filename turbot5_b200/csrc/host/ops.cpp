@@ -91,6 +91,19 @@ void set_common(AttnCall& c, const AttnOptions& o, double sm_scale) {
   a.window = o.window;
 }
 
+// Pointers and strides of the argument block, from the call's tensors.
+void set_operands(AttnCall& c) {
+  t5b_attn_args& a = c.args;
+  const int row = c.packed ? 0 : 2;                 // packed (rows, H, D); dense (B, H, rows, D)
+  auto batch = [&](const Tensor& t) { return c.packed ? 0 : t.stride(0); };
+  a.q = c.q.data_ptr(); a.k = c.k.data_ptr(); a.v = c.v.data_ptr(); a.out = c.out.data_ptr();
+  a.lse = (float*)ptr(c.lse);
+  a.q_stride_b = batch(c.q); a.q_stride_h = c.q.stride(1); a.q_stride_m = c.q.stride(row);
+  a.k_stride_b = batch(c.k); a.k_stride_h = c.k.stride(1); a.k_stride_n = c.k.stride(row);
+  a.v_stride_b = batch(c.v); a.v_stride_h = c.v.stride(1); a.v_stride_n = c.v.stride(row);
+  a.o_stride_b = batch(c.out); a.o_stride_h = c.out.stride(1); a.o_stride_m = c.out.stride(row);
+}
+
 }  // namespace
 
 // softmax(sm_scale * Q K^T + T5 bias(n - m) [+ causal mask]) V; the query at row m sits at key
@@ -118,13 +131,8 @@ void dense_forward(AttnCall& c, const Tensor& q, const Tensor& k, const Tensor& 
   }
   c.lse = want_lse ? empty_like_dense({B, H, M}, at::kFloat, q.device()) : Tensor();
   t5b_attn_args& a = c.args;
-  a.q = c.q.data_ptr(); a.k = c.k.data_ptr(); a.v = c.v.data_ptr(); a.out = c.out.data_ptr();
-  a.lse = (float*)ptr(c.lse);
+  set_operands(c);
   a.cu_seqlens_q = a.cu_seqlens_k = nullptr;
-  a.q_stride_b = c.q.stride(0); a.q_stride_h = c.q.stride(1); a.q_stride_m = c.q.stride(2);
-  a.k_stride_b = c.k.stride(0); a.k_stride_h = c.k.stride(1); a.k_stride_n = c.k.stride(2);
-  a.v_stride_b = c.v.stride(0); a.v_stride_h = c.v.stride(1); a.v_stride_n = c.v.stride(2);
-  a.o_stride_b = c.out.stride(0); a.o_stride_h = c.out.stride(1); a.o_stride_m = c.out.stride(2);
   a.B = (int32_t)B; a.H = (int32_t)H; a.M = (int32_t)M; a.N = (int32_t)N; a.D = (int32_t)D;
   a.total_q = a.total_k = 0;
   a.q_pos_offset = (int32_t)o.q_pos_offset.value_or(N - M);
@@ -172,13 +180,8 @@ void packed_forward(AttnCall& c, const Tensor& q, const Tensor& k, const Tensor&
     zero_async(c.lse);
   }
   t5b_attn_args& a = c.args;
-  a.q = c.q.data_ptr(); a.k = c.k.data_ptr(); a.v = c.v.data_ptr(); a.out = c.out.data_ptr();
-  a.lse = (float*)ptr(c.lse);
+  set_operands(c);
   a.cu_seqlens_q = (const int32_t*)c.cu_q.data_ptr(); a.cu_seqlens_k = (const int32_t*)c.cu_k.data_ptr();
-  a.q_stride_b = 0; a.q_stride_h = c.q.stride(1); a.q_stride_m = c.q.stride(0);
-  a.k_stride_b = 0; a.k_stride_h = c.k.stride(1); a.k_stride_n = c.k.stride(0);
-  a.v_stride_b = 0; a.v_stride_h = c.v.stride(1); a.v_stride_n = c.v.stride(0);
-  a.o_stride_b = 0; a.o_stride_h = c.out.stride(1); a.o_stride_m = c.out.stride(0);
   a.B = (int32_t)(cu_q.numel() - 1); a.H = (int32_t)H; a.M = (int32_t)o.max_q; a.N = (int32_t)o.max_k; a.D = (int32_t)D;
   a.total_q = (int32_t)Tq; a.total_k = (int32_t)k.size(0);
   a.q_pos_offset = 0;
@@ -201,10 +204,6 @@ void attention_backward(AttnCall& c, const Tensor& dout_in, const Tensor& dq, co
   t5b_attn_bwd_args g;
   g.fwd = c.args;
   t5b_attn_args& a = g.fwd;
-  a.out = c.out.data_ptr(); a.lse = (float*)c.lse.data_ptr();
-  a.o_stride_h = c.out.stride(1);
-  a.o_stride_b = c.packed ? 0 : c.out.stride(0);
-  a.o_stride_m = c.packed ? c.out.stride(0) : c.out.stride(2);
   a.workspace = nullptr; a.workspace_bytes = 0;
   g.dout = dout.data_ptr();
   g.do_stride_h = dout.stride(1);
@@ -246,13 +245,23 @@ struct AttentionNode : public Node {
     c.q = q.unpack(); c.k = k.unpack(); c.v = v.unpack();
     c.out = out.unpack(shared_from_this()); c.lse = lse.unpack(shared_from_this());
     if (has_table) c.table = table.unpack();
-    // the kernels read what the forward call read (contiguous copies of inputs with a strided last dim)
+    // A saved-tensor hook may have given back any layout (or, by mistake, another tensor): the argument block is
+    // made anew from what was unpacked.
+    const t5b_attn_args& a = c.args;
+    auto is = [&](const Tensor& t, int64_t rows, int dtype) {
+      return t.is_cuda() && dtype_code(t.scalar_type()) == dtype &&
+             (c.packed ? t.sizes() == at::IntArrayRef({rows, a.H, a.D}) : t.sizes() == at::IntArrayRef({a.B, a.H, rows, a.D}));
+    };
+    const int64_t M = c.packed ? a.total_q : a.M, N = c.packed ? a.total_k : a.N;
+    TORCH_CHECK(is(c.q, M, a.dtype) && is(c.k, N, a.dtype) && is(c.v, N, a.dtype) && is(c.out, M, a.dtype) && c.lse.is_cuda() &&
+                    c.lse.scalar_type() == at::kFloat && c.lse.numel() == (c.packed ? M * a.H : a.B * a.H * M),
+                "a saved tensor of an attention call came back with another shape, type or device");
     c.q = unit_stride_last(c.q); c.k = unit_stride_last(c.k); c.v = unit_stride_last(c.v);
-    c.args.q = c.q.data_ptr(); c.args.k = c.k.data_ptr(); c.args.v = c.v.data_ptr();
-    if (has_table && c.table.stride(1) != 1) c.table = c.table.contiguous();
-    if (has_table) c.args.table = c.table.data_ptr();
+    c.out = unit_stride_last(c.out); c.lse = c.lse.contiguous();
     const at::Device dev = c.q.device();
     const c10::cuda::CUDAGuard guard(dev);
+    set_table(c, has_table ? c.table : Tensor(), a.H);
+    set_operands(c);
     const Tensor dq = empty_strided(c.q.sizes(), c.q.strides(), c.q.scalar_type(), dev);
     const Tensor dk = empty_strided(c.k.sizes(), c.k.strides(), c.k.scalar_type(), dev);
     const Tensor dv = empty_strided(c.v.sizes(), c.v.strides(), c.v.scalar_type(), dev);
