@@ -1,0 +1,79 @@
+"""What a stack's native passes must not change: every call that the module-by-module and operator-by-operator
+passes take (replaced modules, hooks, autocast, float32 norms, odd masks) gives their result, and is refused
+where they refuse it."""
+import pytest
+import torch
+from torch import nn
+
+from tests.test_gpu_t5_stack import _model as _fixture_model
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(dtype=torch.bfloat16, **over):
+    """A small model whose softmaxes are not one-hot (fan-in scaled weights)."""
+    model = _fixture_model(dtype, **{**dict(d_model=128, num_heads=4, d_ff=256), **over})
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if p.dim() > 1 and "shared" not in n:
+                p.mul_(12.5 * p.shape[-1] ** -0.5)
+    return model
+
+
+def _ids(B, L, seed=0):
+    return torch.randint(0, 128, (B, L), generator=torch.Generator().manual_seed(seed)).cuda()
+
+
+def _mask(lens, L):
+    return (torch.arange(L)[None] < torch.tensor(lens)[:, None]).long().cuda()
+
+
+def _rel(a, b):
+    return ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)).item()
+
+
+def _by_modules(stack):
+    """Context: the stack runs module by module (a hook on one of its modules selects that path)."""
+    import contextlib
+
+    @contextlib.contextmanager
+    def cm():
+        h = stack.block[0].layer[0].SelfAttention.q.register_forward_hook(lambda *a: None)
+        try:
+            yield
+        finally:
+            h.remove()
+    return cm()
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("width", [92, 108, 50, 200])
+def test_a_mask_of_another_shape_than_the_rows_is_refused(width, grad):
+    model = _model()
+    ids, dec = _ids(2, 100), _ids(2, 20, 1)
+    bad = _mask([width, width // 2], width)
+    with torch.set_grad_enabled(grad):
+        memory = model.encoder(ids)
+        for call in (lambda: model.encoder(ids, attention_mask=bad),
+                     lambda: model.decoder(dec, encoder_hidden_states=memory, encoder_attention_mask=bad),
+                     lambda: model(ids, dec, attention_mask=bad),
+                     lambda: model.encoder(ids, attention_mask=_mask([100, 90, 80], 100))):
+            with pytest.raises((RuntimeError, ValueError, IndexError)):
+                call()
+    with torch.no_grad(), pytest.raises((RuntimeError, ValueError, IndexError)):
+        model.encoder.forward_fused(ids, attention_mask=bad)
+    torch.cuda.synchronize()
+
+
+def test_a_memory_of_another_batch_than_the_rows_is_not_cut():
+    model = _model()
+    dec = _ids(2, 20, 1)
+    with torch.no_grad():
+        memory = model.encoder(_ids(4, 50))
+        with pytest.raises((RuntimeError, ValueError)):
+            model.decoder.forward_fused(dec, encoder_hidden_states=memory)
+        # the modules view the memory's rows as the decoder's batch; whatever they give, the stack gives too
+        got = model.decoder(dec, encoder_hidden_states=memory)
+        with _by_modules(model.decoder):
+            want = model.decoder(dec, encoder_hidden_states=memory)
+    assert _rel(got, want) < 2e-2

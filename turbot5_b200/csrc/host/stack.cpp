@@ -317,6 +317,23 @@ Tensor decoder_offsets(const PassInputs& in, int64_t B, int64_t S) {
 // memory rows the cross attention projects keys and values from
 Tensor memory_rows(const PassInputs& in) { return in.enc.defined() ? rows_of(in.enc) : Tensor(); }
 
+// Whether the rows, the memory and the plans of their masks belong together.  The gathers and scatters walk a plan's
+// destinations for as many rows as there are, and the attention calls take the batch from the rows, so nothing
+// else may get here; what the modules make of other sizes (an error, mostly) is theirs to say.
+bool matching(const PassInputs& in, bool decoder) {
+  const int64_t B = in.x.size(0), R = B * in.x.size(1);
+  if (in.packed && !in.cu.defined()) return false;
+  if (in.padded && (!in.cu.defined() || in.cu.numel() != B + 1 || !in.dest.defined() || in.dest.numel() != R)) return false;
+  if (!decoder) return !in.enc.defined();
+  if (!in.enc.defined() || in.packed || in.padded) return false;
+  if (in.enc_cu.defined() && in.enc_cu.numel() != B + 1) return false;
+  if (in.enc.dim() == 3) {
+    if (in.enc.size(0) != B) return false;
+    return !in.enc_cu.defined() || (in.enc_dest.defined() && in.enc_dest.numel() == B * in.enc.size(1));
+  }
+  return in.enc.dim() == 2 && in.enc_cu.defined() && !in.enc_dest.defined();
+}
+
 // ------------------------------------------------------------------ inference
 Tensor infer(const Stack& s, const Stacked& w, const PassInputs& in) {
   const int64_t B = in.x.size(0), S = in.x.size(1), R = B * S, HD = s.H * s.D;
@@ -632,6 +649,7 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!in.x.is_cuda() || in.x.dim() != 3 || in.x.size(2) != s.d || !supported(s, in.x.scalar_type())) Py_RETURN_NONE;
   if (in.enc.defined() && (in.enc.scalar_type() != in.x.scalar_type() || in.enc.size(-1) != s.d)) Py_RETURN_NONE;
   if (in.x.numel() == 0 || (in.enc.defined() && in.enc.numel() == 0)) Py_RETURN_NONE;
+  if (!matching(in, s.decoder)) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(in.x.device());
   bool grad = false;
   auto plist = param_list(s);
