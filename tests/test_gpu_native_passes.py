@@ -77,3 +77,28 @@ def test_a_memory_of_another_batch_than_the_rows_is_not_cut():
         with _by_modules(model.decoder):
             want = model.decoder(dec, encoder_hidden_states=memory)
     assert _rel(got, want) < 2e-2
+
+
+@torch.no_grad()
+def test_given_operators_serve_masked_and_packed_passes_too():
+    from turbot5_b200.t5 import _FusedOps
+
+    class Counting(_FusedOps):
+        calls = 0
+
+        @staticmethod
+        def rms_layer_norm(*a):
+            Counting.calls += 1
+            return _FusedOps.rms_layer_norm(*a)
+
+    model = _model()
+    ids, dec = _ids(3, 70), _ids(3, 9, 1)
+    mask = _mask([70, 31, 1], 70)
+    want = model.encoder.forward_fused(ids, attention_mask=mask)
+    got = model.encoder.forward_fused(ids, attention_mask=mask, ops=Counting)
+    assert Counting.calls == 1 and _rel(got, want) < 1e-2 and torch.count_nonzero(got[1, 31:]) == 0
+    packed, plan = model.encoder.forward_fused(ids, attention_mask=mask, packed_rows=110, return_packed=True, ops=Counting)
+    states = model.encoder.forward_fused(ids, attention_mask=mask, packed_rows=110, return_packed=True)[0]
+    want = model.decoder.forward_fused(dec, encoder_hidden_states=states, encoder_plan=plan)
+    got = model.decoder.forward_fused(dec, encoder_hidden_states=packed, encoder_plan=plan, ops=Counting)
+    assert _rel(got, want) < 1e-2

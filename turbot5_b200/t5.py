@@ -25,7 +25,8 @@ import torch
 from torch import nn
 
 from . import _native as nat
-from .attention import flash_attention_with_fusing_bias, flash_decoding_with_fusing_bias
+from .attention import (flash_attention_with_fusing_bias, flash_attention_with_fusing_bias_varlen,
+                        flash_decoding_with_fusing_bias)
 from .modules import (T5ATTENTION_TYPES, T5FlashAttention, T5LayerNorm, add_rms_layer_norm, gated_gelu,
                       rms_layer_norm)
 from .padding import get_unpad_plan, pad_rows, unpad_rows
@@ -293,7 +294,7 @@ class T5Stack(nn.Module):
                 raise ValueError("forward_fused covers full attention (attention_type='flash')")
         if seq_len is not None or ops is not None:
             return self._forward_fused_ops(input_ids, inputs_embeds, seq_len, group, overlap, ops or _FusedOps,
-                                           encoder_hidden_states)
+                                           encoder_hidden_states, attention_mask, packed_rows, return_packed, encoder_plan)
         if attention_mask is not None:
             return self._forward_fused_packed(input_ids, inputs_embeds, attention_mask, packed_rows, return_packed)
         x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
@@ -343,26 +344,42 @@ class T5Stack(nn.Module):
         if normed is None:
             raise NotImplementedError("forward_fused covers bf16/fp16 CUDA stacks (contiguous weights of one type, d_model "
                                       "a multiple of 8 and at most 2048, head dim 16, 32, 64 or 128)")
-        normed = normed[0]
-        n = normed.shape[0]
+        return self._unpacked(normed[0], plan, packed_rows, return_packed)
+
+    @staticmethod
+    def _unpacked(normed, plan, packed_rows, return_packed):
+        """Result of a packed pass from its rows (T, d_model)."""
+        n, total = normed.shape[0], plan.batch * plan.seqlen
         if packed_rows is not None:
             # a bound below the true token count would silently drop tokens: make that loud (NaN
             # everywhere) without reading anything back
             normed = normed.masked_fill(plan.cu_seqlens[-1] > n, float("nan"))
         if return_packed:
             return normed, plan
-        if packed_rows is not None and n < B * L:
+        if packed_rows is not None and n < total:
             # the scatter reads the packed row of every valid token: give it all of them
-            full = normed.new_full((B * L, normed.shape[-1]), float("nan"))
+            full = normed.new_full((total, normed.shape[-1]), float("nan"))
             full[:n] = normed
             normed = full
         return pad_rows(normed, plan)             # (B, L, d_model), zeros at padded positions
 
-    def _forward_fused_ops(self, input_ids, inputs_embeds, seq_len, group, overlap, ops, encoder_hidden_states):
+    def _forward_fused_ops(self, input_ids, inputs_embeds, seq_len, group, overlap, ops, encoder_hidden_states,
+                           attention_mask=None, packed_rows=None, return_packed=False, encoder_plan=None):
         """The fused pass operator by operator: sequence-parallel encoders (a collective per layer) and passes
         with other operators than the library's."""
         cfg = self.cfg
         x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
+        plan = tail = None
+        if attention_mask is not None:
+            plan = get_unpad_plan(attention_mask)
+            n = int(plan.cu_seqlens[-1]) if packed_rows is None else int(packed_rows)
+            n = min(max(n, 1), plan.batch * plan.seqlen)
+            x = unpad_rows(x, plan)[:n].unsqueeze(0)                  # (1, T, d_model): kept tokens, zero tail
+            cu = plan.cu_seqlens
+            if packed_rows is not None:
+                # rows past the last token: as in `_forward_fused_packed`
+                tail = (torch.arange(n, device=x.device) >= cu[-1])[:, None, None]
+                cu = cu.clamp(max=n)
         B, S, _ = x.shape
         H, D = cfg.num_heads, cfg.d_kv
         HD = H * D
@@ -370,14 +387,25 @@ class T5Stack(nn.Module):
         eps = cfg.layer_norm_epsilon
         table = self._table()
         heads = lambda t: t.unflatten(-1, (H, D)).transpose(1, 2)        # (B, L, H*D) -> (B, H, L, D) view
-        x = x.contiguous() if inputs_embeds is None else x.clone(memory_format=torch.contiguous_format)
+        x = x.contiguous() if (inputs_embeds is None or plan is not None) else x.clone(memory_format=torch.contiguous_format)
         normed = ops.rms_layer_norm(x, self.block[0].layer[0].layer_norm.weight, eps).to(x.dtype)
         if seq_len is not None:
             from . import sequence_parallel as sp
+        if encoder_plan is not None:
+            if encoder_plan.batch != B:
+                raise ValueError("encoder_plan was made for another batch size")
+            cu_dec = torch.arange(B + 1, dtype=torch.int32, device=x.device) * S
         for i, blk in enumerate(self.block):
             att, ffl = blk.layer[0].SelfAttention, blk.layer[-1]
             w = self._stacked_weights(i)
-            if seq_len is None:
+            if plan is not None:
+                qkv = nn.functional.linear(normed, w["qkv"])[0]                           # (T, 3*H*D)
+                q, k, v = (qkv[:, j * HD:(j + 1) * HD].unflatten(-1, (H, D)) for j in range(3))
+                attn = flash_attention_with_fusing_bias_varlen(q, k, v, table, cu, cu, plan.seqlen, plan.seqlen,
+                                                               causal=False, sm_scale=1.0, NUM_BUCKETS=nb, MAX_DISTANCE=md)
+                if tail is not None:
+                    attn = attn.masked_fill(tail, 0)
+            elif seq_len is None:
                 qkv = nn.functional.linear(normed, w["qkv"])
                 q, k, v = (heads(qkv[..., j * HD:(j + 1) * HD]) for j in range(3))
                 attn = ops.attention(q, k, v, table, self.is_decoder, 1.0, nb, md, 0).transpose(1, 2)
@@ -399,8 +427,16 @@ class T5Stack(nn.Module):
                 x, normed = ops.add_rms_layer_norm(x, o, ca.layer_norm.weight, eps, inplace=True)
                 catt = ca.EncDecAttention
                 ckv = nn.functional.linear(encoder_hidden_states, w["ckv"])
-                q = heads(nn.functional.linear(normed, catt.q.weight))
-                attn = ops.attention(q, heads(ckv[..., :HD]), heads(ckv[..., HD:]), None, False, 1.0, nb, md, 0).transpose(1, 2)
+                if encoder_plan is None:
+                    q = heads(nn.functional.linear(normed, catt.q.weight))
+                    attn = ops.attention(q, heads(ckv[..., :HD]), heads(ckv[..., HD:]), None, False, 1.0, nb, md, 0).transpose(1, 2)
+                else:
+                    # packed encoder states: every decoder sequence has S query rows, its keys are the valid
+                    # encoder tokens of the same batch row
+                    q = nn.functional.linear(normed, catt.q.weight).view(B * S, H, D)
+                    attn = flash_attention_with_fusing_bias_varlen(
+                        q, ckv[:, :HD].unflatten(-1, (H, D)), ckv[:, HD:].unflatten(-1, (H, D)), None, cu_dec,
+                        encoder_plan.cu_seqlens, S, encoder_plan.seqlen, causal=False, sm_scale=1.0)
                 o = nn.functional.linear(attn.reshape(B, S, HD), catt.o.weight)
             x, normed = ops.add_rms_layer_norm(x, o, ffl.layer_norm.weight, eps, inplace=True)
             ff = ffl.DenseReluDense
@@ -410,7 +446,7 @@ class T5Stack(nn.Module):
                 f = ff(normed)
             nxt = self.block[i + 1].layer[0].layer_norm if i + 1 < len(self.block) else self.final_layer_norm
             x, normed = ops.add_rms_layer_norm(x, f, nxt.weight, eps, inplace=True)
-        return normed
+        return normed if plan is None else self._unpacked(normed[0], plan, packed_rows, return_packed)
 
     # ---- generation with a preallocated cache (decoder only)
     def new_cache(self, encoder_hidden_states, max_len) -> DecoderCache:
