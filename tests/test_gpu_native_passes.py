@@ -102,3 +102,41 @@ def test_given_operators_serve_masked_and_packed_passes_too():
     want = model.decoder.forward_fused(dec, encoder_hidden_states=states, encoder_plan=plan)
     got = model.decoder.forward_fused(dec, encoder_hidden_states=packed, encoder_plan=plan, ops=Counting)
     assert _rel(got, want) < 1e-2
+
+
+def test_inference_under_autocast():
+    model = _model()
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    mask = _mask([70, 31], 70)
+    with torch.no_grad():
+        want, want_masked = model(ids, dec), model(ids, dec, attention_mask=mask)
+        with torch.autocast("cuda", torch.bfloat16):
+            assert _rel(model(ids, dec), want) < 2e-2
+            assert _rel(model(ids, dec, attention_mask=mask), want_masked) < 2e-2
+            assert _rel(model.encoder.forward_fused(ids, attention_mask=mask, packed_rows=110),
+                        model.encoder(ids, attention_mask=mask) * mask[..., None]) < 2e-2
+            tokens = model.generate(ids, attention_mask=mask, max_new_tokens=4, use_cuda_graph=False)
+    assert tokens.shape == (2, 4)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("what", ["norms", "table", "strided"])
+def test_inference_with_weights_the_native_pass_does_not_take(what):
+    """Norm weights or a bias table in float32 beside 16-bit matrices, and weights that are not contiguous: no
+    farther from the float32 model than the native pass is (rounded at the same points or at fewer; half as
+    much again for the chance of single roundings, which these softmaxes magnify)."""
+    model = _model()
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    mask = _mask([70, 31], 70)
+    exact = _model(torch.float32)
+    for p, e in zip(model.parameters(), exact.parameters()):
+        e.copy_(p)
+    exact, exact_masked = exact(ids, dec), exact(ids, dec, attention_mask=mask)
+    bound, bound_masked = 1.5 * _rel(model(ids, dec), exact), 1.5 * _rel(model(ids, dec, attention_mask=mask), exact_masked)
+    for n, p in model.named_parameters():
+        if (what == "norms" and "layer_norm" in n) or (what == "table" and "relative_attention_bias" in n):
+            p.data = p.data.float()
+        if what == "strided" and p.dim() == 2 and ("SelfAttention" in n or "DenseReluDense" in n) and "relative" not in n:
+            p.data = p.data.t().contiguous().t()
+    assert _rel(model(ids, dec), exact) <= bound < 0.2
+    assert _rel(model(ids, dec, attention_mask=mask), exact_masked) <= bound_masked < 0.2

@@ -252,8 +252,9 @@ class T5Stack(nn.Module):
     def forward_fused(self, input_ids=None, inputs_embeds=None, seq_len=None, group=None, overlap=True, ops=None,
                       encoder_hidden_states=None, attention_mask=None, packed_rows=None, return_packed=False,
                       encoder_plan=None):
-        """Forward pass without padding masks and without gradients, with the token-wise work fused
-        around the attention path: per encoder block eight launches -- stacked q/k/v projection,
+        """Forward pass without gradients, with the token-wise work fused around the attention path, as one
+        native launch sequence where that covers the call and operator by operator otherwise: per encoder
+        block eight launches -- stacked q/k/v projection,
         attention, output projection, residual add fused with the next RMSNorm, stacked wi_0|wi_1
         projection, gated GELU, wo projection, residual add + RMSNorm -- and five more per decoder
         block for the cross attention (q projection, stacked k/v projection of the encoder states,
@@ -295,8 +296,12 @@ class T5Stack(nn.Module):
         if seq_len is not None or ops is not None:
             return self._forward_fused_ops(input_ids, inputs_embeds, seq_len, group, overlap, ops or _FusedOps,
                                            encoder_hidden_states, attention_mask, packed_rows, return_packed, encoder_plan)
+        by_operators = lambda: self._forward_fused_ops(input_ids, inputs_embeds, None, None, False, _FusedOps,
+                                                       encoder_hidden_states, attention_mask, packed_rows, return_packed,
+                                                       encoder_plan)
         if attention_mask is not None:
-            return self._forward_fused_packed(input_ids, inputs_embeds, attention_mask, packed_rows, return_packed)
+            out = self._forward_fused_packed(input_ids, inputs_embeds, attention_mask, packed_rows, return_packed)
+            return by_operators() if out is None else out
         x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
         if encoder_plan is None:
             out = self._run_native(x, enc=encoder_hidden_states, need_plain=False)
@@ -307,10 +312,7 @@ class T5Stack(nn.Module):
                 raise ValueError("encoder_plan was made for another batch size")
             out = self._run_native(x, enc=encoder_hidden_states, enc_cu=encoder_plan.cu_seqlens, enc_max=encoder_plan.seqlen,
                                    need_plain=False)
-        if out is None:
-            raise NotImplementedError("forward_fused covers bf16/fp16 CUDA stacks (contiguous weights of one type, d_model "
-                                      "a multiple of 8 and at most 2048, head dim 16, 32, 64 or 128)")
-        return out
+        return by_operators() if out is None else out
 
     def _native_cache(self):
         state = self.__dict__.get("_native_state")
@@ -319,7 +321,7 @@ class T5Stack(nn.Module):
         return state.cache
 
     def _forward_fused_packed(self, input_ids, inputs_embeds, attention_mask, packed_rows, return_packed):
-        """The encoder pass over the valid tokens of a padded batch, packed once."""
+        """The native encoder pass over the valid tokens of a padded batch, packed once; None: not covered."""
         plan = get_unpad_plan(attention_mask)
         B, L = plan.batch, plan.seqlen
         tail, cu = False, plan.cu_seqlens
@@ -342,8 +344,7 @@ class T5Stack(nn.Module):
             tail, cu = True, plan.cu_seqlens.clamp(max=n)
         normed = self._run_native(x.unsqueeze(0), mode=1, cu=cu, max_len=L, zero_tail=tail, need_plain=False)
         if normed is None:
-            raise NotImplementedError("forward_fused covers bf16/fp16 CUDA stacks (contiguous weights of one type, d_model "
-                                      "a multiple of 8 and at most 2048, head dim 16, 32, 64 or 128)")
+            return None
         return self._unpacked(normed[0], plan, packed_rows, return_packed)
 
     @staticmethod
@@ -365,8 +366,9 @@ class T5Stack(nn.Module):
 
     def _forward_fused_ops(self, input_ids, inputs_embeds, seq_len, group, overlap, ops, encoder_hidden_states,
                            attention_mask=None, packed_rows=None, return_packed=False, encoder_plan=None):
-        """The fused pass operator by operator: sequence-parallel encoders (a collective per layer) and passes
-        with other operators than the library's."""
+        """The fused pass operator by operator: sequence-parallel encoders (a collective per layer), passes with
+        other operators than the library's, and calls that the native pass does not take (autocast, norm weights
+        or a bias table of another type than the matrices, weights that are not contiguous)."""
         cfg = self.cfg
         x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
         plan = tail = None
