@@ -140,3 +140,47 @@ def test_inference_with_weights_the_native_pass_does_not_take(what):
             p.data = p.data.t().contiguous().t()
     assert _rel(model(ids, dec), exact) <= bound < 0.2
     assert _rel(model(ids, dec, attention_mask=mask), exact_masked) <= bound_masked < 0.2
+
+
+class _Squared(nn.Module):
+    """A feed-forward layer with the names of the plain one and another activation."""
+
+    def __init__(self, old):
+        super().__init__()
+        self.wi, self.wo = old.wi, old.wo
+
+    def forward(self, x):
+        return self.wo(torch.relu(self.wi(x)).square())
+
+
+def test_a_replaced_feed_forward_module_is_the_one_that_runs():
+    model = _model(feed_forward_proj="relu")
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    plain = model.encoder.forward_fused(ids)
+    for stack in (model.encoder, model.decoder):
+        for blk in stack.block:
+            blk.layer[-1].DenseReluDense = _Squared(blk.layer[-1].DenseReluDense)
+    with torch.no_grad():
+        got, want = model.encoder.forward_fused(ids), model.encoder(ids)
+        assert _rel(got, want) < 2e-2 and _rel(plain, want) > 5e-2
+        logits = model(ids, dec)
+        want = model.logits(model.decoder(dec, encoder_hidden_states=want))
+        assert _rel(logits, want) < 3e-2
+        masked = model(ids, dec, attention_mask=_mask([70, 70], 70))
+        assert _rel(masked, want) < 3e-2
+
+
+def test_hooks_and_biases_of_a_feed_forward_layer_are_honoured():
+    model = _model(feed_forward_proj="relu")
+    ids = _ids(2, 70)
+    want_plain = model.encoder.forward_fused(ids)
+    seen = []
+    handle = model.encoder.block[0].layer[-1].DenseReluDense.register_forward_hook(lambda *a: seen.append(1))
+    got = model.encoder.forward_fused(ids)
+    handle.remove()
+    assert seen and _rel(got, want_plain) < 2e-2
+    wi = model.encoder.block[1].layer[-1].DenseReluDense.wi
+    wi.bias = nn.Parameter(torch.full((256,), 0.5, device="cuda", dtype=torch.bfloat16))
+    with torch.no_grad():
+        want = model.encoder(ids)
+    assert _rel(model.encoder.forward_fused(ids), want) < 2e-2 < _rel(want_plain, want)

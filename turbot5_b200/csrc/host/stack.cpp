@@ -70,6 +70,7 @@ struct Stack {
   double eps = 1e-6;
   bool plain = true;                     // every module is of the expected class and has no hooks
   bool flash = true;                     // every attention module is the full-attention one
+  bool plain_ff = true;                  // `plain` of the feed-forward layers alone
 };
 
 struct Names {
@@ -137,7 +138,7 @@ struct Walker {
 
 // dims: (heads, head dim, buckets, max distance, eps)
 Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t D, int nb, int md, double eps) {
-  Walker w{types};
+  Walker w{types}, wf{types};            // feed-forward layers are looked at apart
   Stack s;
   s.decoder = decoder; s.H = H; s.D = D; s.nb = nb; s.md = md; s.eps = eps;
   PyObject* blocks = PyDict_GetItemString(w.dict_of(stack, names().modules), "block");
@@ -165,11 +166,13 @@ Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t
     l.ln_ff = w.weight(ffl, "layer_norm", K_NORM);
     PyObject* ff = PyDict_GetItemString(w.dict_of(ffl, names().modules), "DenseReluDense");
     TORCH_CHECK(ff, "the feed-forward layer has no DenseReluDense");
-    s.gated = PyDict_GetItemString(w.dict_of(ff, names().modules), "wi_0") != nullptr;
-    w.look(ff, s.gated ? K_GATED : K_RELU);
-    l.wi0 = w.weight(ff, s.gated ? "wi_0" : "wi", K_LINEAR);
-    if (s.gated) l.wi1 = w.weight(ff, "wi_1", K_LINEAR);
-    l.wo = w.weight(ff, "wo", K_LINEAR);
+    const bool gated = PyDict_GetItemString(w.dict_of(ff, names().modules), "wi_0") != nullptr;
+    if (!s.layers.empty() && gated != s.gated) wf.plain = false;
+    s.gated = gated;
+    wf.look(ff, s.gated ? K_GATED : K_RELU);
+    l.wi0 = wf.weight(ff, s.gated ? "wi_0" : "wi", K_LINEAR);
+    if (s.gated) l.wi1 = wf.weight(ff, "wi_1", K_LINEAR);
+    l.wo = wf.weight(ff, "wo", K_LINEAR);
     s.layers.push_back(std::move(l));
   }
   TORCH_CHECK(!s.layers.empty(), "the stack has no blocks");
@@ -179,7 +182,8 @@ Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t
   s.final_ln = w.parameter(fin, "weight");
   s.d = s.final_ln.size(0);
   s.F = s.layers[0].wi0.size(0);
-  s.plain = w.plain;
+  s.plain = w.plain && wf.plain;
+  s.plain_ff = wf.plain;
   s.flash = w.flash;
   return s;
 }
@@ -632,8 +636,9 @@ PyObject* py_new_stack_cache(PyObject*, PyObject* const*, Py_ssize_t) {
 // stack_forward(stack, types, cache, decoder, heads, d_kv, buckets, max_distance, eps, need_plain,
 //               x, mode, cu, dest, max_len, zero_tail, enc, enc_cu, enc_dest, enc_max)
 // mode: 0 plain rows, 1 packed rows (cu), 2 padded rows with a mask (cu, dest).
-// Returns None when the pass is not one of the native ones (types, sizes; with `need_plain` or in training also
-// when a module of the stack is not of the expected class or carries hooks): the caller then runs the modules.
+// Returns None when the pass is not one of the native ones (types, sizes, a feed-forward layer of another class or
+// with hooks; with `need_plain` or in training also when any other module of the stack is): the caller then runs the
+// modules or operators.
 PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 20);
@@ -645,7 +650,8 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   in.cu = tensor_arg(a[12]); in.dest = tensor_arg(a[13]); in.max_len = int_arg(a[14]); in.zero_tail = bool_arg(a[15]);
   in.enc = tensor_arg(a[16]); in.enc_cu = tensor_arg(a[17]); in.enc_dest = tensor_arg(a[18]); in.enc_max = int_arg(a[19]);
   if (!s.flash || (s.D != 16 && s.D != 32 && s.D != 64 && s.D != 128) || s.table.size(0) != s.nb || s.md > 2048) Py_RETURN_NONE;
-  if (bool_arg(a[9]) && !s.plain) Py_RETURN_NONE;
+  // (a feed-forward layer is always the caller's module: what it computes shows in its class and nowhere else)
+  if (!s.plain_ff || (bool_arg(a[9]) && !s.plain)) Py_RETURN_NONE;
   if (!in.x.is_cuda() || in.x.dim() != 3 || in.x.size(2) != s.d || !supported(s, in.x.scalar_type())) Py_RETURN_NONE;
   if (in.enc.defined() && (in.enc.scalar_type() != in.x.scalar_type() || in.enc.size(-1) != s.d)) Py_RETURN_NONE;
   if (in.x.numel() == 0 || (in.enc.defined() && in.enc.numel() == 0)) Py_RETURN_NONE;

@@ -218,7 +218,7 @@ class T5Stack(nn.Module):
         """One native pass over the rows x (B, S, d_model); modes as in csrc/host/stack.cpp.  None: not covered."""
         if not x.is_cuda or x.dtype not in _HALF or torch.is_autocast_enabled():
             return None
-        if need_plain and torch.nn.modules.module._has_any_global_hook():
+        if torch.nn.modules.module._has_any_global_hook():
             return None
         cfg = self.cfg
         return _host.stack_forward(self, _STACK_CLASSES, self._native_cache(), self.is_decoder, cfg.num_heads, cfg.d_kv,
@@ -368,7 +368,8 @@ class T5Stack(nn.Module):
                            attention_mask=None, packed_rows=None, return_packed=False, encoder_plan=None):
         """The fused pass operator by operator: sequence-parallel encoders (a collective per layer), passes with
         other operators than the library's, and calls that the native pass does not take (autocast, norm weights
-        or a bias table of another type than the matrices, weights that are not contiguous)."""
+        or a bias table of another type than the matrices, weights that are not contiguous, replaced or hooked
+        feed-forward layers)."""
         cfg = self.cfg
         x = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
         plan = tail = None
