@@ -184,3 +184,44 @@ def test_hooks_and_biases_of_a_feed_forward_layer_are_honoured():
     with torch.no_grad():
         want = model.encoder(ids)
     assert _rel(model.encoder.forward_fused(ids), want) < 2e-2 < _rel(want_plain, want)
+
+
+def _shift_weights(model, factor=0.5, data=False):
+    for stack in (model.encoder, model.decoder):
+        for blk in stack.block:
+            sa = blk.layer[0].SelfAttention
+            for p in (sa.q.weight, sa.v.weight, blk.layer[-1].DenseReluDense.wi_0.weight):
+                p.data.mul_(factor) if data else p.mul_(factor)
+
+
+def test_weights_made_under_inference_mode_are_never_stale():
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    with torch.inference_mode():
+        model = _model()
+        model(ids, dec)
+        _shift_weights(model)
+        got, states = model(ids, dec), model.encoder(ids)
+        tokens, last = model.greedy_decode(states, 7)
+        fresh = _model()
+        _shift_weights(fresh)
+        assert torch.equal(got, fresh(ids, dec)) and torch.equal(states, fresh.encoder(ids))
+        want_tokens, want_last = fresh.greedy_decode(states, 7)
+        assert torch.equal(tokens, want_tokens) and torch.equal(last, want_last)
+
+
+@torch.no_grad()
+def test_a_pass_of_the_module_interface_sees_updates_that_no_version_counter_shows():
+    """`p.data` updates (optimisers, moving averages, collectives) leave a parameter's version as it is; passes
+    that ran module by module saw them."""
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    model, fresh = _model(), _model()
+    states = model.encoder(ids)
+    model.decoder(dec, encoder_hidden_states=states)
+    model.greedy_decode(states, 7)
+    _shift_weights(model, data=True)
+    _shift_weights(fresh)
+    got, want = model.encoder(ids), fresh.encoder(ids)
+    assert torch.equal(got, want)
+    assert torch.equal(model.decoder(dec, encoder_hidden_states=got), fresh.decoder(dec, encoder_hidden_states=want))
+    for a, b in zip(model.greedy_decode(got, 7), fresh.greedy_decode(want, 7)):
+        assert torch.equal(a, b)

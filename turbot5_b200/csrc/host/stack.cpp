@@ -224,8 +224,10 @@ Stacked stack_weights(const Stack& s) {
   return r;
 }
 
-// Kept with the module: the stacked weights of the last inference pass, rebuilt when a parameter has been
-// modified in place or replaced.
+// Kept with the module for `forward_fused`: the stacked weights of its last pass, rebuilt when a parameter has been
+// modified in place or replaced.  Inference tensors have no version that would show a change: weights that hold
+// one are stacked anew by every pass, as they are wherever the modules used to read the weights themselves (the
+// module interface, a decoding session): those see changes through `p.data` too, which no version shows.
 struct StackCache {
   std::mutex mu;
   // (storage, first element, version) of every stacked parameter; a storage that has been freed never matches
@@ -234,12 +236,18 @@ struct StackCache {
   std::vector<Entry> key;
   std::shared_ptr<Stacked> weights;
 };
-std::shared_ptr<Stacked> cached_weights(StackCache& c, const Stack& s) {
+std::shared_ptr<Stacked> cached_weights(StackCache* cache, const Stack& s) {
+  auto fresh = [&]() { return std::make_shared<Stacked>(stack_weights(s)); };
+  if (!cache) return fresh();
+  StackCache& c = *cache;
   std::vector<const Tensor*> ts;
   for (const Layer& l : s.layers)
     for (const Tensor* t : {&l.q, &l.k, &l.v, &l.ck, &l.cv, &l.wi0, &l.wi1})
-      if (t->defined()) ts.push_back(t);
-  auto version = [](const Tensor& t) { return t.is_inference() ? 0u : (uint32_t)t._version(); };
+      if (t->defined()) {
+        if (t->is_inference()) return fresh();
+        ts.push_back(t);
+      }
+  auto version = [](const Tensor& t) { return (uint32_t)t._version(); };
   std::lock_guard<std::mutex> lock(c.mu);
   bool same = c.weights && c.key.size() == ts.size();
   for (size_t i = 0; same && i < ts.size(); ++i) {
@@ -248,7 +256,7 @@ std::shared_ptr<Stacked> cached_weights(StackCache& c, const Stack& s) {
            e.storage._unsafe_get_target() == ts[i]->storage().unsafeGetStorageImpl() && !e.storage.expired();
   }
   if (!same) {
-    c.weights = std::make_shared<Stacked>(stack_weights(s));
+    c.weights = fresh();
     c.key.clear();
     for (const Tensor* t : ts)
       c.key.push_back({c10::weak_intrusive_ptr<c10::StorageImpl>(t->storage().getWeakStorageImpl()), t->data_ptr(), version(*t)});
@@ -633,7 +641,7 @@ PyObject* py_new_stack_cache(PyObject*, PyObject* const*, Py_ssize_t) {
   END_HANDLE_TH_ERRORS
 }
 
-// stack_forward(stack, types, cache, decoder, heads, d_kv, buckets, max_distance, eps, need_plain,
+// stack_forward(stack, types, cache or None, decoder, heads, d_kv, buckets, max_distance, eps, need_plain,
 //               x, mode, cu, dest, max_len, zero_tail, enc, enc_cu, enc_dest, enc_max)
 // mode: 0 plain rows, 1 packed rows (cu), 2 padded rows with a mask (cu, dest).
 // Returns None when the pass is not one of the native ones (types, sizes, a feed-forward layer of another class or
@@ -664,14 +672,14 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (Tensor* t : plist) grad = grad || t->requires_grad();
   }
   if (!grad) {
-    auto* cache = (StackCache*)PyCapsule_GetPointer(a[2], "t5b_stack_cache");
-    if (!cache) throw python_error();
+    auto* cache = a[2] == Py_None ? nullptr : (StackCache*)PyCapsule_GetPointer(a[2], "t5b_stack_cache");
+    if (!cache && a[2] != Py_None) throw python_error();
     at::AutoGradMode no_grad(false);
     if (in.enc.defined()) in.enc = in.enc.contiguous();
     Tensor r;
     {
       pybind11::gil_scoped_release nogil;
-      r = infer(s, *cached_weights(*cache, s), in);
+      r = infer(s, *cached_weights(cache, s), in);
     }
     return wrap(r);
   }
@@ -709,7 +717,7 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // One generation: caches, weights and the argument block of t5b_decoder_step.
 struct DecodeSession {
   Stack s;
-  std::shared_ptr<Stacked> w;
+  Stacked w;
   Tensor head, embedding, hidden, logits, tokens, seqlens, enc_seqlens, workspace;
   std::vector<Tensor> self_kv, ckv;
   std::vector<t5b_decoder_layer> layers;
@@ -763,20 +771,20 @@ DecodeSession& session_arg(PyObject* o) {
 }
 void free_session(PyObject* o) { delete (DecodeSession*)PyCapsule_GetPointer(o, "t5b_decode_session"); }
 
-// new_decode_session(stack, types, cache, heads, d_kv, buckets, max_distance, eps,
+// new_decode_session(stack, types, heads, d_kv, buckets, max_distance, eps,
 //                    memory, enc_seqlens, max_len, lm_head weight, embedding weight, lm_scale, start_token)
 // None when the step kernels do not cover this decoder (types, sizes, replaced modules or hooks).
 PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 15);
+  expect(n, 14);
   auto ses = std::make_unique<DecodeSession>();
   DecodeSession& d = *ses;
-  d.s = collect(a[0], a[1], true, int_arg(a[3]), int_arg(a[4]), (int)int_arg(a[5]), (int)int_arg(a[6]), float_arg(a[7]));
-  const Tensor memory = tensor_arg(a[8]);
-  d.enc_seqlens = tensor_arg(a[9]);
-  const int64_t max_len = int_arg(a[10]);
-  d.head = tensor_arg(a[11]); d.embedding = tensor_arg(a[12]);
-  d.start_token = int_arg(a[14]);
+  d.s = collect(a[0], a[1], true, int_arg(a[2]), int_arg(a[3]), (int)int_arg(a[4]), (int)int_arg(a[5]), float_arg(a[6]));
+  const Tensor memory = tensor_arg(a[7]);
+  d.enc_seqlens = tensor_arg(a[8]);
+  const int64_t max_len = int_arg(a[9]);
+  d.head = tensor_arg(a[10]); d.embedding = tensor_arg(a[11]);
+  d.start_token = int_arg(a[13]);
   const Stack& s = d.s;
   if (!s.plain || !memory.is_cuda() || memory.dim() != 3 || memory.size(2) != s.d || memory.numel() == 0 || max_len <= 0) Py_RETURN_NONE;
   const at::ScalarType dt = memory.scalar_type();
@@ -797,7 +805,7 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   k.d_model = (int32_t)s.d; k.d_ff = (int32_t)s.F; k.gated = s.gated; k.vocab = (int32_t)d.head.size(0);
   k.max_len = (int32_t)max_len; k.enc_len = (int32_t)L;
   k.num_buckets = s.nb; k.max_distance = s.md;
-  k.eps = (float)s.eps; k.lm_scale = (float)float_arg(a[13]);
+  k.eps = (float)s.eps; k.lm_scale = (float)float_arg(a[12]);
   k.cross_stride_b = L * 2 * HD; k.cross_stride_n = 2 * HD; k.cross_stride_h = s.D;
   d.workspace = empty_like_dense({t5b_decoder_step_workspace_bytes(&k)}, at::kByte, dev);
   k.workspace = d.workspace.data_ptr(); k.workspace_bytes = d.workspace.numel();
@@ -808,11 +816,9 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int st = t5b_decoder_step_prepare(&k, stream_of(dev));
   if (st == T5B_ERR_UNSUPPORTED) Py_RETURN_NONE;
   check_status(st, "decoder step");
-  auto* cache = (StackCache*)PyCapsule_GetPointer(a[2], "t5b_stack_cache");
-  if (!cache) throw python_error();
   {
     pybind11::gil_scoped_release nogil;
-    d.w = cached_weights(*cache, s);
+    d.w = stack_weights(s);
     d.hidden = empty_like_dense({B, s.d}, dt, dev);
     d.logits = empty_like_dense({B, 1, d.head.size(0)}, dt, dev);
     d.tokens = empty_like_dense({B, max_len}, at::kLong, dev);
@@ -826,13 +832,13 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (size_t i = 0; i < s.layers.size(); ++i) {
       // cross keys and values of the layer, projected once: rows of k | v per memory token
       d.ckv.push_back(new_rows(mem, B * L, 2 * HD));
-      linear(mem, d.w->ckv_of(i), d.ckv.back());
+      linear(mem, d.w.ckv_of(i), d.ckv.back());
       d.self_kv.push_back(empty_like_dense({2, B, s.H, max_len, s.D}, dt, dev));
       const Layer& l = s.layers[i];
       t5b_decoder_layer& o = d.layers[i];
-      o.ln_self = l.ln_self.data_ptr(); o.wqkv = d.w->qkv_of(i).data_ptr(); o.wo = l.o.data_ptr();
+      o.ln_self = l.ln_self.data_ptr(); o.wqkv = d.w.qkv_of(i).data_ptr(); o.wo = l.o.data_ptr();
       o.ln_cross = l.ln_cross.data_ptr(); o.wcq = l.cq.data_ptr(); o.wco = l.co.data_ptr();
-      o.ln_ff = l.ln_ff.data_ptr(); o.wi = d.w->wi_of(i, s).data_ptr(); o.wff = l.wo.data_ptr();
+      o.ln_ff = l.ln_ff.data_ptr(); o.wi = d.w.wi_of(i, s).data_ptr(); o.wff = l.wo.data_ptr();
       o.self_kv = d.self_kv.back().data_ptr();
       o.cross_k = d.ckv.back().data_ptr();
       o.cross_v = (const char*)d.ckv.back().data_ptr() + HD * 2;

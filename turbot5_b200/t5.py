@@ -142,7 +142,7 @@ class DecoderCache:
 
 
 class _NativeState:
-    """What the native passes keep with a stack (stacked weights of the last inference pass).  Copies and
+    """What the native passes keep with a stack (stacked weights of the last `forward_fused`).  Copies and
     pickles of the module start without it."""
 
     def __init__(self):
@@ -221,10 +221,10 @@ class T5Stack(nn.Module):
         if torch.nn.modules.module._has_any_global_hook():
             return None
         cfg = self.cfg
-        return _host.stack_forward(self, _STACK_CLASSES, self._native_cache(), self.is_decoder, cfg.num_heads, cfg.d_kv,
-                                   cfg.relative_attention_num_buckets, cfg.relative_attention_max_distance,
-                                   cfg.layer_norm_epsilon, need_plain, x, mode, cu, dest, max_len, zero_tail, enc, enc_cu,
-                                   enc_dest, enc_max)
+        return _host.stack_forward(self, _STACK_CLASSES, None if need_plain else self._native_cache(), self.is_decoder,
+                                   cfg.num_heads, cfg.d_kv, cfg.relative_attention_num_buckets,
+                                   cfg.relative_attention_max_distance, cfg.layer_norm_epsilon, need_plain, x, mode, cu,
+                                   dest, max_len, zero_tail, enc, enc_cu, enc_dest, enc_max)
 
     # ---- inference pass of an encoder with the token-wise work fused around the attention path
     def _stacked_weights(self, i):
@@ -597,7 +597,7 @@ def _native_decoding(model, encoder_hidden_states, max_len, encoder_seqlens=None
             not encoder_hidden_states.is_cuda or encoder_hidden_states.dtype not in _HALF:
         return None
     scale = cfg.d_model ** -0.5 if cfg.tie_word_embeddings else 1.0
-    return _host.new_decode_session(dec, _STACK_CLASSES, dec._native_cache(), cfg.num_heads, cfg.d_kv,
+    return _host.new_decode_session(dec, _STACK_CLASSES, cfg.num_heads, cfg.d_kv,
                                     cfg.relative_attention_num_buckets, cfg.relative_attention_max_distance,
                                     cfg.layer_norm_epsilon, encoder_hidden_states, encoder_seqlens, max_len, head.weight,
                                     emb.weight, scale, cfg.decoder_start_token_id)
