@@ -225,3 +225,45 @@ def test_a_pass_of_the_module_interface_sees_updates_that_no_version_counter_sho
     assert torch.equal(model.decoder(dec, encoder_hidden_states=got), fresh.decoder(dec, encoder_hidden_states=want))
     for a, b in zip(model.greedy_decode(got, 7), fresh.greedy_decode(want, 7)):
         assert torch.equal(a, b)
+
+
+@torch.no_grad()
+def test_a_first_pass_inside_a_capture_leaves_nothing_behind_for_later_passes():
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    want = _model()(ids, dec)                  # library handles exist from here on
+    model = _model()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = model(ids, dec)
+    assert torch.equal(model(ids, dec), want)  # before any replay: nothing that the graph would write may be read
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    # updated weights: eager passes and replays both see them, and a replay reads no memory that was given back
+    _shift_weights(model)
+    fresh = _model()
+    _shift_weights(fresh)
+    want = fresh(ids, dec)
+    assert torch.equal(model(ids, dec), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+
+
+@torch.no_grad()
+def test_passes_on_several_streams_share_the_stacked_weights_in_order():
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    model = _model()
+    want = _model()(ids, dec)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    filler = torch.randn(8192, 8192, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        for _ in range(4):
+            filler @ filler                    # the stacked copies are built behind some milliseconds of work
+        first = model(ids, dec)
+    with torch.cuda.stream(b):
+        second = model(ids, dec)
+    torch.cuda.synchronize()
+    assert torch.equal(first, want) and torch.equal(second, want)

@@ -10,6 +10,9 @@
 #include "host.h"
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <cublas_v2.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -228,6 +231,9 @@ Stacked stack_weights(const Stack& s) {
 // modified in place or replaced.  Inference tensors have no version that would show a change: weights that hold
 // one are stacked anew by every pass, as they are wherever the modules used to read the weights themselves (the
 // module interface, a decoding session): those see changes through `p.data` too, which no version shows.
+// A pass on another stream waits for the copies and keeps their memory from being given out while it reads.  A
+// captured pass stacks inside its graph: eager passes must not read what only a replay would write, a replay
+// must not read what a later update has freed, and so a replay sees updated weights.
 struct StackCache {
   std::mutex mu;
   // (storage, first element, version) of every stacked parameter; a storage that has been freed never matches
@@ -235,10 +241,12 @@ struct StackCache {
   struct Entry { c10::weak_intrusive_ptr<c10::StorageImpl> storage; const void* data; uint32_t version; };
   std::vector<Entry> key;
   std::shared_ptr<Stacked> weights;
+  at::cuda::CUDAEvent ready;             // the copies are written
+  std::optional<c10::cuda::CUDAStream> stream;   // ... on this stream
 };
 std::shared_ptr<Stacked> cached_weights(StackCache* cache, const Stack& s) {
   auto fresh = [&]() { return std::make_shared<Stacked>(stack_weights(s)); };
-  if (!cache) return fresh();
+  if (!cache || at::cuda::currentStreamCaptureStatus() != at::cuda::CaptureStatus::None) return fresh();
   StackCache& c = *cache;
   std::vector<const Tensor*> ts;
   for (const Layer& l : s.layers)
@@ -255,11 +263,19 @@ std::shared_ptr<Stacked> cached_weights(StackCache* cache, const Stack& s) {
     same = e.data == ts[i]->data_ptr() && e.version == version(*ts[i]) &&
            e.storage._unsafe_get_target() == ts[i]->storage().unsafeGetStorageImpl() && !e.storage.expired();
   }
+  const auto stream = c10::cuda::getCurrentCUDAStream();
   if (!same) {
     c.weights = fresh();
+    c.ready = at::cuda::CUDAEvent();   // (of this device)
+    c.ready.record(stream);
+    c.stream = stream;
     c.key.clear();
     for (const Tensor* t : ts)
       c.key.push_back({c10::weak_intrusive_ptr<c10::StorageImpl>(t->storage().getWeakStorageImpl()), t->data_ptr(), version(*t)});
+  } else if (stream != *c.stream) {
+    c.ready.block(stream);
+    for (const Tensor* t : {&c.weights->qkv, &c.weights->ckv, &c.weights->wi})
+      if (t->defined()) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
   }
   return c.weights;
 }
