@@ -267,3 +267,72 @@ def test_passes_on_several_streams_share_the_stacked_weights_in_order():
         second = model(ids, dec)
     torch.cuda.synchronize()
     assert torch.equal(first, want) and torch.equal(second, want)
+
+
+def _into_flat_buffer(model, offset):
+    """Every parameter a view into one buffer, each starting `offset` elements past a 16-byte boundary."""
+    params = list(model.parameters())
+    room = [(p.numel() + 15) // 8 * 8 + 8 for p in params]
+    flat = torch.zeros(sum(room) + 8, device="cuda", dtype=params[0].dtype)
+    at = 0
+    for p, n in zip(params, room):
+        view = flat[at + offset:at + offset + p.numel()].view_as(p)
+        view.copy_(p.data)
+        p.data = view
+        at += n
+    return model
+
+
+@pytest.mark.parametrize("offset", [1, 4])
+def test_parameters_that_are_views_at_odd_offsets(offset):
+    """Sharding and data-parallel wrappers keep parameters in flat buffers; 16-byte loads and bulk copies must not
+    meet them there.  (The library takes other products for such weights: sums in another order, so no farther
+    from the float32 model than the aligned run, and half as much again for the chance of single roundings.)"""
+    ids, dec, mask = _ids(3, 70), _ids(3, 9, 1), _mask([70, 31, 2], 70)
+    aligned, model = _model(), _into_flat_buffer(_model(), offset)
+    exact = _model(torch.float32)
+    with torch.no_grad():
+        for p, e in zip(aligned.parameters(), exact.parameters()):
+            e.copy_(p)
+        exact = exact(ids, dec, attention_mask=mask)
+        assert _rel(model(ids, dec, attention_mask=mask), exact) <= 1.5 * _rel(aligned(ids, dec, attention_mask=mask), exact) < 0.2
+        states = aligned.encoder(ids)
+        for graph in (False, True):
+            tokens, last = model.greedy_decode(states, 8, use_cuda_graph=graph)
+            dec_in = torch.cat([torch.zeros((3, 1), dtype=torch.long, device="cuda"), tokens[:, :-1]], dim=1)
+            full = aligned.logits(aligned.decoder(dec_in, encoder_hidden_states=states))
+            assert _rel(last[:, -1], full[:, -1]) < 4e-2
+    embedded = aligned.shared(ids).detach()
+    room = torch.zeros(embedded.numel() + 8, device="cuda", dtype=embedded.dtype)
+    odd = room[offset:offset + embedded.numel()].view_as(embedded).copy_(embedded)
+    grads = []
+    for m, x in ((aligned, embedded), (model, odd)):
+        out = m.encoder(inputs_embeds=x.requires_grad_())
+        dout = torch.randn(out.shape, generator=torch.Generator().manual_seed(5)).to(out)
+        grads.append(torch.autograd.grad(out, [x] + list(m.encoder.block.parameters()), dout))
+    for a, b in zip(*grads):
+        assert _rel(b, a) < 4e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_norm_backward_with_a_residual_gradient_at_any_offset(offset, dtype):
+    from turbot5_b200 import _native as nat
+    rows, d, eps = 37, 768, 1e-6
+    g = torch.Generator().manual_seed(7)
+    x, dy, add = (torch.randn((rows, d), generator=g).to("cuda", dtype) for _ in range(3))
+    w = (1 + 0.1 * torch.randn(d, generator=g)).to("cuda", dtype)
+    room = torch.zeros(rows * d + 8, device="cuda", dtype=dtype)
+    odd = room[offset:offset + rows * d].view(rows, d).copy_(add)
+    dx, dw = torch.empty_like(x), torch.zeros(d, device="cuda")
+    code = nat.dtype_code(dtype)
+    st = nat.lib().t5b_rmsnorm_bwd_add(x.data_ptr(), w.data_ptr(), dy.data_ptr(), odd.data_ptr(), dx.data_ptr(), dw.data_ptr(),
+                                       rows, d, d, d, d, code, code, eps, nat.stream_ptr(x.device))
+    assert st == 0
+    xf, wf = x.double().requires_grad_(), w.double().requires_grad_()
+    (xf * torch.rsqrt(xf.square().mean(-1, keepdim=True) + eps) * wf).backward(dy.double())
+    want = xf.grad + add.double()
+    # one rounding of the result (2^-9 or 2^-12 relative), float32 sums before it
+    assert (dx.double() - want).abs().max().item() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * want.abs().max().item()
+    # the kernel rounds x * rstd as the forward pass does: that error is at most one half ulp a term
+    assert _rel(dw, wf.grad) < 2.0 ** -8

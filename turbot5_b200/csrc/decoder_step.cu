@@ -937,6 +937,21 @@ static int validate(const t5b_decoder_step_args* a) {
   return T5B_OK;
 }
 
+// Everything that is fetched with 16-byte loads or bulk copies.
+static int check_pointers(const t5b_decoder_step_args& a) {
+  uintptr_t bits = (uintptr_t)a.hidden | (uintptr_t)a.lm_head | (uintptr_t)a.embedding | (uintptr_t)a.final_ln;
+  for (int i = 0; i < a.n_layers; ++i) {
+    const t5b_decoder_layer& l = a.layers[i];
+    const void* all[] = {l.ln_self, l.wqkv, l.wo, l.ln_cross, l.wcq, l.wco, l.ln_ff, l.wi, l.wff, l.self_kv, l.cross_k, l.cross_v};
+    for (const void* p : all) {
+      if (!p) return T5B_ERR_ARG;
+      bits |= (uintptr_t)p;
+    }
+  }
+  if ((bits & 15) != 0 || ((a.cross_stride_b | a.cross_stride_h | a.cross_stride_n) % 8) != 0) return T5B_ERR_ALIGN;
+  return T5B_OK;
+}
+
 }  // namespace step
 }  // namespace t5b
 
@@ -965,6 +980,8 @@ extern "C" int t5b_decoder_step(const t5b_decoder_step_args* a, void* stream) {
   const int vst = step::validate(a);
   if (vst != T5B_OK) return vst;
   if (!a->hidden || !a->logits || !a->tokens || !a->seqlens || !a->lm_head || !a->embedding || !a->final_ln) return T5B_ERR_ARG;
+  const int pst = step::check_pointers(*a);
+  if (pst != T5B_OK) return pst;
   return a->dtype == T5B_BF16 ? step::run_step<__nv_bfloat16>(*a, (cudaStream_t)stream)
                               : step::run_step<__half>(*a, (cudaStream_t)stream);
 }

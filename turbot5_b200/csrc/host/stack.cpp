@@ -467,6 +467,7 @@ Tensor train_forward(StackNode& n) {
   const PassInputs& in = n.in;
   const int64_t B = in.x.size(0), S = in.x.size(1), R = B * S, HD = s.H * s.D;
   Tensor x = in.x.contiguous().view({R, s.d});
+  if ((uintptr_t)x.data_ptr() & 15) x = x.clone();           // a view of the caller's; the residual adds read vectors
   const Tensor mem = memory_rows(in);
   n.cu_dec = decoder_offsets(in, B, S);
   const Tensor branch = new_rows(x, R, s.d);
@@ -806,6 +807,12 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::ScalarType dt = memory.scalar_type();
   auto plain = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == dt && t.is_contiguous() && t.dim() == 2 && t.size(1) == s.d; };
   if (!supported(s, dt) || !plain(d.head) || !plain(d.embedding) || s.table.size(0) != s.nb) Py_RETURN_NONE;
+  // what the step kernels fetch with 16-byte loads and bulk copies (the stacked copies are allocations of their own)
+  auto aligned = [](const Tensor& t) { return !t.defined() || ((uintptr_t)t.data_ptr() & 15) == 0; };
+  if (!aligned(d.head) || !aligned(d.embedding) || !aligned(s.final_ln)) Py_RETURN_NONE;
+  for (const Layer& l : s.layers)
+    if (!aligned(l.ln_self) || !aligned(l.o) || !aligned(l.ln_cross) || !aligned(l.cq) || !aligned(l.co) || !aligned(l.ln_ff) ||
+        !aligned(l.wi0) || !aligned(l.wo)) Py_RETURN_NONE;
   if (d.start_token < 0 || d.start_token >= d.embedding.size(0) || d.head.size(0) > d.embedding.size(0)) Py_RETURN_NONE;
   const int64_t B = memory.size(0), L = memory.size(1), HD = s.H * s.D;
   if (d.enc_seqlens.defined()) {

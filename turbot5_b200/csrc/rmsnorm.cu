@@ -306,7 +306,7 @@ int launch_bwd(const void* x, const void* w, const void* dy, const void* dx_add,
                int64_t xs, int64_t dys, int64_t dxs, float eps, cudaStream_t st) {
   if constexpr (sizeof(TX) == 2 && std::is_same<TX, TDY>::value) {
     const bool aligned = ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0) && ((uintptr_t)dx % 16 == 0) &&
-                         xs % 8 == 0 && dys % 8 == 0 && dxs % 8 == 0;
+                         ((uintptr_t)dx_add % 16 == 0) && xs % 8 == 0 && dys % 8 == 0 && dxs % 8 == 0;
     if (aligned && (d == 512 || d == 768 || d == 1024)) {
       // four rows per warp before a second block joins an SM (every block costs one atomic per column)
       int64_t nblk = (rows + 31) / 32;
