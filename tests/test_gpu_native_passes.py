@@ -336,3 +336,63 @@ def test_norm_backward_with_a_residual_gradient_at_any_offset(offset, dtype):
     assert (dx.double() - want).abs().max().item() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * want.abs().max().item()
     # the kernel rounds x * rstd as the forward pass does: that error is at most one half ulp a term
     assert _rel(dw, wf.grad) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("width", [64, 512])
+def test_layers_of_different_widths(width, grad):
+    """One layer's feed-forward pruned or widened (plain modules of other sizes): run module by module."""
+    model = _model()
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    g = torch.Generator().manual_seed(3)
+    for stack in (model.encoder, model.decoder):
+        ff = stack.block[1].layer[-1].DenseReluDense
+        for name, shape in (("wi_0", (width, 128)), ("wi_1", (width, 128)), ("wo", (128, width))):
+            linear = nn.Linear(shape[1], shape[0], bias=False)
+            linear.weight.data = torch.randn(shape, generator=g) * shape[1] ** -0.5
+            setattr(ff, name, linear.cuda().bfloat16())
+    with torch.set_grad_enabled(grad):
+        states = model.encoder(ids)
+        hidden = model.decoder(dec, encoder_hidden_states=states)
+        with _by_modules(model.encoder), _by_modules(model.decoder):
+            want_states = model.encoder(ids)
+            want = model.decoder(dec, encoder_hidden_states=want_states)
+    assert torch.equal(states, want_states) and torch.equal(hidden, want)
+    with torch.no_grad():
+        fused = model.decoder.forward_fused(dec, encoder_hidden_states=model.encoder.forward_fused(ids))
+        assert _rel(fused, want) < 4e-2
+        tokens, last = model.greedy_decode(states.detach(), 5)
+        with _by_modules(model.decoder):
+            want_tokens, want_last = model.greedy_decode(states.detach(), 5)
+    assert torch.equal(tokens, want_tokens) and torch.equal(last, want_last)
+
+
+class _Held(torch.Tensor):
+    """A weight that lives in another tensor, as quantised and sharded weights do."""
+
+    @staticmethod
+    def __new__(cls, inner):
+        return torch.Tensor._make_wrapper_subclass(cls, inner.shape, dtype=inner.dtype, device=inner.device,
+                                                   strides=inner.stride())
+
+    def __init__(self, inner):
+        self.inner = inner
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        from torch.utils._pytree import tree_map_only
+        plain = tree_map_only(_Held, lambda t: t.inner, (args, kwargs or {}))
+        out = func(*plain[0], **plain[1])
+        return _Held(out) if func is torch.ops.aten.detach.default else out
+
+
+@torch.no_grad()
+def test_weights_that_are_tensor_subclasses():
+    model = _model()
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    want = model.decoder(dec, encoder_hidden_states=model.encoder(ids))
+    for stack in (model.encoder, model.decoder):
+        q = stack.block[0].layer[0].SelfAttention.q
+        q.weight = nn.Parameter(_Held(q.weight.detach()), requires_grad=False)
+    got = model.decoder(dec, encoder_hidden_states=model.encoder(ids))
+    assert _rel(got, want) < 4e-2

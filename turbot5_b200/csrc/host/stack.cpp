@@ -183,23 +183,33 @@ Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t
   TORCH_CHECK(fin, "the stack has no final_layer_norm");
   w.look(fin, K_NORM);
   s.final_ln = w.parameter(fin, "weight");
-  s.d = s.final_ln.size(0);
-  s.F = s.layers[0].wi0.size(0);
+  s.d = s.final_ln.dim() == 1 ? s.final_ln.size(0) : 0;
+  s.F = s.layers[0].wi0.dim() == 2 ? s.layers[0].wi0.size(0) : 0;
   s.plain = w.plain && wf.plain;
   s.plain_ff = wf.plain;
   s.flash = w.flash;
   return s;
 }
 
-// Whether the native passes take this stack: 16-bit weights of one type throughout, contiguous, d_model of
-// whole 16-byte vectors and at most 2048 (the norm kernels keep a row in registers).
-bool supported(const Stack& s, at::ScalarType dtype) {
-  if (!is_half_type(dtype) || s.d % 8 || s.d > 2048 || s.F % 8) return false;
-  auto ok = [&](const Tensor& t) { return !t.defined() || (t.is_cuda() && t.scalar_type() == dtype && t.is_contiguous()); };
-  for (const Layer& l : s.layers)
-    for (const Tensor* t : {&l.ln_self, &l.q, &l.k, &l.v, &l.o, &l.ln_cross, &l.cq, &l.ck, &l.cv, &l.co, &l.ln_ff, &l.wi0, &l.wi1, &l.wo})
-      if (!ok(*t)) return false;
-  return ok(s.final_ln) && ok(s.table);
+// Whether the native passes take this stack: 16-bit weights of one type throughout, on the rows' device, contiguous, of
+// the sizes that the products assume (a layer may have been replaced or pruned) and plain tensors (a subclass
+// keeps its data elsewhere); d_model of whole 16-byte vectors and at most 2048 (the norm kernels keep a row in
+// registers).
+bool plain_tensor(const Tensor& t) { return t.is_cuda() && !t.unsafeGetTensorImpl()->is_python_dispatch(); }
+bool supported(const Stack& s, const Tensor& x) {
+  const at::ScalarType dtype = x.scalar_type();
+  if (!is_half_type(dtype) || s.d <= 0 || s.d % 8 || s.d > 2048 || s.F <= 0 || s.F % 8) return false;
+  auto ok = [&](const Tensor& t, at::IntArrayRef sizes) {
+    return plain_tensor(t) && t.device() == x.device() && t.scalar_type() == dtype && t.sizes() == sizes && t.is_contiguous();
+  };
+  const int64_t HD = s.H * s.D;
+  const int64_t in[] = {HD, s.d}, out[] = {s.d, HD}, up[] = {s.F, s.d}, down[] = {s.d, s.F}, norm[] = {s.d}, table[] = {s.nb, s.H};
+  for (const Layer& l : s.layers) {
+    if (!ok(l.ln_self, norm) || !ok(l.q, in) || !ok(l.k, in) || !ok(l.v, in) || !ok(l.o, out)) return false;
+    if (s.decoder && (!ok(l.ln_cross, norm) || !ok(l.cq, in) || !ok(l.ck, in) || !ok(l.cv, in) || !ok(l.co, out))) return false;
+    if (!ok(l.ln_ff, norm) || !ok(l.wi0, up) || !ok(l.wo, down) || (s.gated && !ok(l.wi1, up))) return false;
+  }
+  return plain_tensor(x) && ok(s.final_ln, norm) && ok(s.table, table);
 }
 
 // Stacked weights: [q; k; v], the cross attention's [k; v] and [wi_0; wi_1] of every layer, so that each group
@@ -674,11 +684,12 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   in.packed = mode == 1; in.padded = mode == 2;
   in.cu = tensor_arg(a[12]); in.dest = tensor_arg(a[13]); in.max_len = int_arg(a[14]); in.zero_tail = bool_arg(a[15]);
   in.enc = tensor_arg(a[16]); in.enc_cu = tensor_arg(a[17]); in.enc_dest = tensor_arg(a[18]); in.enc_max = int_arg(a[19]);
-  if (!s.flash || (s.D != 16 && s.D != 32 && s.D != 64 && s.D != 128) || s.table.size(0) != s.nb || s.md > 2048) Py_RETURN_NONE;
+  if (!s.flash || (s.D != 16 && s.D != 32 && s.D != 64 && s.D != 128) || s.md > 2048) Py_RETURN_NONE;
   // (a feed-forward layer is always the caller's module: what it computes shows in its class and nowhere else)
   if (!s.plain_ff || (bool_arg(a[9]) && !s.plain)) Py_RETURN_NONE;
-  if (!in.x.is_cuda() || in.x.dim() != 3 || in.x.size(2) != s.d || !supported(s, in.x.scalar_type())) Py_RETURN_NONE;
-  if (in.enc.defined() && (in.enc.scalar_type() != in.x.scalar_type() || in.enc.size(-1) != s.d)) Py_RETURN_NONE;
+  if (!in.x.is_cuda() || in.x.dim() != 3 || in.x.size(2) != s.d || !supported(s, in.x)) Py_RETURN_NONE;
+  if (in.enc.defined() && (!plain_tensor(in.enc) || in.enc.device() != in.x.device() || in.enc.scalar_type() != in.x.scalar_type() ||
+                           in.enc.size(-1) != s.d)) Py_RETURN_NONE;
   if (in.x.numel() == 0 || (in.enc.defined() && in.enc.numel() == 0)) Py_RETURN_NONE;
   if (!matching(in, s.decoder)) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(in.x.device());
@@ -805,8 +816,10 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Stack& s = d.s;
   if (!s.plain || !memory.is_cuda() || memory.dim() != 3 || memory.size(2) != s.d || memory.numel() == 0 || max_len <= 0) Py_RETURN_NONE;
   const at::ScalarType dt = memory.scalar_type();
-  auto plain = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == dt && t.is_contiguous() && t.dim() == 2 && t.size(1) == s.d; };
-  if (!supported(s, dt) || !plain(d.head) || !plain(d.embedding) || s.table.size(0) != s.nb) Py_RETURN_NONE;
+  auto plain = [&](const Tensor& t) {
+    return plain_tensor(t) && t.device() == memory.device() && t.scalar_type() == dt && t.is_contiguous() && t.dim() == 2 && t.size(1) == s.d;
+  };
+  if (!supported(s, memory) || !plain(d.head) || !plain(d.embedding)) Py_RETURN_NONE;
   // what the step kernels fetch with 16-byte loads and bulk copies (the stacked copies are allocations of their own)
   auto aligned = [](const Tensor& t) { return !t.defined() || ((uintptr_t)t.data_ptr() & 15) == 0; };
   if (!aligned(d.head) || !aligned(d.embedding) || !aligned(s.final_ln)) Py_RETURN_NONE;
@@ -816,7 +829,8 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (d.start_token < 0 || d.start_token >= d.embedding.size(0) || d.head.size(0) > d.embedding.size(0)) Py_RETURN_NONE;
   const int64_t B = memory.size(0), L = memory.size(1), HD = s.H * s.D;
   if (d.enc_seqlens.defined()) {
-    if (!d.enc_seqlens.is_cuda() || d.enc_seqlens.scalar_type() != at::kInt || d.enc_seqlens.numel() != B) Py_RETURN_NONE;
+    if (!plain_tensor(d.enc_seqlens) || d.enc_seqlens.device() != memory.device() || d.enc_seqlens.scalar_type() != at::kInt ||
+        d.enc_seqlens.numel() != B) Py_RETURN_NONE;
     d.enc_seqlens = d.enc_seqlens.contiguous();
   }
   const at::Device dev = memory.device();
