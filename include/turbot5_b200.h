@@ -73,6 +73,8 @@ T5B_API int t5b_abi_version(void);
  * as before. */
 T5B_API int t5b_check_status(int32_t* device_status, int32_t* code_out, void* stream);
 T5B_API int t5b_selftest_bounded_wait(int32_t* device_status, int64_t limit_cycles, void* stream);
+/* The same for the waits of t5b_decoder_step. */
+T5B_API int t5b_selftest_decoder_wait(int32_t* device_status, int64_t limit_cycles, void* stream);
 
 /* ---- relative-position buckets ------------------------------------------------
  * Stands in for T5Attention._relative_position_bucket
@@ -290,6 +292,7 @@ typedef struct {
   int32_t n_layers, B, H, D, d_model, d_ff, gated, vocab, max_len, enc_len;
   int32_t num_buckets, max_distance;
   float eps, lm_scale;                  /* lm_scale multiplies the normed states before the head (tied embeddings) */
+  int32_t* device_status;               /* optional: as in t5b_attn_args (a wait that ran out; the step's results are void) */
 } t5b_decoder_step_args;
 
 T5B_API int64_t t5b_decoder_step_workspace_bytes(const t5b_decoder_step_args* args);

@@ -73,3 +73,29 @@ def test_cu_seqlens_past_the_tensors_touch_nothing_beyond_them():
     assert all(torch.isfinite(x).all() for x in grads)
     for b in bufs:
         assert (b[rows:] == 777.0).all()
+
+
+def test_a_wait_that_runs_out_in_a_decoder_step_is_reported():
+    """The end of the step kernels: the status word is set, the block's copies are waited for (with a limit: the
+    announced bytes never come), and the kernel returns; a generation afterwards is clean."""
+    import turbot5_b200 as t5b
+    from turbot5_b200 import _native as nat
+    from turbot5_b200.attention import device_status
+    L = nat.lib()
+    dev = torch.device("cuda", 0)
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    t5b.check_device_status(dev)
+    word = device_status(dev)
+    assert L.t5b_selftest_decoder_wait(word.data_ptr(), 200000, stream) == 0
+    code = ctypes.c_int32(0)
+    assert L.t5b_check_status(word.data_ptr(), ctypes.byref(code), stream) == nat.ERR_DEVICE_TIMEOUT
+    assert code.value == 4003
+    assert L.t5b_selftest_decoder_wait(word.data_ptr(), 0, stream) == 5
+    assert L.t5b_selftest_decoder_wait(None, 1000, stream) == 5
+    from tests.test_gpu_t5_stack import _model
+    model = _model(torch.bfloat16, d_model=128, num_heads=4, d_ff=256)
+    enc = seeded((3, 50, 128), 1, dtype=torch.bfloat16).cuda()
+    tokens, last = model.greedy_decode(enc, 7)
+    t5b.check_device_status(dev)
+    again, last2 = model.greedy_decode(enc, 7)
+    assert torch.equal(tokens, again) and torch.equal(last, last2)

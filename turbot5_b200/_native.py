@@ -29,7 +29,7 @@ SYMBOLS = ("t5b_status_string", "t5b_abi_version", "t5b_bucket_table_host", "t5b
            "t5b_decoder_step_workspace_bytes", "t5b_decoder_step_prepare", "t5b_decoder_step",
            "t5b_rmsnorm_fwd", "t5b_rmsnorm_bwd", "t5b_rmsnorm_bwd_add", "t5b_gated_gelu_bwd", "t5b_unpad_plan", "t5b_gather_rows",
            "t5b_scatter_rows", "t5b_attention_merge", "t5b_add_rmsnorm_fwd", "t5b_gated_gelu_fwd",
-           "t5b_check_status", "t5b_selftest_bounded_wait")
+           "t5b_check_status", "t5b_selftest_bounded_wait", "t5b_selftest_decoder_wait")
 
 
 class AttnArgs(C.Structure):
@@ -147,8 +147,9 @@ def lib():
                                  C.c_void_p, C.c_void_p]
     L.t5b_check_status.restype = C.c_int
     L.t5b_check_status.argtypes = [C.c_void_p, C.POINTER(C.c_int32), C.c_void_p]
-    L.t5b_selftest_bounded_wait.restype = C.c_int
-    L.t5b_selftest_bounded_wait.argtypes = [C.c_void_p, C.c_int64, C.c_void_p]
+    for f in (L.t5b_selftest_bounded_wait, L.t5b_selftest_decoder_wait):
+        f.restype = C.c_int
+        f.argtypes = [C.c_void_p, C.c_int64, C.c_void_p]
     L.t5b_attention_merge.restype = C.c_int
     L.t5b_attention_merge.argtypes = [C.POINTER(MergeArgs), C.c_void_p]
     L.t5b_add_rmsnorm_fwd.restype = C.c_int

@@ -117,6 +117,7 @@ struct GemmParams {
   int32_t B, N, K, F;              // F: E_GATED: rows of wi_0 (w holds wi_0 | wi_1)
   int32_t H, D, max_len;
   float eps, x_scale;              // x_scale: multiplies the normed rows (tied embeddings), 1 = off
+  int32_t* status;                 // device_status: a wait that gave up (see close_waits), or NULL
 };
 
 __device__ __forceinline__ float gelu_tanh(float a) {
@@ -129,6 +130,19 @@ __device__ __forceinline__ bool argmax_before(float a, int ia, float b, int ib) 
   if (na != nb) return na;
   if (!na && a != b) return a > b;
   return ia < ib;
+}
+
+// Last act of a kernel with bounded waits, by one thread, after a block barrier that follows every wait: a wait that gave
+// up has left wrong numbers, which the status word tells the host, and a copy may still be on its way into this
+// block's shared memory, which the block must not leave before.  `flags[0]` was raised by the wait; the two
+// barriers are the block's (phase 0).
+__device__ __noinline__ void close_waits(volatile int* flags, int32_t* status, int code, uint32_t bar_a, uint32_t bar_b,
+                                         long long limit) {
+  if (status != nullptr) atomicCAS(status, 0, code);
+  flags[1] = 0;
+  mbar_wait_bounded(bar_a, 0, flags + 1, limit);
+  flags[1] = 0;
+  mbar_wait_bounded(bar_b, 0, flags + 1, limit);
 }
 
 constexpr int WARPS = 8, THREADS = WARPS * 32;
@@ -219,7 +233,7 @@ step_gemm_kernel(const __grid_constant__ GemmParams p) {
   constexpr int OUT_COLS = kEpi == E_GATED ? COLS / 2 : COLS;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long bar_words[2];
-  __shared__ int abort_word;
+  __shared__ int abort_words[2];
   __shared__ float part[W];
   __shared__ float squares[kFold ? W : 1][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -235,7 +249,7 @@ step_gemm_kernel(const __grid_constant__ GemmParams p) {
 
   // the block's weights, before anything that depends on an earlier kernel
   if (tid == 0) {
-    abort_word = 0;
+    abort_words[0] = 0;
     mbar_init(w_bar, 1);
     mbar_init(ln_bar, 1);
     fence_barrier_init();
@@ -255,8 +269,7 @@ step_gemm_kernel(const __grid_constant__ GemmParams p) {
     if (ok) bulk_load(sW + r * pitch, (const char*)p.w + (int64_t)n * K * 2, (uint32_t)K * 2, w_bar);
   }
   __syncthreads();
-  volatile int* abort_flag = &abort_word;
-  // (a wait that gave up leaves wrong numbers, never a hang)
+  volatile int* abort_flag = abort_words;
   if (kFold) mbar_wait_bounded(ln_bar, 0, abort_flag);
   grid_wait();
 
@@ -374,6 +387,7 @@ step_gemm_kernel(const __grid_constant__ GemmParams p) {
     }
     if (m0 + 16 < p.B) __syncthreads();                       // `red` is written again
   }
+  if (tid == 0 && abort_flag[0] != 0) close_waits(abort_flag, p.status, 4001, w_bar, kNorm ? ln_bar : w_bar, T5B_WAIT_LIMIT_CYCLES);
 }
 
 // ---------------------------------------------------------------- LM head
@@ -388,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long bar_words[WARPS * LM_MAX_STAGES + 1];
-  __shared__ int abort_word;
+  __shared__ int abort_words[2];
   __shared__ float part[WARPS];
   __shared__ float best_v[WARPS][16 * M_TILES];
   __shared__ int best_i[WARPS][16 * M_TILES];
@@ -412,7 +426,7 @@ step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) 
   grid_launch_dependents();
   if (lane == 0) {
     for (int i = 0; i < stages; ++i) mbar_init(bar0 + 8 * i, 1);
-    if (tid == 0) { abort_word = 0; mbar_init(ln_bar, 1); }
+    if (tid == 0) { abort_words[0] = 0; mbar_init(ln_bar, 1); }
     fence_barrier_init();
     fence_proxy_async();
     if (tid == 0) {
@@ -423,7 +437,7 @@ step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) 
   __syncwarp();
   for (int i = 0; i < stages; ++i) load(i);
   __syncthreads();
-  volatile int* abort_flag = &abort_word;
+  volatile int* abort_flag = abort_words;
   grid_wait();
   #pragma unroll 1
   for (int m = 0; m < M_TILES; ++m) {
@@ -438,7 +452,8 @@ step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) 
     #pragma unroll
     for (int r = 0; r < 2; ++r) { bv[m][r] = -INFINITY; bi[m][r] = 0x7fffffff; }
   int it = 0;
-  for (int i = 0; i < n_mine; ++i) {
+  bool arrived = true;
+  for (int i = 0; i < n_mine && arrived; ++i) {
     const int tile = first + i * step;
     float acc[M_TILES][2][4];                                // two chains per sixteen rows
     #pragma unroll
@@ -448,7 +463,8 @@ step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) 
     for (int pc = 0; pc < pieces; ++pc, ++it) {
       const uint32_t w0 = sW + (it % stages) * stage_bytes + g * wpitch + t * 16;
       const uint32_t x0 = sX + g * pitch + pc * piece * 2 + t * 16;
-      mbar_wait_bounded(bar0 + 8 * (it % stages), (uint32_t)((it / stages) & 1), abort_flag);
+      arrived = mbar_wait_warp_fast(bar0 + 8 * (it % stages), (uint32_t)((it / stages) & 1), abort_flag);
+      if (!arrived) break;                                   // (the warp as one: its ring is drained below)
       #pragma unroll 4
       for (int kb = 0; kb < piece / 32; ++kb) {
         const uint4 w4 = lds128(w0 + kb * 64);
@@ -476,6 +492,12 @@ step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) 
         }
       }
   }
+  if (!arrived && lane == 0) {                               // the pieces that were requested and not used
+    abort_words[1] = 0;
+    for (int j = it; j < it + stages && j < n_mine * pieces; ++j)
+      mbar_wait_bounded(bar0 + 8 * (j % stages), (uint32_t)((j / stages) & 1), abort_words + 1);
+  }
+  __syncwarp();
   #pragma unroll
   for (int m = 0; m < M_TILES; ++m)
     #pragma unroll
@@ -496,6 +518,7 @@ step_logits_kernel(const __grid_constant__ GemmParams p, int piece, int stages) 
       if (argmax_before(best_v[w][tid], best_i[w][tid], v, n)) { v = best_v[w][tid]; n = best_i[w][tid]; }
     p.cand[(int64_t)tid * gridDim.x + blockIdx.x] = make_float2(v, __int_as_float(n));
   }
+  if (tid == 0 && abort_flag[0] != 0) close_waits(abort_flag, p.status, 4002, ln_bar, ln_bar, T5B_WAIT_LIMIT_CYCLES);
 }
 
 // ---------------------------------------------------------------- attention of one query row per (batch, head)
@@ -727,6 +750,26 @@ __global__ void step_prepare_kernel(float* bias, const void* table, int table_dt
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0;
 }
 
+// Self-test of close_waits: two barriers, a copy's worth of bytes announced on one and never sent.
+__global__ void wait_selftest_kernel(int32_t* status, long long limit) {
+  __shared__ __align__(8) unsigned long long bar_words[2];
+  __shared__ int abort_words[2];
+  const uint32_t bar = smem_u32(&bar_words[0]), done_bar = smem_u32(&bar_words[1]);
+  if (threadIdx.x == 0) {
+    abort_words[0] = 0;
+    mbar_init(bar, 1);
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+    mbar_expect_tx(bar, 64);
+    mbar_arrive(done_bar);
+  }
+  __syncthreads();
+  volatile int* flags = abort_words;
+  mbar_wait_bounded(bar, 0, flags, limit);
+  __syncthreads();
+  if (threadIdx.x == 0 && flags[0] != 0) close_waits(flags, status, 4003, done_bar, bar, limit);
+}
+
 // ------------------------------------------------------------------ host side
 struct Launcher {
   cudaStream_t stream;
@@ -881,7 +924,7 @@ static int run_step(const t5b_decoder_step_args& a, cudaStream_t stream) {
   for (int i = 0; i < a.n_layers; ++i) {
     const t5b_decoder_layer& w = a.layers[i];
     GemmParams g = {};
-    g.B = a.B; g.eps = a.eps; g.x_scale = 1.f; g.H = a.H; g.D = a.D; g.max_len = a.max_len; g.F = a.d_ff;
+    g.B = a.B; g.eps = a.eps; g.x_scale = 1.f; g.status = a.device_status; g.H = a.H; g.D = a.D; g.max_len = a.max_len; g.F = a.d_ff;
     auto project = [&](const void* x, int K, const void* weight, const void* ln, void* out, int N) {
       g.x = x; g.K = K; g.w = weight; g.ln = ln; g.out = out; g.N = N;
     };
@@ -914,7 +957,7 @@ static int run_step(const t5b_decoder_step_args& a, cudaStream_t stream) {
     residual_gemm<T>(go, g);
   }
   GemmParams g = {};
-  g.B = a.B; g.eps = a.eps; g.x_scale = a.lm_scale; g.x = a.hidden; g.K = a.d_model;
+  g.B = a.B; g.eps = a.eps; g.x_scale = a.lm_scale; g.status = a.device_status; g.x = a.hidden; g.K = a.d_model;
   g.w = a.lm_head; g.ln = a.final_ln; g.out = a.logits; g.N = a.vocab; g.cand = (float2*)(ws + l.cand);
   if (a.B <= 16) launch_logits<T, 1>(go, g);
   else if (a.B <= 32) launch_logits<T, 2>(go, g);
@@ -984,4 +1027,11 @@ extern "C" int t5b_decoder_step(const t5b_decoder_step_args* a, void* stream) {
   if (pst != T5B_OK) return pst;
   return a->dtype == T5B_BF16 ? step::run_step<__nv_bfloat16>(*a, (cudaStream_t)stream)
                               : step::run_step<__half>(*a, (cudaStream_t)stream);
+}
+
+extern "C" int t5b_selftest_decoder_wait(int32_t* device_status, int64_t limit_cycles, void* stream) {
+  if (!device_status) return T5B_ERR_ARG;
+  if (limit_cycles <= 0 || limit_cycles > 2000000000LL) return T5B_ERR_ARG;     // at most about a second
+  step::wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(device_status, (long long)limit_cycles);
+  return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
 }

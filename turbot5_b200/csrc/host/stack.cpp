@@ -838,6 +838,7 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   at::AutoGradMode no_grad(false);
   t5b_decoder_step_args& k = d.a;
   k.dtype = dtype_code(dt); k.table_dtype = dtype_code(s.table.scalar_type());
+  k.device_status = device_status(dev.index()).data_ptr<int32_t>();
   k.n_layers = (int32_t)s.layers.size(); k.B = (int32_t)B; k.H = (int32_t)s.H; k.D = (int32_t)s.D;
   k.d_model = (int32_t)s.d; k.d_ff = (int32_t)s.F; k.gated = s.gated; k.vocab = (int32_t)d.head.size(0);
   k.max_len = (int32_t)max_len; k.enc_len = (int32_t)L;
