@@ -295,6 +295,7 @@ typedef struct {
   int32_t* device_status;               /* optional: as in t5b_attn_args (a wait that ran out; the step's results are void) */
 } t5b_decoder_step_args;
 
+/* 0: no kernel takes these sizes. */
 T5B_API int64_t t5b_decoder_step_workspace_bytes(const t5b_decoder_step_args* args);
 T5B_API int t5b_decoder_step_prepare(const t5b_decoder_step_args* args, void* stream);
 T5B_API int t5b_decoder_step(const t5b_decoder_step_args* args, void* stream);

@@ -204,3 +204,40 @@ def test_hot_kernels_stay_within_their_register_and_spill_budget():
     assert k["registers"] <= 96 and k["spill_stores"] <= 16, k
     k = pick(bwd, "attn_bwd_dkv_wide_kernel", "ILb1ELb0E")
     assert k["registers"] <= 96 and k["spill_stores"] <= 64, k
+
+
+def test_decoder_step_takes_every_documented_size():
+    """One plan of tiles serves the size check and the launches, so a size that is accepted is one that runs: every
+    documented width at every kind of batch, and nothing beyond."""
+    import ctypes as C
+    from turbot5_b200 import _native as nat
+    P, I = C.c_void_p, C.c_int32
+
+    class Args(C.Structure):
+        _fields_ = [(n, P) for n in ("layers", "final_ln", "lm_head", "embedding", "table", "hidden", "logits", "tokens", "seqlens",
+                                     "enc_seqlens", "workspace")] + \
+                   [(n, C.c_int64) for n in ("workspace_bytes", "tokens_stride", "table_stride0", "cross_stride_b", "cross_stride_h",
+                                             "cross_stride_n")] + \
+                   [(n, I) for n in ("dtype", "table_dtype", "n_layers", "B", "H", "D", "d_model", "d_ff", "gated", "vocab", "max_len",
+                                     "enc_len", "num_buckets", "max_distance")] + \
+                   [("eps", C.c_float), ("lm_scale", C.c_float), ("device_status", P)]
+    size = nat.lib().t5b_decoder_step_workspace_bytes
+    size.restype, size.argtypes = C.c_int64, [P]
+
+    def taken(dtype=nat.BF16, B=16, H=12, D=64, d_model=768, d_ff=2048, gated=1, max_distance=128):
+        a = Args(dtype=dtype, table_dtype=dtype, n_layers=1, B=B, H=H, D=D, d_model=d_model, d_ff=d_ff, gated=gated, vocab=32128,
+                 max_len=64, enc_len=512, num_buckets=32, max_distance=max_distance)
+        return size(C.byref(a)) > 0
+    for dtype in (nat.BF16, nat.F16):
+        for B in (1, 2, 16, 17, 32, 33, 48, 64):
+            for d_model in range(32, 2049, 32):
+                assert taken(dtype, B, d_model=d_model), (dtype, B, d_model)
+                assert taken(dtype, B, H=64, d_model=d_model, d_ff=8192), (dtype, B, d_model)
+        for gated in (0, 1):
+            for d_ff in range(32, 8193, 32):
+                assert taken(dtype, d_model=2048, H=32, d_ff=d_ff, gated=gated), (dtype, d_ff, gated)
+        for H, D in ((1, 32), (2, 16), (64, 64), (32, 128), (33, 64), (256, 16)):
+            assert taken(dtype, H=H, D=D)
+    for bad in (dict(B=65), dict(B=0), dict(d_model=2080), dict(d_model=40), dict(d_ff=8224), dict(H=65), dict(D=48), dict(dtype=nat.F32),
+                dict(max_distance=2049)):
+        assert not taken(**bad), bad

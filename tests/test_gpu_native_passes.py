@@ -396,3 +396,31 @@ def test_weights_that_are_tensor_subclasses():
         q.weight = nn.Parameter(_Held(q.weight.detach()), requires_grad=False)
     got = model.decoder(dec, encoder_hidden_states=model.encoder(ids))
     assert _rel(got, want) < 4e-2
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("B,over,dtype", [
+    (2, dict(d_model=2048, num_heads=32, d_ff=5120), torch.float16),        # a normed product of several tiles
+    (64, dict(d_model=2048, num_heads=4), torch.bfloat16),                  # 64 rows beside a wide LM head
+    (33, dict(d_model=1664, num_heads=4), torch.float16),
+    (2, dict(d_ff=8192), torch.bfloat16), (3, dict(d_ff=6624, feed_forward_proj="relu"), torch.float16),
+    (1, dict(d_model=2016, num_heads=2), torch.bfloat16), (17, dict(d_model=1728, num_heads=2), torch.bfloat16),
+    (40, dict(d_model=1696, num_heads=2), torch.float16)])
+def test_wide_decoders_generate(B, over, dtype):
+    """Widths whose largest tiles do not fit in shared memory: smaller tiles serve them.  No row of the last logits
+    is farther from the float32 model over the same tokens than the worst row of the uncached 16-bit pass (half as
+    much again for the chance of single roundings), and a chosen token trails the best by no more than two such elements' errors."""
+    model = _model(dtype, num_layers=1, num_decoder_layers=1, **over)
+    exact = _model(torch.float32, num_layers=1, num_decoder_layers=1, **over)
+    for p, e in zip(model.parameters(), exact.parameters()):
+        e.copy_(p)
+    g = torch.Generator().manual_seed(31)
+    enc = torch.randn((B, 40, model.cfg.d_model), generator=g).to("cuda", dtype)
+    tokens, last = model.greedy_decode(enc, 7, use_cuda_graph=True)
+    dec_in = torch.cat([torch.zeros((B, 1), dtype=torch.long, device="cuda"), tokens[:, :-1]], dim=1)
+    full = model.logits(model.decoder(dec_in, encoder_hidden_states=enc)).float()
+    exact = exact.logits(exact.decoder(dec_in, encoder_hidden_states=enc.float()))
+    rows = lambda a, b: ((a.float() - b).norm(dim=-1) / b.norm(dim=-1)).max().item()
+    assert rows(last[:, -1], exact[:, -1]) <= 1.5 * rows(full, exact) < 0.2
+    chosen = exact.gather(-1, tokens[..., None])[..., 0]
+    assert (exact.max(-1).values - chosen).max().item() <= 4 * (full - exact).abs().max().item()

@@ -804,39 +804,75 @@ static bool allow_smem(F kern, std::atomic<bool>* done) {
 }
 constexpr size_t kMaxSmem = 223 * 1024, kLmSmem = 220 * 1024;       // dynamic; the kernels' own words take the rest
 
-template <typename T, int W, int NT, bool kNorm, int kEpi>
-static void launch_gemm(Launcher& go, const GemmParams& p) {
-  auto kern = step_gemm_kernel<T, W, NT, kNorm, kEpi>;
-  const size_t K = p.K, pitch = K * 2 + 64;
-  const size_t smem = NT * 8 * pitch + (kNorm ? K * 2 : 0) + (kNorm && !kIsBf16<T> ? 16 * pitch : 0) + (size_t)W * 16 * NT * 8 * 4;
-  static std::atomic<bool> attributes[64];
-  if (smem > kMaxSmem) { go.status = T5B_ERR_UNSUPPORTED; return; }
-  if (!allow_smem(kern, attributes)) { go.status = T5B_ERR_LAUNCH; return; }
-  const int cols = kEpi == E_GATED ? NT * 4 : NT * 8, n = kEpi == E_GATED ? p.F : p.N;
-  go(kern, dim3((unsigned)((n + cols - 1) / cols), 1, 1), W * 32, smem, p);
+// ---- tiles of every product, for `validate` and for the launches alike
+constexpr int GEMM_WARPS = 16;
+static size_t gemm_smem(int K, int nt, bool norm, bool bf16) {
+  const size_t pitch = (size_t)K * 2 + 64;
+  return nt * 8 * pitch + (norm ? (size_t)K * 2 : 0) + (norm && !bf16 ? 16 * pitch : 0) + (size_t)GEMM_WARPS * 16 * nt * 8 * 4;
 }
-
+// `want` tiles of eight rows of w per block, or fewer where their rows do not fit in shared memory; 0: none fits
+static int fitting_tiles(int want, int least, int K, bool norm, bool bf16) {
+  while (want > least && gemm_smem(K, want, norm, bf16) > kMaxSmem) want /= 2;
+  return gemm_smem(K, want, norm, bf16) <= kMaxSmem ? want : 0;
+}
 // Rows of w per block of the products that start with a norm: one tensor-core tile (8 rows) while that gives at
 // most two blocks per SM, so that all SMs pull weights and the successor's blocks still find room; two or
 // four tiles beyond.
-template <typename T, int kEpi>
-static void norm_gemm(Launcher& go, const GemmParams& p) {
-  const int tiles = ((kEpi == E_GATED ? 2 * p.F : p.N) + 7) / 8;
-  if constexpr (kEpi == E_GATED) {
-    if (tiles <= 592) launch_gemm<T, 16, 2, true, kEpi>(go, p);
-    else launch_gemm<T, 16, 4, true, kEpi>(go, p);
-  } else {
-    if (tiles <= 296) launch_gemm<T, 16, 1, true, kEpi>(go, p);
-    else if (tiles <= 592) launch_gemm<T, 16, 2, true, kEpi>(go, p);
-    else launch_gemm<T, 16, 4, true, kEpi>(go, p);
-  }
+static int norm_tiles(int K, int n_rows, bool gated, bool bf16) {
+  const int tiles = (n_rows + 7) / 8;
+  return gated ? fitting_tiles(tiles <= 592 ? 2 : 4, 2, K, true, bf16)
+               : fitting_tiles(tiles <= 296 ? 1 : tiles <= 592 ? 2 : 4, 1, K, true, bf16);
 }
 // Output projections: at K = 4096 a block of one tile reads 128 KB of activations for 64 KB of weights, so from there
-// on a block takes two (4.2 us against 5.2 us at 16 rows).
+// on a block takes two (4.2 us against 5.2 us at 16 rows) while they fit.
+static int residual_tiles(int K) { return fitting_tiles(K >= 4096 ? 2 : 1, 1, K, false, true); }
+
+// LM head: sixteen-row tiles of the normed rows that a block holds (further rows take a launch of their own), and the
+// ring beside them: pieces of K / 2, K / 4, ... columns until two fit, else of the largest divisor of K in whole 32s.
+struct LmPlan { int m_tiles = 0, piece = 0, stages = 0; };
+static LmPlan lm_plan(int K, int B) {
+  LmPlan best;
+  for (int m = B <= 16 ? 1 : B <= 32 ? 2 : 4; m >= 1; m /= 2) {
+    const size_t fixed = (size_t)K * 2 + (size_t)m * 16 * ((size_t)K * 2 + 64);
+    auto stages = [&](int piece) {
+      const size_t n = fixed < kLmSmem ? (kLmSmem - fixed) / ((size_t)WARPS * 8 * ((size_t)piece * 2 + 64)) : 0;
+      return n > LM_MAX_STAGES ? LM_MAX_STAGES : (int)n;
+    };
+    int piece = K;
+    while (stages(piece) < 2 && piece % 64 == 0) piece /= 2;
+    for (int p = K; stages(piece) < 2 && p >= 32; p -= 32)
+      if (K % p == 0 && stages(p) >= 2) piece = p;
+    if (stages(piece) > best.stages) { best.m_tiles = m; best.piece = piece; best.stages = stages(piece); }
+    if (best.stages >= 2) break;
+  }
+  return best;
+}
+
+template <typename T, int NT, bool kNorm, int kEpi>
+static void launch_gemm(Launcher& go, const GemmParams& p) {
+  auto kern = step_gemm_kernel<T, GEMM_WARPS, NT, kNorm, kEpi>;
+  static std::atomic<bool> attributes[64];
+  if (!allow_smem(kern, attributes)) { go.status = T5B_ERR_LAUNCH; return; }
+  const int cols = kEpi == E_GATED ? NT * 4 : NT * 8, n = kEpi == E_GATED ? p.F : p.N;
+  go(kern, dim3((unsigned)((n + cols - 1) / cols), 1, 1), GEMM_WARPS * 32, gemm_smem(p.K, NT, kNorm, kIsBf16<T>), p);
+}
+
+template <typename T, int kEpi>
+static void norm_gemm(Launcher& go, const GemmParams& p) {
+  switch (norm_tiles(p.K, kEpi == E_GATED ? 2 * p.F : p.N, kEpi == E_GATED, kIsBf16<T>)) {
+    case 1: if constexpr (kEpi != E_GATED) launch_gemm<T, 1, true, kEpi>(go, p); break;
+    case 2: launch_gemm<T, 2, true, kEpi>(go, p); break;
+    case 4: launch_gemm<T, 4, true, kEpi>(go, p); break;
+    default: go.status = T5B_ERR_UNSUPPORTED;
+  }
+}
 template <typename T>
 static void residual_gemm(Launcher& go, const GemmParams& p) {
-  if (p.K >= 4096) launch_gemm<T, 16, 2, false, E_RESIDUAL>(go, p);
-  else launch_gemm<T, 16, 1, false, E_RESIDUAL>(go, p);
+  switch (residual_tiles(p.K)) {
+    case 1: launch_gemm<T, 1, false, E_RESIDUAL>(go, p); break;
+    case 2: launch_gemm<T, 2, false, E_RESIDUAL>(go, p); break;
+    default: go.status = T5B_ERR_UNSUPPORTED;
+  }
 }
 
 static int lm_blocks(int vocab) {
@@ -851,23 +887,31 @@ static int lm_blocks(int vocab) {
   const int blocks = ((vocab + 7) / 8 + WARPS - 1) / WARPS;
   return blocks < n ? blocks : n;
 }
-// Pieces of half of K where that is whole 32s (a ring of two to four then fits beside the normed rows), else all of K.
 template <typename T, int M_TILES>
-static void launch_logits(Launcher& go, const GemmParams& p) {
+static void launch_logits(Launcher& go, const GemmParams& p, const LmPlan& plan) {
   auto kern = step_logits_kernel<T, M_TILES>;
-  const size_t fixed = (size_t)p.K * 2 + (size_t)M_TILES * 16 * ((size_t)p.K * 2 + 64);
-  int piece = p.K, stages = 0;
-  auto fits = [&]() {
-    const size_t stage = (size_t)WARPS * 8 * ((size_t)piece * 2 + 64);
-    const size_t n = fixed < kLmSmem ? (kLmSmem - fixed) / stage : 0;
-    stages = n > LM_MAX_STAGES ? LM_MAX_STAGES : (int)n;
-  };
-  fits();
-  while (stages < 2 && piece % 64 == 0) { piece /= 2; fits(); }
   static std::atomic<bool> attributes[64];
-  if (stages < 1) { go.status = T5B_ERR_UNSUPPORTED; return; }
   if (!allow_smem(kern, attributes)) { go.status = T5B_ERR_LAUNCH; return; }
-  go(kern, dim3((unsigned)lm_blocks(p.N), 1, 1), THREADS, fixed + (size_t)stages * WARPS * 8 * ((size_t)piece * 2 + 64), p, piece, stages);
+  const size_t fixed = (size_t)p.K * 2 + (size_t)M_TILES * 16 * ((size_t)p.K * 2 + 64);
+  const size_t ring = (size_t)plan.stages * WARPS * 8 * ((size_t)plan.piece * 2 + 64);
+  for (int row = 0; row < p.B; row += M_TILES * 16) {
+    GemmParams q = p;
+    q.B = p.B - row < M_TILES * 16 ? p.B - row : M_TILES * 16;
+    q.x = (const T*)p.x + (int64_t)row * p.K;
+    q.out = (T*)p.out + (int64_t)row * p.N;
+    q.cand = p.cand + (int64_t)row * lm_blocks(p.N);
+    go(kern, dim3((unsigned)lm_blocks(p.N), 1, 1), THREADS, fixed + ring, q, plan.piece, plan.stages);
+  }
+}
+template <typename T>
+static void logits(Launcher& go, const GemmParams& p) {
+  const LmPlan plan = lm_plan(p.K, p.B);
+  switch (plan.m_tiles) {
+    case 1: launch_logits<T, 1>(go, p, plan); break;
+    case 2: launch_logits<T, 2>(go, p, plan); break;
+    case 4: launch_logits<T, 4>(go, p, plan); break;
+    default: go.status = T5B_ERR_UNSUPPORTED;
+  }
 }
 
 template <typename T, bool kSelf>
@@ -959,23 +1003,33 @@ static int run_step(const t5b_decoder_step_args& a, cudaStream_t stream) {
   GemmParams g = {};
   g.B = a.B; g.eps = a.eps; g.x_scale = a.lm_scale; g.status = a.device_status; g.x = a.hidden; g.K = a.d_model;
   g.w = a.lm_head; g.ln = a.final_ln; g.out = a.logits; g.N = a.vocab; g.cand = (float2*)(ws + l.cand);
-  if (a.B <= 16) launch_logits<T, 1>(go, g);
-  else if (a.B <= 32) launch_logits<T, 2>(go, g);
-  else launch_logits<T, 4>(go, g);
+  logits<T>(go, g);
   go(step_choose_kernel<T>, dim3((unsigned)a.B, 1, 1), 256, 0, (const float2*)(ws + l.cand), l.n_cand, a.tokens, a.tokens_stride,
      a.seqlens, (const T*)a.embedding, (T*)a.hidden, a.d_model, a.max_len);
   return go.status;
 }
 
+// What the kernels take, the same answer for every entry point: sizes the launches would refuse show before anything runs.
+static int validate_sizes(const t5b_decoder_step_args& a) {
+  if (a.dtype != T5B_BF16 && a.dtype != T5B_F16) return T5B_ERR_DTYPE;
+  if (a.D != 16 && a.D != 32 && a.D != 64 && a.D != 128) return T5B_ERR_HEAD_DIM;
+  if (a.B <= 0 || a.H <= 0 || a.d_model <= 0 || a.d_ff <= 0 || a.vocab <= 0 || a.max_len <= 0 || a.enc_len <= 0) return T5B_ERR_SHAPE;
+  // 32-wide pieces of every contraction; a norm's row in registers; the weights of a block in shared memory
+  if (a.B > 64 || a.H > 4096 || a.d_model % 32 || (a.H * a.D) % 32 || a.d_ff % 32 || a.d_model > 2048 || a.H * a.D > 4096 ||
+      a.d_ff > 8192 || a.max_distance > 2048)
+    return T5B_ERR_UNSUPPORTED;
+  const bool bf16 = a.dtype == T5B_BF16, gated = a.gated != 0;
+  const int HD = a.H * a.D;
+  if (!norm_tiles(a.d_model, 3 * HD, false, bf16) || !norm_tiles(a.d_model, HD, false, bf16) ||
+      !norm_tiles(a.d_model, gated ? 2 * a.d_ff : a.d_ff, gated, bf16) || !residual_tiles(HD) || !residual_tiles(a.d_ff) ||
+      !lm_plan(a.d_model, a.B).m_tiles)
+    return T5B_ERR_UNSUPPORTED;
+  return T5B_OK;
+}
 static int validate(const t5b_decoder_step_args* a) {
   if (!a || !a->layers || a->n_layers <= 0) return T5B_ERR_ARG;
-  if (a->dtype != T5B_BF16 && a->dtype != T5B_F16) return T5B_ERR_DTYPE;
-  if (a->D != 16 && a->D != 32 && a->D != 64 && a->D != 128) return T5B_ERR_HEAD_DIM;
-  if (a->B <= 0 || a->H <= 0 || a->d_model <= 0 || a->d_ff <= 0 || a->vocab <= 0 || a->max_len <= 0 || a->enc_len <= 0) return T5B_ERR_SHAPE;
-  // 32-wide pieces of every contraction; a norm's row in registers; the weights of a block in shared memory
-  if (a->B > 64 || a->d_model % 32 || (a->H * a->D) % 32 || a->d_ff % 32 || a->d_model > 2048 || a->H * a->D > 4096 ||
-      a->d_ff > 8192 || a->max_distance > 2048)
-    return T5B_ERR_UNSUPPORTED;
+  const int st = validate_sizes(*a);
+  if (st != T5B_OK) return st;
   if (((uintptr_t)a->workspace & 255) != 0 || !a->workspace || a->workspace_bytes < layout(*a).total) return T5B_ERR_WORKSPACE;
   return T5B_OK;
 }
@@ -1001,7 +1055,7 @@ static int check_pointers(const t5b_decoder_step_args& a) {
 using namespace t5b;
 
 extern "C" int64_t t5b_decoder_step_workspace_bytes(const t5b_decoder_step_args* a) {
-  if (!a || a->B <= 0 || a->H <= 0 || a->D <= 0 || a->max_len <= 0 || a->enc_len <= 0 || a->vocab <= 0) return 0;
+  if (!a || step::validate_sizes(*a) != T5B_OK) return 0;
   return step::layout(*a).total;
 }
 
