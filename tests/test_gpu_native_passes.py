@@ -424,3 +424,95 @@ def test_wide_decoders_generate(B, over, dtype):
     assert rows(last[:, -1], exact[:, -1]) <= 1.5 * rows(full, exact) < 0.2
     chosen = exact.gather(-1, tokens[..., None])[..., 0]
     assert (exact.max(-1).values - chosen).max().item() <= 4 * (full - exact).abs().max().item()
+
+
+class _Adapter(nn.Module):
+    """Another feed-forward layer altogether: no child of the plain one's names."""
+
+    def __init__(self, d):
+        super().__init__()
+        self.scale = nn.Parameter(torch.full((d,), 0.25, device="cuda", dtype=torch.bfloat16))
+
+    def forward(self, x):
+        return x * self.scale
+
+
+class _NoWeight(nn.Module):
+    def __init__(self, linear):
+        super().__init__()
+        self.inner = linear
+
+    def forward(self, x):
+        return self.inner(x)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("what", ["feed-forward", "projection", "norm", "instance forward", "eps"])
+def test_replaced_modules_run_as_modules(what, grad):
+    """A module of another class, without the children or the weight that the plain one has, with a `forward`
+    of its own in the instance, or with another epsilon: run by calling it, as before."""
+    model = _model()
+    ids, dec = _ids(2, 70), _ids(2, 9, 1)
+    calls = []
+
+    class Norm(nn.Module):
+        def __init__(self, d):
+            super().__init__()
+            self.g = nn.Parameter(torch.ones(d, device="cuda", dtype=torch.bfloat16))
+
+        def forward(self, x):
+            calls.append(1)
+            return x * self.g
+
+    for stack in (model.encoder, model.decoder):
+        blk = stack.block[1]
+        if what == "feed-forward":
+            blk.layer[-1].DenseReluDense = _Adapter(128)
+        elif what == "projection":
+            blk.layer[0].SelfAttention.k = _NoWeight(blk.layer[0].SelfAttention.k)
+        elif what == "norm":
+            blk.layer[-1].layer_norm = Norm(128)
+        elif what == "eps":
+            blk.layer[-1].layer_norm.eps = 10.0
+        else:
+            blk.layer[-1].DenseReluDense.forward = lambda x: x * 0.25
+    with torch.set_grad_enabled(grad):
+        states = model.encoder(ids)
+        hidden = model.decoder(dec, encoder_hidden_states=states)
+        if what == "norm":
+            assert len(calls) == 2
+        with _by_modules(model.encoder), _by_modules(model.decoder):
+            want_states = model.encoder(ids)
+            want = model.decoder(dec, encoder_hidden_states=want_states)
+        assert torch.equal(states, want_states) and torch.equal(hidden, want)
+    with torch.no_grad():
+        # (the cached steps by operators read the projections' weights themselves: they never took such a module)
+        if what != "projection":
+            tokens, last = model.greedy_decode(states.detach(), 5)
+            with _by_modules(model.decoder):
+                want_tokens, want_last = model.greedy_decode(states.detach(), 5)
+            assert torch.equal(tokens, want_tokens) and torch.equal(last, want_last)
+
+
+def test_a_wrapped_encoder_is_called_in_training():
+    class Wrapped(nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner, self.calls = inner, 0
+
+        def forward(self, *a, **k):
+            self.calls += 1
+            return self.inner(*a, **k)
+
+        def __getattr__(self, name):
+            try:
+                return super().__getattr__(name)
+            except AttributeError:
+                return getattr(super().__getattr__("inner"), name)
+
+    model = _model()
+    ids, dec, mask = _ids(2, 70), _ids(2, 9, 1), _mask([70, 31], 70)
+    want = model(ids, dec, attention_mask=mask)
+    model.encoder = Wrapped(model.encoder)
+    got = model(ids, dec, attention_mask=mask)
+    assert model.encoder.calls == 1 and _rel(got, want) < 2e-2

@@ -74,65 +74,102 @@ struct Stack {
   bool plain = true;                     // every module is of the expected class and has no hooks
   bool flash = true;                     // every attention module is the full-attention one
   bool plain_ff = true;                  // `plain` of the feed-forward layers alone
+  bool complete = true;                  // every module and weight was found
 };
 
 struct Names {
-  PyObject *modules, *parameters, *hooks[4];
+  PyObject *modules, *parameters, *forward, *eps, *hooks[4], *attention[4];
   Names() {
-    modules = PyUnicode_InternFromString("_modules");
-    parameters = PyUnicode_InternFromString("_parameters");
-    hooks[0] = PyUnicode_InternFromString("_forward_hooks");
-    hooks[1] = PyUnicode_InternFromString("_forward_pre_hooks");
-    hooks[2] = PyUnicode_InternFromString("_backward_hooks");
-    hooks[3] = PyUnicode_InternFromString("_backward_pre_hooks");
+    auto intern = PyUnicode_InternFromString;
+    modules = intern("_modules"); parameters = intern("_parameters"); forward = intern("forward"); eps = intern("eps");
+    hooks[0] = intern("_forward_hooks"); hooks[1] = intern("_forward_pre_hooks");
+    hooks[2] = intern("_backward_hooks"); hooks[3] = intern("_backward_pre_hooks");
+    attention[0] = intern("n_heads"); attention[1] = intern("key_value_proj_dim");
+    attention[2] = intern("relative_attention_num_buckets"); attention[3] = intern("relative_attention_max_distance");
   }
 };
 const Names& names() { static const Names* n = new Names(); return *n; }
 
-// Walks the module tree.  `types`: the classes a plain stack is made of, in the order of enum Kind.
+// Walks the module tree.  `types`: the classes a plain stack is made of, in the order of enum Kind.  A module that is
+// not plain (another class, hooks, a `forward` in the instance, other settings than the stack's) is for the
+// caller to run; one that has not the children or weights looked for makes the walk incomplete.
 enum Kind { K_BLOCK = 0, K_LIST, K_SELF, K_CROSS, K_FF, K_ATTENTION, K_NORM, K_LINEAR, K_GATED, K_RELU, K_EMBEDDING };
 struct Walker {
   PyObject* types;
-  bool plain = true, flash = true;
+  const Stack* s;
+  bool plain = true, flash = true, complete = true;
 
-  PyObject* dict_of(PyObject* m, PyObject* name) {          // borrowed: the module keeps its dict alive
-    PyObject* d = PyObject_GetAttr(m, name);
-    if (!d) throw python_error();
+  static PyObject* instance(PyObject* m) {                  // borrowed: the module keeps its dict alive
+    PyObject* d = m ? PyObject_GetAttrString(m, "__dict__") : nullptr;
+    if (!d) { PyErr_Clear(); return nullptr; }
     Py_DECREF(d);
-    return d;
+    return PyDict_Check(d) ? d : nullptr;
+  }
+  static PyObject* table(PyObject* m, PyObject* name) {     // _modules or _parameters (borrowed), or null
+    PyObject* d = instance(m);
+    PyObject* t = d ? PyDict_GetItem(d, name) : nullptr;
+    return t && PyDict_Check(t) ? t : nullptr;
+  }
+  static PyObject* find(PyObject* m, const char* name) {
+    PyObject* t = table(m, names().modules);
+    PyObject* c = t ? PyDict_GetItemString(t, name) : nullptr;
+    return c && c != Py_None ? c : nullptr;
   }
   PyObject* child(PyObject* m, const char* name, int kind) {
-    PyObject* c = PyDict_GetItemString(dict_of(m, names().modules), name);
-    TORCH_CHECK(c, "the stack has no submodule ", name);
+    PyObject* c = find(m, name);
+    if (!c) { complete = plain = false; return nullptr; }
     look(c, kind);
     return c;
   }
+  bool has_int(PyObject* dict, PyObject* name, int64_t want) {
+    PyObject* v = PyDict_GetItem(dict, name);
+    if (!v || !PyLong_Check(v)) return false;
+    const long long got = PyLong_AsLongLong(v);
+    if (got == -1 && PyErr_Occurred()) PyErr_Clear();
+    return got == want;
+  }
   void look(PyObject* c, int kind) {
-    if (kind == K_ATTENTION && (PyObject*)Py_TYPE(c) != PyTuple_GET_ITEM(types, kind)) flash = false;
+    const bool exact = (PyObject*)Py_TYPE(c) == PyTuple_GET_ITEM(types, kind);
+    if (kind == K_ATTENTION && !exact) flash = false;
     if (!plain) return;
-    if ((PyObject*)Py_TYPE(c) != PyTuple_GET_ITEM(types, kind)) { plain = false; return; }
+    PyObject* d = exact ? instance(c) : nullptr;
+    if (!d || PyDict_GetItem(d, names().forward)) { plain = false; return; }
     for (PyObject* h : names().hooks) {
-      PyObject* d = PyObject_GetAttr(c, h);
-      if (!d) throw python_error();
-      if (PyObject_Size(d) != 0) plain = false;
-      Py_DECREF(d);
+      PyObject* t = PyDict_GetItem(d, h);
+      if (!t || PyObject_Size(t) != 0) { PyErr_Clear(); plain = false; return; }
+    }
+    if (kind == K_NORM) {
+      PyObject* e = PyDict_GetItem(d, names().eps);
+      const double v = e ? PyFloat_AsDouble(e) : -1.0;
+      if (v == -1.0 && PyErr_Occurred()) PyErr_Clear();
+      plain = v == s->eps;
+    } else if (kind == K_ATTENTION) {
+      const int64_t want[4] = {s->H, s->D, s->nb, s->md};
+      for (int i = 0; i < 4; ++i) plain = plain && has_int(d, names().attention[i], want[i]);
     }
   }
   Tensor parameter(PyObject* m, const char* name) {
-    PyObject* p = PyDict_GetItemString(dict_of(m, names().parameters), name);
+    if (!m) { complete = false; return Tensor(); }
+    PyObject* t = table(m, names().parameters);
+    PyObject* p = t ? PyDict_GetItemString(t, name) : nullptr;
     if (p && THPVariable_Check(p)) return THPVariable_Unpack(p);
     plain = false;                                          // a parametrised weight: ask the module for it
     PyObject* a = PyObject_GetAttrString(m, name);
-    if (!a) throw python_error();
-    TORCH_CHECK_TYPE(THPVariable_Check(a), "expected a tensor parameter");
-    Tensor t = THPVariable_Unpack(a);
+    if (!a || !THPVariable_Check(a)) {
+      PyErr_Clear();
+      Py_XDECREF(a);
+      complete = false;
+      return Tensor();
+    }
+    Tensor w = THPVariable_Unpack(a);
     Py_DECREF(a);
-    return t;
+    return w;
   }
   Tensor weight(PyObject* m, const char* name, int kind) {
     PyObject* c = child(m, name, kind);
     if (kind == K_LINEAR && plain) {                        // a bias is not part of these blocks
-      PyObject* b = PyDict_GetItemString(dict_of(c, names().parameters), "bias");
+      PyObject* t = table(c, names().parameters);
+      PyObject* b = t ? PyDict_GetItemString(t, "bias") : nullptr;
       if (b && b != Py_None) plain = false;
     }
     return parameter(c, "weight");
@@ -141,14 +178,13 @@ struct Walker {
 
 // dims: (heads, head dim, buckets, max distance, eps)
 Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t D, int nb, int md, double eps) {
-  Walker w{types}, wf{types};            // feed-forward layers are looked at apart
   Stack s;
+  Walker w{types, &s}, wf{types, &s};    // feed-forward layers are looked at apart
   s.decoder = decoder; s.H = H; s.D = D; s.nb = nb; s.md = md; s.eps = eps;
-  PyObject* blocks = PyDict_GetItemString(w.dict_of(stack, names().modules), "block");
-  TORCH_CHECK(blocks, "the stack has no blocks");
+  PyObject* blocks = Walker::table(Walker::find(stack, "block"), names().modules);
   PyObject *key, *blk;
   Py_ssize_t pos = 0;
-  while (PyDict_Next(w.dict_of(blocks, names().modules), &pos, &key, &blk)) {
+  while (blocks && w.complete && wf.complete && PyDict_Next(blocks, &pos, &key, &blk)) {
     w.look(blk, K_BLOCK);
     PyObject* list = w.child(blk, "layer", K_LIST);
     Layer l;
@@ -167,9 +203,9 @@ Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t
     }
     PyObject* ffl = w.child(list, decoder ? "2" : "1", K_FF);
     l.ln_ff = w.weight(ffl, "layer_norm", K_NORM);
-    PyObject* ff = PyDict_GetItemString(w.dict_of(ffl, names().modules), "DenseReluDense");
-    TORCH_CHECK(ff, "the feed-forward layer has no DenseReluDense");
-    const bool gated = PyDict_GetItemString(w.dict_of(ff, names().modules), "wi_0") != nullptr;
+    PyObject* ff = Walker::find(ffl, "DenseReluDense");
+    if (!ff) { s.complete = false; return s; }
+    const bool gated = Walker::find(ff, "wi_0") != nullptr;
     if (!s.layers.empty() && gated != s.gated) wf.plain = false;
     s.gated = gated;
     wf.look(ff, s.gated ? K_GATED : K_RELU);
@@ -178,11 +214,11 @@ Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t
     l.wo = wf.weight(ff, "wo", K_LINEAR);
     s.layers.push_back(std::move(l));
   }
-  TORCH_CHECK(!s.layers.empty(), "the stack has no blocks");
-  PyObject* fin = PyDict_GetItemString(w.dict_of(stack, names().modules), "final_layer_norm");
-  TORCH_CHECK(fin, "the stack has no final_layer_norm");
-  w.look(fin, K_NORM);
+  PyObject* fin = Walker::find(stack, "final_layer_norm");
+  if (fin) w.look(fin, K_NORM);
   s.final_ln = w.parameter(fin, "weight");
+  s.complete = w.complete && wf.complete && !s.layers.empty();
+  if (!s.complete) return s;
   s.d = s.final_ln.dim() == 1 ? s.final_ln.size(0) : 0;
   s.F = s.layers[0].wi0.dim() == 2 ? s.layers[0].wi0.size(0) : 0;
   s.plain = w.plain && wf.plain;
@@ -671,8 +707,8 @@ PyObject* py_new_stack_cache(PyObject*, PyObject* const*, Py_ssize_t) {
 // stack_forward(stack, types, cache or None, decoder, heads, d_kv, buckets, max_distance, eps, need_plain,
 //               x, mode, cu, dest, max_len, zero_tail, enc, enc_cu, enc_dest, enc_max)
 // mode: 0 plain rows, 1 packed rows (cu), 2 padded rows with a mask (cu, dest).
-// Returns None when the pass is not one of the native ones (types, sizes, a feed-forward layer of another class or
-// with hooks; with `need_plain` or in training also when any other module of the stack is): the caller then runs the
+// Returns None when the pass is not one of the native ones (types, sizes, missing modules, a feed-forward layer of
+// another class or with hooks; with `need_plain` or in training also when any other module of the stack is): the caller then runs the
 // modules or operators.
 PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -684,7 +720,7 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   in.packed = mode == 1; in.padded = mode == 2;
   in.cu = tensor_arg(a[12]); in.dest = tensor_arg(a[13]); in.max_len = int_arg(a[14]); in.zero_tail = bool_arg(a[15]);
   in.enc = tensor_arg(a[16]); in.enc_cu = tensor_arg(a[17]); in.enc_dest = tensor_arg(a[18]); in.enc_max = int_arg(a[19]);
-  if (!s.flash || (s.D != 16 && s.D != 32 && s.D != 64 && s.D != 128) || s.md > 2048) Py_RETURN_NONE;
+  if (!s.complete || !s.flash || (s.D != 16 && s.D != 32 && s.D != 64 && s.D != 128) || s.md > 2048) Py_RETURN_NONE;
   // (a feed-forward layer is always the caller's module: what it computes shows in its class and nowhere else)
   if (!s.plain_ff || (bool_arg(a[9]) && !s.plain)) Py_RETURN_NONE;
   if (!in.x.is_cuda() || in.x.dim() != 3 || in.x.size(2) != s.d || !supported(s, in.x)) Py_RETURN_NONE;
@@ -814,7 +850,7 @@ PyObject* py_new_decode_session(PyObject*, PyObject* const* a, Py_ssize_t n) {
   d.head = tensor_arg(a[10]); d.embedding = tensor_arg(a[11]);
   d.start_token = int_arg(a[13]);
   const Stack& s = d.s;
-  if (!s.plain || !memory.is_cuda() || memory.dim() != 3 || memory.size(2) != s.d || memory.numel() == 0 || max_len <= 0) Py_RETURN_NONE;
+  if (!s.complete || !s.plain || !memory.is_cuda() || memory.dim() != 3 || memory.size(2) != s.d || memory.numel() == 0 || max_len <= 0) Py_RETURN_NONE;
   const at::ScalarType dt = memory.scalar_type();
   auto plain = [&](const Tensor& t) {
     return plain_tensor(t) && t.device() == memory.device() && t.scalar_type() == dt && t.is_contiguous() && t.dim() == 2 && t.size(1) == s.d;

@@ -589,8 +589,8 @@ def _native_decoding(model, encoder_hidden_states, max_len, encoder_seqlens=None
     csrc/decoder_step.cu), or None when the step kernels do not cover it: float32, more than 64 rows, replaced
     modules or hooks, sizes they do not take."""
     dec, head, emb, cfg = model.decoder, model.lm_head, model.decoder.embed_tokens, model.cfg
-    plain = lambda m: not (m._forward_hooks or m._forward_pre_hooks)
-    if type(model).logits is not T5ForConditionalGeneration.logits or type(dec) is not T5Stack or \
+    plain = lambda m: not (m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__)
+    if type(model).logits is not T5ForConditionalGeneration.logits or "logits" in model.__dict__ or type(dec) is not T5Stack or \
             type(head) is not nn.Linear or type(emb) is not nn.Embedding or head.bias is not None or \
             emb.max_norm is not None or not (plain(head) and plain(emb) and plain(dec)) or \
             torch.nn.modules.module._has_any_global_hook() or torch.is_autocast_enabled() or \
@@ -750,7 +750,8 @@ class T5ForConditionalGeneration(nn.Module):
         enc, dec = self.encoder, self.decoder
         if not input_ids.is_cuda or self.shared.weight.dtype not in _HALF or self.cfg.attention_type != "flash" or \
                 attention_mask.shape != input_ids.shape or \
-                any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (enc, dec)):
+                any(type(m) is not T5Stack or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or
+                    m._backward_hooks or m._backward_pre_hooks for m in (enc, dec)):
             return None
         ids = input_ids[attention_mask != 0]             # the one read-back of the pass
         if ids.shape[0] == 0:
