@@ -516,3 +516,32 @@ def test_a_wrapped_encoder_is_called_in_training():
     model.encoder = Wrapped(model.encoder)
     got = model(ids, dec, attention_mask=mask)
     assert model.encoder.calls == 1 and _rel(got, want) < 2e-2
+
+
+def test_a_masked_training_step_can_be_captured():
+    """No pass reads a count back where that is forbidden: in a capture, and under the synchronisation check."""
+    model = _model().train()
+    ids, dec, mask = _ids(3, 70), _ids(3, 9, 1), _mask([70, 31, 2], 70)
+    params = list(model.parameters())
+
+    def step():
+        logits = model(ids, dec, attention_mask=mask)
+        return torch.autograd.grad(logits.float().square().mean(), params)
+    want = step()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        step()
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 4e-2

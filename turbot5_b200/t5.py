@@ -746,13 +746,16 @@ class T5ForConditionalGeneration(nn.Module):
     def _packed_training_pass(self, input_ids, decoder_input_ids, attention_mask):
         """Decoder states of a padded batch in training: the valid tokens are packed once (padded rows get no
         gradient and give none), both stacks run as native passes and the cross attention reads the packed
-        encoder states.  None when the stacks are not ones the native passes cover."""
+        encoder states.  None when the stacks are not ones the native passes cover, and where nothing may be read
+        back from the device (a capture, the synchronisation check): the padded passes read nothing back."""
         enc, dec = self.encoder, self.decoder
         if not input_ids.is_cuda or self.shared.weight.dtype not in _HALF or self.cfg.attention_type != "flash" or \
                 attention_mask.shape != input_ids.shape or \
                 any(type(m) is not T5Stack or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or
                     m._backward_hooks or m._backward_pre_hooks for m in (enc, dec)):
             return None
+        if torch.cuda.is_current_stream_capturing() or torch.cuda.get_sync_debug_mode():
+            return None                                  # packing reads the token count back: not here
         ids = input_ids[attention_mask != 0]             # the one read-back of the pass
         if ids.shape[0] == 0:
             return None
