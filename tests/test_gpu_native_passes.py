@@ -545,3 +545,40 @@ def test_a_masked_training_step_can_be_captured():
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert _rel(a, b) < 4e-2
+
+
+def test_saved_tensor_hooks_see_the_activations_of_a_stack():
+    """Offloading and checkpointing work by hooks on what autograd saves: under them a stack runs module by module,
+    so every activation goes through the hooks."""
+    model = _model().train()
+    ids, dec, mask = _ids(3, 70), _ids(3, 9, 1), _mask([70, 31, 2], 70)
+    params = list(model.parameters())
+    own = {p.untyped_storage().data_ptr() for p in params}
+
+    def grads():
+        logits = model(ids, dec, attention_mask=mask)
+        return torch.autograd.grad(logits.float().square().mean(), params)
+    want = grads()
+    packed = []
+
+    def pack(t):
+        if t.untyped_storage().data_ptr() not in own:
+            packed.append(tuple(t.shape))
+        return t
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        got = grads()
+    rows = [s for s in packed if len(s) >= 2 and s[-1] == 256]    # feed-forward rows: two products a layer at least
+    assert len(rows) >= 2 * 4, packed
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 4e-2
+    with torch.autograd.graph.save_on_cpu(pin_memory=True):
+        got = grads()
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 4e-2
+    from torch.utils.checkpoint import checkpoint
+    embedded = model.encoder.embed_tokens(ids).detach().requires_grad_()
+    out = model.encoder(inputs_embeds=embedded)
+    dout = torch.randn(out.shape, generator=torch.Generator().manual_seed(5)).to(out)
+    want = torch.autograd.grad(out, embedded, dout)[0]
+    out = checkpoint(lambda e: model.encoder(inputs_embeds=e), embedded, use_reentrant=False)
+    assert _rel(torch.autograd.grad(out, embedded, dout)[0], want) < 4e-2

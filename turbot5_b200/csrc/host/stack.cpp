@@ -9,6 +9,7 @@
 // per launch, more than most of the kernels of a batch of short sequences; here it costs 2-4 us.
 #include "host.h"
 
+#include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
@@ -748,6 +749,9 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return wrap(r);
   }
   if (!s.plain) Py_RETURN_NONE;
+  // Hooks on what is saved (offloading, checkpointing) have to see the activations: the modules save them one by
+  // one, where the node keeps them to itself.
+  if (at::SavedTensorDefaultHooks::get_hooks().has_value()) Py_RETURN_NONE;
   auto node = std::make_shared<StackNode>();
   Tensor y;
   {
