@@ -582,3 +582,21 @@ def test_saved_tensor_hooks_see_the_activations_of_a_stack():
     want = torch.autograd.grad(out, embedded, dout)[0]
     out = checkpoint(lambda e: model.encoder(inputs_embeds=e), embedded, use_reentrant=False)
     assert _rel(torch.autograd.grad(out, embedded, dout)[0], want) < 4e-2
+
+
+def test_forward_mode_inputs_that_ask_for_gradients_are_refused():
+    import torch.autograd.forward_ad as fw
+    import turbot5_b200 as t5b
+    model = _model()
+    q = torch.randn(1, 2, 64, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    w = torch.ones(128, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    x = torch.randn(2, 16, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    plan = t5b.get_unpad_plan(_mask([16, 3], 16))
+    with fw.dual_level():
+        dual = lambda t: fw.make_dual(t, torch.ones_like(t))
+        for call in (lambda: t5b.flash_attention_with_fusing_bias(dual(q), q, q, None),
+                     lambda: t5b.rms_layer_norm(dual(x), w),
+                     lambda: t5b.unpad_rows(dual(x), plan),
+                     lambda: model.encoder(inputs_embeds=dual(x))):
+            with pytest.raises((RuntimeError, NotImplementedError)):
+                call()

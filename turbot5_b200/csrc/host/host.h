@@ -47,6 +47,7 @@ inline Tensor empty_like_dense(at::IntArrayRef sizes, at::ScalarType dtype, at::
 inline Tensor empty_strided(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, at::Device dev) {
   return Tensor(at::detail::empty_strided_cuda(sizes, strides, dtype, dev));
 }
+inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline cudaStream_t stream_of(at::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
 inline Tensor unit_stride_last(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }

@@ -291,11 +291,17 @@ struct AttentionNode : public Node {
   std::string name() const override { return "T5FusedBiasAttentionBackward"; }
 };
 
+// Whether a call is recorded.  The nodes have no forward-mode derivative: a tangent would be dropped.
 bool wants_grad(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
+  bool grad = false, tangent = false;
   for (const Tensor* t : ts)
-    if (t->defined() && t->requires_grad()) return true;
-  return false;
+    if (t->defined()) {
+      grad = grad || t->requires_grad();
+      tangent = tangent || has_tangent(*t);
+    }
+  TORCH_CHECK_NOT_IMPLEMENTED(!grad || !tangent, "turbot5_b200 operators have no forward-mode derivative");
+  return grad;
 }
 
 // (out, lse) of a call, recorded for autograd when an input asks for it

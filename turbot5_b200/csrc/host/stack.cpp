@@ -752,6 +752,10 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   // Hooks on what is saved (offloading, checkpointing) have to see the activations: the modules save them one by
   // one, where the node keeps them to itself.
   if (at::SavedTensorDefaultHooks::get_hooks().has_value()) Py_RETURN_NONE;
+  // (the operators refuse forward-mode inputs)
+  if (has_tangent(in.x) || has_tangent(in.enc)) Py_RETURN_NONE;
+  for (Tensor* t : plist)
+    if (has_tangent(*t)) Py_RETURN_NONE;
   auto node = std::make_shared<StackNode>();
   Tensor y;
   {
