@@ -533,3 +533,27 @@ def test_a_hook_that_gives_back_another_tensor_is_refused():
             out = flash_attention_with_fusing_bias(q, q, q, None)
             with pytest.raises(RuntimeError, match="saved tensor"):
                 out.sum().backward()
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_gradients_beside_inference_tensors(packed):
+    """Keys and values that were computed under inference_mode (a frozen encoder): the other inputs' gradients as
+    beside ordinary tensors of the same values."""
+    t5b = _ops()
+    q, k, v = (seeded((1, 2, 100, 64), i, 0.5, torch.bfloat16).cuda() for i in (1, 2, 3))
+    table = seeded((32, 2), 4, 0.1, torch.bfloat16).cuda().requires_grad_()
+    q.requires_grad_()
+    cu = torch.tensor([0, 60, 100], dtype=torch.int32, device="cuda")
+    with torch.inference_mode():
+        ki, vi = k.clone(), v.clone()
+
+    def grads(k, v):
+        if packed:
+            rows = lambda t: t[0].transpose(0, 1)
+            out = t5b.flash_attention_with_fusing_bias_varlen(rows(q), rows(k), rows(v), table, cu, cu, 60, 60, sm_scale=1.0)
+        else:
+            out = t5b.flash_attention_with_fusing_bias(q, k, v, table, sm_scale=1.0)
+        return torch.autograd.grad(out, (q, table), torch.ones_like(out))
+    got, want = grads(ki, vi), grads(k, v)
+    assert torch.equal(got[0], want[0])
+    check_grad_close(got[1], want[1], "dtable")

@@ -231,10 +231,24 @@ void attention_backward(AttnCall& c, const Tensor& dout_in, const Tensor& dq, co
 
 namespace {
 
+// An input kept for the backward pass.  Inference tensors (frozen states computed once) cannot be saved variables; they
+// are kept as they are.
+struct KeptInput {
+  SavedVariable saved;
+  Tensor inference;
+  void keep(const Tensor& t) {
+    if (t.is_inference()) inference = t;
+    else saved = SavedVariable(t, false);
+  }
+  Tensor unpack() const { return inference.defined() ? inference : saved.unpack(); }
+  void reset() { saved.reset_data(); inference = Tensor(); }
+};
+
 // Backward of one attention call, as FlashAttentionBias (src/turbot5/ops/fused_bias_attention.py:822-873).
 struct AttentionNode : public Node {
   AttnCall call;                                  // argument block; its tensors are kept by the saved variables
-  SavedVariable q, k, v, table, out, lse;
+  KeptInput q, k, v, table;
+  SavedVariable out, lse;
   bool has_table = false;
 
   variable_list apply(variable_list&& grads) override {
@@ -285,7 +299,7 @@ struct AttentionNode : public Node {
   }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    q.reset_data(); k.reset_data(); v.reset_data(); table.reset_data(); out.reset_data(); lse.reset_data();
+    q.reset(); k.reset(); v.reset(); table.reset(); out.reset_data(); lse.reset_data();
     call.q = call.k = call.v = call.table = call.out = call.lse = Tensor();
   }
   std::string name() const override { return "T5FusedBiasAttentionBackward"; }
@@ -317,9 +331,9 @@ void run_attention(AttnCall& c, const Tensor& q, const Tensor& k, const Tensor& 
   auto node = std::make_shared<AttentionNode>();
   node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, bias));
   // inputs that were copied for the kernels are copied again in the backward pass: what is saved is the input
-  node->q = SavedVariable(q, false); node->k = SavedVariable(k, false); node->v = SavedVariable(v, false);
+  node->q.keep(q); node->k.keep(k); node->v.keep(v);
   node->has_table = bias.defined();
-  if (bias.defined()) node->table = SavedVariable(bias, false);
+  if (bias.defined()) node->table.keep(bias);
   torch::autograd::set_history(c.out, node);
   node->out = SavedVariable(c.out, true);
   node->lse = SavedVariable(c.lse, false);
