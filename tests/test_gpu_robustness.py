@@ -99,3 +99,31 @@ def test_a_wait_that_runs_out_in_a_decoder_step_is_reported():
     t5b.check_device_status(dev)
     again, last2 = model.greedy_decode(enc, 7)
     assert torch.equal(tokens, again) and torch.equal(last, last2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_float32_calls_with_short_and_long_tables_from_several_threads(D):
+    """Each call's shared memory grows with its table; one thread's short table must not lower the limit under
+    another's long one."""
+    import threading
+    import turbot5_b200 as t5b
+    q, table = seeded((1, 2, 70, D), 1, 0.3).cuda(), seeded((32, 2), 2, 0.1).cuda()
+    spans = (64, 2048, 200, 1500)
+    want = {md: t5b.flash_attention_with_fusing_bias(q, q, q, table, sm_scale=1.0, MAX_DISTANCE=md) for md in spans}
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(md):
+        try:
+            for _ in range(200):
+                out = t5b.flash_attention_with_fusing_bias(q, q, q, table, sm_scale=1.0, MAX_DISTANCE=md)
+            torch.cuda.synchronize()
+            assert torch.equal(out, want[md])
+        except Exception as e:                    # reported by the main thread
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(md,)) for md in spans]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors

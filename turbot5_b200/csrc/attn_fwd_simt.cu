@@ -13,6 +13,8 @@
 #include "t5b_common.cuh"
 #include "attn_params.cuh"
 
+#include <atomic>
+
 namespace t5b {
 namespace simt {
 
@@ -282,9 +284,18 @@ static int launch(const t5b_attn_args& a, AttnParams p, const BucketSpec& spec, 
   const bool vec = aligned(a.q, a.q_stride_b, a.q_stride_h, a.q_stride_m) && aligned(a.k, a.k_stride_b, a.k_stride_h, a.k_stride_n) &&
                    aligned(a.v, a.v_stride_b, a.v_stride_h, a.v_stride_n);
   auto kern = attn_fwd_simt_kernel<T, D, RPT>;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return T5B_ERR_LAUNCH;
+  // Room for the largest table, once per device and kernel: a limit set call by call would be lowered under another
+  // thread's launch with a longer table.
+  static std::atomic<bool> attr_set[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+    const size_t most = (smem_floats<D, RPT>() + 2 * 2048 + 1) * sizeof(float);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
+      cudaGetLastError();
+      return T5B_ERR_LAUNCH;
+    }
+    if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
   }
   kern<<<grid, THREADS, smem, stream>>>(p, spec, vec);
   return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
