@@ -241,3 +241,13 @@ def test_decoder_step_takes_every_documented_size():
     for bad in (dict(B=65), dict(B=0), dict(d_model=2080), dict(d_model=40), dict(d_ff=8224), dict(H=65), dict(D=48), dict(dtype=nat.F32),
                 dict(max_distance=2049)):
         assert not taken(**bad), bad
+
+
+def test_whole_numbers_beyond_64_bits_raise_at_the_binding():
+    import turbot5_b200 as t5b
+    q = torch.zeros(1, 1, 4, 16)
+    for kw in (dict(NUM_BUCKETS=1 << 70), dict(MAX_DISTANCE=-(1 << 70)), dict(q_pos_offset=1 << 64)):
+        with pytest.raises(OverflowError):
+            t5b.flash_attention_with_fusing_bias(q, q, q, None, **kw)
+    with pytest.raises(RuntimeError):
+        t5b.flash_attention_with_fusing_bias(q, q, q, None, q_pos_offset=-1)     # (there is no CPU path)

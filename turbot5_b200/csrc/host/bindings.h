@@ -14,11 +14,11 @@ inline Tensor tensor_arg(PyObject* o) {
   return THPVariable_Unpack(o);
 }
 inline int64_t int_arg(PyObject* o) {
-  if (PyLong_Check(o)) return (int64_t)PyLong_AsLongLong(o);
-  PyObject* n = PyNumber_Long(o);
+  PyObject* n = PyLong_Check(o) ? (Py_INCREF(o), o) : PyNumber_Long(o);
   if (!n) throw python_error();
   const int64_t v = (int64_t)PyLong_AsLongLong(n);
   Py_DECREF(n);
+  if (v == -1 && PyErr_Occurred()) throw python_error();       // does not fit in 64 bits
   return v;
 }
 inline double float_arg(PyObject* o) {
