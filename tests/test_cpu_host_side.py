@@ -251,3 +251,17 @@ def test_whole_numbers_beyond_64_bits_raise_at_the_binding():
             t5b.flash_attention_with_fusing_bias(q, q, q, None, **kw)
     with pytest.raises(RuntimeError):
         t5b.flash_attention_with_fusing_bias(q, q, q, None, q_pos_offset=-1)     # (there is no CPU path)
+
+
+def test_norm_backward_keeps_two_blocks_per_sm():
+    """256 threads and two blocks per SM need 128 registers at most: at d = 768 the residual's vectors would cost the
+    second block, so the call without a residual has a kernel of its own (template arguments: type, weight type,
+    columns / 256, residual)."""
+    from turbot5_b200 import build
+    report = build.resource_report("rmsnorm.cu")
+    for t in ("13__nv_bfloat16", "6__half"):
+        for variant in ("Li2ELb0E", "Li2ELb1E", "Li3ELb0E"):
+            names = [n for n in report if "rmsnorm_bwd_vec_kernelI" + t in n and variant in n]
+            assert len(names) == 1, (t, variant)
+            k = report[names[0]]
+            assert k["registers"] <= 128 and k["spill_stores"] == 0, (names[0], k)

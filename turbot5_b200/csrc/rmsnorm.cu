@@ -230,8 +230,12 @@ rmsnorm_bwd_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const TDY
 // sums in shared memory side by side and one addition per column and block goes to the result
 // (adding into one shared row with atomics retries eight-fold: 8.3 us against 4.4 us on average over the
 // norms of a training step of 512-wide rows, 512 to 4096 of them).
-template <typename TX, typename TW, int NT>
-__global__ void __launch_bounds__(256)
+// kAdd apart: the residual's vectors, held from the loads to the output, cost the second block per SM at d = 768 (137
+// registers; 128 is the limit for two).  100 000 x 768 without them 84 us in a kernel of its own, 122 us in one
+// kernel for both; with them 131 us held from the start, 138 us loaded after the reductions in 128 registers (and
+// 12.1 against 8.3 us at 4096 x 512).
+template <typename TX, typename TW, int NT, bool kAdd>
+__global__ void __launch_bounds__(256, NT == 2 || (NT == 3 && !kAdd) ? 2 : 1)
 rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const TX* __restrict__ dy,
                        const TX* dx_add, TX* dx, float* __restrict__ dw, int64_t rows,
                        int64_t x_stride, int64_t dy_stride, int64_t dx_stride, float eps) {
@@ -254,7 +258,7 @@ rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const
       const uint4 xa = ld_stream16(x + r * x_stride + t * 256 + lane * 8);
       const uint4 ga = ld_stream16(dy + r * dy_stride + t * 256 + lane * 8);
       add[t] = make_uint4(0, 0, 0, 0);
-      if (dx_add) add[t] = *reinterpret_cast<const uint4*>(dx_add + r * dx_stride + t * 256 + lane * 8);
+      if (kAdd) add[t] = *reinterpret_cast<const uint4*>(dx_add + r * dx_stride + t * 256 + lane * 8);
       const TX* xe = reinterpret_cast<const TX*>(&xa);
       const TX* ge = reinterpret_cast<const TX*>(&ga);
       #pragma unroll
@@ -279,7 +283,8 @@ rmsnorm_bwd_vec_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const
       const TX* ae = reinterpret_cast<const TX*>(&add[t]);
       #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        oe[k] = from_float<TX>(rstd * wv[t][k] * gv[t][k] - xv[t][k] * kk + to_float(ae[k]));
+        const float through = rstd * wv[t][k] * gv[t][k] - xv[t][k] * kk;
+        oe[k] = from_float<TX>(kAdd ? through + to_float(ae[k]) : through);
         const float xhat = to_float(from_float<TW>(xv[t][k] * rstd));
         acc[t][k] = fmaf(gv[t][k], xhat, acc[t][k]);
       }
@@ -312,9 +317,15 @@ int launch_bwd(const void* x, const void* w, const void* dy, const void* dx_add,
       int64_t nblk = (rows + 31) / 32;
       if (nblk < 148) nblk = (rows + 7) / 8 < 148 ? (rows + 7) / 8 : 148;
       if (nblk > 148 * 4) nblk = 148 * 4;
-#define T5B_RMSB_VEC(NT)                                                                            \
-      rmsnorm_bwd_vec_kernel<TX, TW, NT><<<(unsigned)nblk, 256, 0, st>>>(                               \
-          (const TX*)x, (const TW*)w, (const TX*)dy, (const TX*)dx_add, (TX*)dx, dw, rows, xs, dys, dxs, eps)
+      auto go = [&](auto kern) {
+        kern<<<(unsigned)nblk, 256, 0, st>>>((const TX*)x, (const TW*)w, (const TX*)dy, (const TX*)dx_add, (TX*)dx, dw, rows, xs, dys,
+                                             dxs, eps);
+      };
+#define T5B_RMSB_VEC(NT)                                           \
+      do {                                                         \
+        if (dx_add) go(rmsnorm_bwd_vec_kernel<TX, TW, NT, true>);  \
+        else go(rmsnorm_bwd_vec_kernel<TX, TW, NT, false>);        \
+      } while (0)
       if (d == 512) T5B_RMSB_VEC(2); else if (d == 768) T5B_RMSB_VEC(3); else T5B_RMSB_VEC(4);
 #undef T5B_RMSB_VEC
       return cudaGetLastError() == cudaSuccess ? T5B_OK : T5B_ERR_LAUNCH;
