@@ -601,3 +601,57 @@ def test_forward_mode_inputs_that_ask_for_gradients_are_refused():
                      lambda: model.encoder(inputs_embeds=dual(x))):
             with pytest.raises((RuntimeError, NotImplementedError)):
                 call()
+
+
+def _same_until_a_near_tie(model, states, got, want, lens=None):
+    """Two greedy runs of the same model: equal tokens, or the first difference of a row is at a step where the two
+    tokens' logits in an uncached pass over the common prefix are within what 16-bit passes differ by."""
+    tokens, other = got, want
+    for b in range(tokens.shape[0]):
+        diff = (tokens[b] != other[b]).nonzero()
+        if diff.numel() == 0:
+            continue
+        t = int(diff[0])
+        dec_in = torch.cat([torch.zeros((1, 1), dtype=torch.long, device="cuda"), tokens[b:b + 1, :t]], dim=1)
+        logits = model.logits(model.decoder(dec_in, encoder_hidden_states=states[b:b + 1]))[0, -1].float()
+        gap = (logits[tokens[b, t]] - logits[other[b, t]]).abs().item()
+        assert gap <= 0.1 * logits.abs().mean().item(), (b, t, gap)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("ff", ["gated-gelu", "relu"])
+@pytest.mark.parametrize("B,steps,why", [(3, 7, "hook"), (65, 7, "rows"), (1, 530, "hook")])
+def test_the_decoding_paths_without_the_step_kernels(B, steps, why, ff):
+    """What serves models and batches that the step kernels do not take: the eager cached steps and the captured
+    static step, against each other and against the step kernels where those run (530 cached keys: the captured
+    self attention splits them)."""
+    from turbot5_b200 import _native as nat
+    from turbot5_b200.t5 import _native_decoding
+    model = _model(feed_forward_proj=ff)
+    states = model.encoder(_ids(B, 120, 6))
+    native = None
+    if why == "hook":
+        native, _ = model.greedy_decode(states, steps)
+        handle = model.decoder.block[0].layer[0].SelfAttention.q.register_forward_hook(lambda *a: None)
+    assert _native_decoding(model, states, steps) is None
+    eager, eager_last = model.greedy_decode(states, steps)
+    graphed, graphed_last = model.greedy_decode(states, steps, use_cuda_graph=True)
+    if steps > 500:
+        assert nat.lib().t5b_decode_num_splits(B, 4, steps) > 1
+    if why == "hook":
+        handle.remove()
+        _same_until_a_near_tie(model, states, native, eager)
+    _same_until_a_near_tie(model, states, graphed, eager)
+    same = (eager == graphed).all(1)
+    assert same.float().mean() >= 0.5 or steps > 500
+    if same.any():
+        assert _rel(graphed_last[same], eager_last[same]) < 6e-2
+
+
+@torch.no_grad()
+def test_float32_decoding_through_a_graph():
+    model = _model(torch.float32)
+    states = model.encoder(_ids(2, 60))
+    eager, eager_last = model.greedy_decode(states, 9)
+    graphed, graphed_last = model.greedy_decode(states, 9, use_cuda_graph=True)
+    assert torch.equal(eager, graphed) and _rel(graphed_last, eager_last) < 1e-4
