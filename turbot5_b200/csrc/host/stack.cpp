@@ -95,31 +95,38 @@ const Names& names() { static const Names* n = new Names(); return *n; }
 // not plain (another class, hooks, a `forward` in the instance, other settings than the stack's) is for the
 // caller to run; one that has not the children or weights looked for makes the walk incomplete.
 enum Kind { K_BLOCK = 0, K_LIST, K_SELF, K_CROSS, K_FF, K_ATTENTION, K_NORM, K_LINEAR, K_GATED, K_RELU, K_EMBEDDING };
+#define T5B_KEY(name) ([] { static PyObject* const k = PyUnicode_InternFromString(name); return k; }())
+
+// A module's own dicts, looked up once (borrowed: the module keeps them alive); null where there is none.
+struct Module {
+  PyObject *self = nullptr, *dict = nullptr, *modules = nullptr, *parameters = nullptr;
+  Module() = default;
+  explicit Module(PyObject* m) : self(m) {
+    PyObject* d = m ? PyObject_GenericGetDict(m, nullptr) : nullptr;
+    if (!d) { PyErr_Clear(); return; }
+    Py_DECREF(d);
+    if (!PyDict_Check(d)) return;
+    dict = d;
+    modules = PyDict_GetItem(d, names().modules);
+    parameters = PyDict_GetItem(d, names().parameters);
+    if (modules && !PyDict_Check(modules)) modules = nullptr;
+    if (parameters && !PyDict_Check(parameters)) parameters = nullptr;
+  }
+  Module find(PyObject* key) const {
+    PyObject* c = modules ? PyDict_GetItem(modules, key) : nullptr;
+    return c && c != Py_None ? Module(c) : Module();
+  }
+};
+
 struct Walker {
   PyObject* types;
   const Stack* s;
   bool plain = true, flash = true, complete = true;
 
-  static PyObject* instance(PyObject* m) {                  // borrowed: the module keeps its dict alive
-    PyObject* d = m ? PyObject_GetAttrString(m, "__dict__") : nullptr;
-    if (!d) { PyErr_Clear(); return nullptr; }
-    Py_DECREF(d);
-    return PyDict_Check(d) ? d : nullptr;
-  }
-  static PyObject* table(PyObject* m, PyObject* name) {     // _modules or _parameters (borrowed), or null
-    PyObject* d = instance(m);
-    PyObject* t = d ? PyDict_GetItem(d, name) : nullptr;
-    return t && PyDict_Check(t) ? t : nullptr;
-  }
-  static PyObject* find(PyObject* m, const char* name) {
-    PyObject* t = table(m, names().modules);
-    PyObject* c = t ? PyDict_GetItemString(t, name) : nullptr;
-    return c && c != Py_None ? c : nullptr;
-  }
-  PyObject* child(PyObject* m, const char* name, int kind) {
-    PyObject* c = find(m, name);
-    if (!c) { complete = plain = false; return nullptr; }
-    look(c, kind);
+  Module child(const Module& m, PyObject* key, int kind) {
+    const Module c = m.find(key);
+    if (c.self) look(c, kind);
+    else complete = plain = false;
     return c;
   }
   bool has_int(PyObject* dict, PyObject* name, int64_t want) {
@@ -129,33 +136,31 @@ struct Walker {
     if (got == -1 && PyErr_Occurred()) PyErr_Clear();
     return got == want;
   }
-  void look(PyObject* c, int kind) {
-    const bool exact = (PyObject*)Py_TYPE(c) == PyTuple_GET_ITEM(types, kind);
+  void look(const Module& c, int kind) {
+    const bool exact = (PyObject*)Py_TYPE(c.self) == PyTuple_GET_ITEM(types, kind);
     if (kind == K_ATTENTION && !exact) flash = false;
     if (!plain) return;
-    PyObject* d = exact ? instance(c) : nullptr;
-    if (!d || PyDict_GetItem(d, names().forward)) { plain = false; return; }
+    if (!exact || !c.dict || PyDict_GetItem(c.dict, names().forward)) { plain = false; return; }
     for (PyObject* h : names().hooks) {
-      PyObject* t = PyDict_GetItem(d, h);
-      if (!t || PyObject_Size(t) != 0) { PyErr_Clear(); plain = false; return; }
+      PyObject* t = PyDict_GetItem(c.dict, h);
+      if (!t || !PyDict_Check(t) || PyDict_Size(t) != 0) { plain = false; return; }
     }
     if (kind == K_NORM) {
-      PyObject* e = PyDict_GetItem(d, names().eps);
+      PyObject* e = PyDict_GetItem(c.dict, names().eps);
       const double v = e ? PyFloat_AsDouble(e) : -1.0;
       if (v == -1.0 && PyErr_Occurred()) PyErr_Clear();
       plain = v == s->eps;
     } else if (kind == K_ATTENTION) {
       const int64_t want[4] = {s->H, s->D, s->nb, s->md};
-      for (int i = 0; i < 4; ++i) plain = plain && has_int(d, names().attention[i], want[i]);
+      for (int i = 0; i < 4; ++i) plain = plain && has_int(c.dict, names().attention[i], want[i]);
     }
   }
-  Tensor parameter(PyObject* m, const char* name) {
-    if (!m) { complete = false; return Tensor(); }
-    PyObject* t = table(m, names().parameters);
-    PyObject* p = t ? PyDict_GetItemString(t, name) : nullptr;
+  Tensor parameter(const Module& m) {                       // its weight
+    if (!m.self) { complete = false; return Tensor(); }
+    PyObject* p = m.parameters ? PyDict_GetItem(m.parameters, T5B_KEY("weight")) : nullptr;
     if (p && THPVariable_Check(p)) return THPVariable_Unpack(p);
     plain = false;                                          // a parametrised weight: ask the module for it
-    PyObject* a = PyObject_GetAttrString(m, name);
+    PyObject* a = PyObject_GetAttr(m.self, T5B_KEY("weight"));
     if (!a || !THPVariable_Check(a)) {
       PyErr_Clear();
       Py_XDECREF(a);
@@ -166,14 +171,13 @@ struct Walker {
     Py_DECREF(a);
     return w;
   }
-  Tensor weight(PyObject* m, const char* name, int kind) {
-    PyObject* c = child(m, name, kind);
+  Tensor weight(const Module& m, PyObject* key, int kind) {
+    const Module c = child(m, key, kind);
     if (kind == K_LINEAR && plain) {                        // a bias is not part of these blocks
-      PyObject* t = table(c, names().parameters);
-      PyObject* b = t ? PyDict_GetItemString(t, "bias") : nullptr;
+      PyObject* b = c.parameters ? PyDict_GetItem(c.parameters, T5B_KEY("bias")) : nullptr;
       if (b && b != Py_None) plain = false;
     }
-    return parameter(c, "weight");
+    return parameter(c);
   }
 };
 
@@ -182,42 +186,42 @@ Stack collect(PyObject* stack, PyObject* types, bool decoder, int64_t H, int64_t
   Stack s;
   Walker w{types, &s}, wf{types, &s};    // feed-forward layers are looked at apart
   s.decoder = decoder; s.H = H; s.D = D; s.nb = nb; s.md = md; s.eps = eps;
-  PyObject* blocks = Walker::table(Walker::find(stack, "block"), names().modules);
+  const Module top(stack);
+  PyObject* blocks = top.find(T5B_KEY("block")).modules;
   PyObject *key, *blk;
   Py_ssize_t pos = 0;
   while (blocks && w.complete && wf.complete && PyDict_Next(blocks, &pos, &key, &blk)) {
-    w.look(blk, K_BLOCK);
-    PyObject* list = w.child(blk, "layer", K_LIST);
+    const Module block(blk);
+    w.look(block, K_BLOCK);
+    const Module list = w.child(block, T5B_KEY("layer"), K_LIST);
     Layer l;
-    PyObject* sa = w.child(list, "0", K_SELF);
-    PyObject* att = w.child(sa, "SelfAttention", K_ATTENTION);
-    l.ln_self = w.weight(sa, "layer_norm", K_NORM);
-    l.q = w.weight(att, "q", K_LINEAR); l.k = w.weight(att, "k", K_LINEAR);
-    l.v = w.weight(att, "v", K_LINEAR); l.o = w.weight(att, "o", K_LINEAR);
-    if (s.layers.empty()) s.table = w.weight(att, "relative_attention_bias", K_EMBEDDING);
+    const Module sa = w.child(list, T5B_KEY("0"), K_SELF);
+    const Module att = w.child(sa, T5B_KEY("SelfAttention"), K_ATTENTION);
+    l.ln_self = w.weight(sa, T5B_KEY("layer_norm"), K_NORM);
+    l.q = w.weight(att, T5B_KEY("q"), K_LINEAR); l.k = w.weight(att, T5B_KEY("k"), K_LINEAR);
+    l.v = w.weight(att, T5B_KEY("v"), K_LINEAR); l.o = w.weight(att, T5B_KEY("o"), K_LINEAR);
+    if (s.layers.empty()) s.table = w.weight(att, T5B_KEY("relative_attention_bias"), K_EMBEDDING);
     if (decoder) {
-      PyObject* ca = w.child(list, "1", K_CROSS);
-      PyObject* catt = w.child(ca, "EncDecAttention", K_ATTENTION);
-      l.ln_cross = w.weight(ca, "layer_norm", K_NORM);
-      l.cq = w.weight(catt, "q", K_LINEAR); l.ck = w.weight(catt, "k", K_LINEAR);
-      l.cv = w.weight(catt, "v", K_LINEAR); l.co = w.weight(catt, "o", K_LINEAR);
+      const Module ca = w.child(list, T5B_KEY("1"), K_CROSS);
+      const Module catt = w.child(ca, T5B_KEY("EncDecAttention"), K_ATTENTION);
+      l.ln_cross = w.weight(ca, T5B_KEY("layer_norm"), K_NORM);
+      l.cq = w.weight(catt, T5B_KEY("q"), K_LINEAR); l.ck = w.weight(catt, T5B_KEY("k"), K_LINEAR);
+      l.cv = w.weight(catt, T5B_KEY("v"), K_LINEAR); l.co = w.weight(catt, T5B_KEY("o"), K_LINEAR);
     }
-    PyObject* ffl = w.child(list, decoder ? "2" : "1", K_FF);
-    l.ln_ff = w.weight(ffl, "layer_norm", K_NORM);
-    PyObject* ff = Walker::find(ffl, "DenseReluDense");
-    if (!ff) { s.complete = false; return s; }
-    const bool gated = Walker::find(ff, "wi_0") != nullptr;
+    const Module ffl = w.child(list, decoder ? T5B_KEY("2") : T5B_KEY("1"), K_FF);
+    l.ln_ff = w.weight(ffl, T5B_KEY("layer_norm"), K_NORM);
+    const Module ff = ffl.find(T5B_KEY("DenseReluDense"));
+    if (!ff.self) { s.complete = false; return s; }
+    const bool gated = ff.find(T5B_KEY("wi_0")).self != nullptr;
     if (!s.layers.empty() && gated != s.gated) wf.plain = false;
     s.gated = gated;
     wf.look(ff, s.gated ? K_GATED : K_RELU);
-    l.wi0 = wf.weight(ff, s.gated ? "wi_0" : "wi", K_LINEAR);
-    if (s.gated) l.wi1 = wf.weight(ff, "wi_1", K_LINEAR);
-    l.wo = wf.weight(ff, "wo", K_LINEAR);
+    l.wi0 = wf.weight(ff, s.gated ? T5B_KEY("wi_0") : T5B_KEY("wi"), K_LINEAR);
+    if (s.gated) l.wi1 = wf.weight(ff, T5B_KEY("wi_1"), K_LINEAR);
+    l.wo = wf.weight(ff, T5B_KEY("wo"), K_LINEAR);
     s.layers.push_back(std::move(l));
   }
-  PyObject* fin = Walker::find(stack, "final_layer_norm");
-  if (fin) w.look(fin, K_NORM);
-  s.final_ln = w.parameter(fin, "weight");
+  s.final_ln = w.weight(top, T5B_KEY("final_layer_norm"), K_NORM);
   s.complete = w.complete && wf.complete && !s.layers.empty();
   if (!s.complete) return s;
   s.d = s.final_ln.dim() == 1 ? s.final_ln.size(0) : 0;
