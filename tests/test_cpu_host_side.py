@@ -265,3 +265,14 @@ def test_norm_backward_keeps_two_blocks_per_sm():
             assert len(names) == 1, (t, variant)
             k = report[names[0]]
             assert k["registers"] <= 128 and k["spill_stores"] == 0, (names[0], k)
+
+
+def test_forward_kernels_of_every_form_of_call_stay_within_their_budget():
+    """The forms that serve most calls (dense causal, dense whole, packed, block-local): 96 registers for two blocks per
+    SM, and next to no spills (the kernels with the merge of a split wave have 48-92 bytes outside the loop)."""
+    from turbot5_b200 import build
+    report = build.resource_report("attn_fwd_sm100.cu")
+    forms = {n: k for n, k in report.items() if "attn_fwd_case_kernel" in n}
+    assert len(forms) == 2 * 2 * 4          # types, head dims, forms
+    for n, k in forms.items():
+        assert k["registers"] <= 96 and k["spill_stores"] <= 24, (n, k)

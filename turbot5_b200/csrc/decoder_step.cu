@@ -20,7 +20,9 @@
 // predecessor has completed, its own wait included: after it everything earlier in the chain is visible.
 //
 // Semantics: the cached step of the decoder stack (src/turbot5/model/modeling.py:166-219 per block,
-// src/turbot5/model/attentions.py:198,229-234), rounding points as the separate operators.
+// src/turbot5/model/attentions.py:198,229-234).  Rounding points as the separate operators, except for the norm that
+// opens a product in bf16: there the raw row times the norm weight is rounded once and rstd multiplies the float32 sum
+// (step_gemm_kernel), where the operators round the normed row and then its product with the weight.
 #include "t5b_common.cuh"
 
 #include <atomic>
