@@ -657,3 +657,19 @@ def test_every_form_of_call_matches_the_cuda_core_kernel(D, dtype, M, N, causal,
     got, want = (t5b.flash_attention_with_fusing_bias_varlen(*flat, table, cu_q, cu_k, M, N, kernel=kn, **kw) for kn in ("tcgen05", "simt"))
     check_close(got, want, dtype)
     t5b.check_device_status()
+
+
+@pytest.mark.parametrize("D", [16, 32, 64, 128])
+@pytest.mark.parametrize("B,H", [(1, 2), (160, 12)])            # 32 and 64 query rows per block
+def test_float32_keys_past_the_last_query_are_not_touched(B, H, D):
+    """A preallocated cache read with causal=True and an explicit position: what lies past the last query's key may be
+    anything, NaN included, and gives the result of the cut cache."""
+    import turbot5_b200 as t5b
+    M, N, at = 5, 200, 100
+    q = seeded((B, H, M, D), 1, 0.3).cuda()
+    k, v = seeded((B, H, N, D), 2, 0.3).cuda(), seeded((B, H, N, D), 3).cuda()
+    table = seeded((32, H), 4, 0.1).cuda()
+    k[:, :, at + M:], v[:, :, at + M:] = float("nan"), float("nan")
+    out = t5b.flash_attention_with_fusing_bias(q, k, v, table, causal=True, sm_scale=1.0, q_pos_offset=at)
+    want = t5b.flash_attention_with_fusing_bias(q, k[:, :, :at + M], v[:, :, :at + M], table, causal=True, sm_scale=1.0)
+    assert torch.isfinite(out).all() and torch.equal(out, want)

@@ -100,7 +100,7 @@ attn_fwd_simt_kernel(const __grid_constant__ AttnParams p, const __grid_constant
     for (int i = 0; i < CHUNKS; ++i) {
       const int c = tid + i * THREADS, n = n0 + c / (D / 4), d = c % (D / 4) * 4;
       kn[i] = vn[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (n < w.len_k) {
+      if (n < kv_end) {                             // (beyond: not visible to any row here, and 0 x NaN is NaN)
         kn[i] = load4<T>(kbase + (int64_t)n * p.k_stride_n + d, vec);
         vn[i] = load4<T>(vbase + (int64_t)n * p.v_stride_n + d, vec);
       }
