@@ -603,10 +603,9 @@ def test_forward_mode_inputs_that_ask_for_gradients_are_refused():
                 call()
 
 
-def _same_until_a_near_tie(model, states, got, want, lens=None):
+def _same_until_a_near_tie(model, states, tokens, other):
     """Two greedy runs of the same model: equal tokens, or the first difference of a row is at a step where the two
     tokens' logits in an uncached pass over the common prefix are within what 16-bit passes differ by."""
-    tokens, other = got, want
     for b in range(tokens.shape[0]):
         diff = (tokens[b] != other[b]).nonzero()
         if diff.numel() == 0:
